@@ -43,6 +43,7 @@
 #include "sgm_common.cuh"
 #include "sgm_launch.h"
 #include "k_paths_packed.cuh"
+#include "k_paths_seg.cuh"
 #include "k_fused.cuh"
 
 namespace pg {
@@ -760,11 +761,120 @@ cudaError_t launch_paths_shape(const Jobs<NJ>& jobs, const LevelExtent& e, cudaS
     return launched(st, "k_path_row");
 }
 
-// Words per thread of the packed kernels for a launch: 8 (one thread per
-// 16-label chain, the fewest instructions per pixel) when the launch has
-// rows enough for one such warp per SM, else the shorter-step shape
-// (2 words, or 4 for 64 labels).  packed_words_override() (set through
-// pyrsgm_gb300_set_packed_words) forces one of them.
+// Winner-take-all of the packed levels.
+template <int D, bool PYR, int NJ>
+cudaError_t launch_wta(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
+{
+    dim3 gw((e.max_w + 31) / 32, (e.max_h + 7) / 8, jobs.n);
+    prof_begin(st);
+    k_wta<D, PYR, NJ><<<gw, 256, 0, st>>>(jobs);
+    count_launch();
+    prof_end(PK_WTA, jobs_vox(jobs) * 2 * (jobs.d[0].paths >= 3 ? 3 : jobs.d[0].paths) + jobs_px(jobs) * (2 + 6 + 4), st);
+    return launched(st, "k_wta");
+}
+
+// The wide shape: one thread per 16 labels.
+template <int T, bool PYR, int NJ>
+cudaError_t launch_paths_wide(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
+{
+    constexpr int NW = 8;
+    using G = pk::Grp<NW, T>;
+    cudaError_t err;
+    bool any_tb = false;
+    for (int i = 0; i < jobs.n; ++i) any_tb = any_tb || jobs.d[i].paths >= 3;
+    // T->B and the horizontal paths run one after the other: launches of
+    // this shape fill the GPU, side by side they would only contend.
+    // 16-label pyramid levels, wide shape, three paths everywhere, and
+    // columns for at least kTbwMinWarpsPerSm warps per SM: the row pass
+    // first, then T->B with the winner-take-all (k_gtbw).  Its serial chain
+    // step carries the winner's work, so with few warps per SM it loses to
+    // k_gtb + k_wta: per launch, 16 pairs of 1080p, 1165 against 1031 us
+    // at 6.3 warps per SM and 467 against 308 us at 3.2; at 12.6 warps per
+    // SM (32 pairs) it is about 15 % faster.
+    bool tbw = false;
+    if constexpr (PYR && T == 1) {
+        long long cols = 0;
+        tbw = tbw_mode() != 0;
+        for (int i = 0; i < jobs.n; ++i) {
+            tbw = tbw && jobs.d[i].paths >= 3;
+            cols += jobs.d[i].w;
+        }
+        tbw = tbw && (tbw_mode() == 2 || cols >= 32LL * pk::kTbwMinWarpsPerSm * sm_count());
+    }
+    if (tbw) any_tb = false;
+    if (any_tb) {
+        Jobs<NJ> tbj = jobs;
+        int n = 0;
+        for (int i = 0; i < jobs.n; ++i)
+            if (jobs.d[i].paths >= 3) tbj.d[n++] = jobs.d[i];
+        tbj.n = n;
+        constexpr size_t smem = pk::tb_smem<NW, T>();
+        if ((err = cudaFuncSetAttribute(k_gtb<NW, T, PYR, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)smem)) != cudaSuccess)
+            return err;
+        constexpr int kWarps = pk::kPackedWarps;
+        const int cols = kWarps * G::CPW;
+        dim3 g((e.max_w + cols - 1) / cols, n);
+        prof_begin(st);
+        k_gtb<NW, T, PYR, NJ><<<g, kWarps * 32, smem, st>>>(tbj);
+        count_launch();
+        prof_end(PK_PATH_TB, jobs_vox(tbj) * 4 + jobs_px(tbj) * ((tbj.d[0].refine ? 2 : 0) + (tbj.d[0].adaptive ? 1 : 0)), st);
+        if ((err = launched(st, "k_gtb")) != cudaSuccess) return err;
+    }
+    constexpr int kWarps = pk::kPackedWarps;
+    const int rows = kWarps * G::CPW / 2;
+    dim3 g((e.max_h + rows - 1) / rows, jobs.n);
+    constexpr size_t smem = pk::row_smem<NW, T>();
+    if ((err = cudaFuncSetAttribute(k_grow<NW, T, PYR, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+        cudaSuccess)
+        return err;
+    prof_begin(st);
+    k_grow<NW, T, PYR, NJ><<<g, kWarps * 32, smem, st>>>(jobs);
+    count_launch();
+    if (prof_enabled()) {
+        // algorithmic bytes: each horizontal path reads the cost volume and
+        // writes its costs once
+        double by = 0;
+        for (int i = 0; i < jobs.n; ++i) {
+            const LevelDesc& d = jobs.d[i];
+            const double px = (double)d.w * d.h;
+            by += px * d.D * 2 * (d.paths >= 2 ? 4 : 2) + px * 2 * ((d.refine ? 2 : 0) + (d.adaptive ? 1 : 0));
+        }
+        prof_end(PK_PATH_ROW, by, st);
+    }
+    if ((err = launched(st, "k_grow")) != cudaSuccess) return err;
+    if constexpr (PYR && T == 1) {
+        if (tbw) {
+            constexpr size_t smem = pk::tbw_smem();
+            if ((err = cudaFuncSetAttribute(k_gtbw<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+                cudaSuccess)
+                return err;
+            dim3 gt((e.max_w + 127) / 128, jobs.n);
+            prof_begin(st);
+            k_gtbw<NJ><<<gt, 128, smem, st>>>(jobs);
+            count_launch();
+            prof_end(PK_TBW, jobs_vox(jobs) * 6 + jobs_px(jobs) * ((jobs.d[0].refine ? 2 : 0) + (jobs.d[0].adaptive ? 1 : 0) + 10),
+                     st);
+            return launched(st, "k_gtbw");
+        }
+    }
+    return launch_wta<G::D, PYR, NJ>(jobs, e, st);
+}
+
+// The segmented shape: every chain cut into segments that run at the same
+// time, rows and columns in one launch.
+template <int NW, int T, bool PYR, int NJ>
+cudaError_t launch_paths_seg(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
+{
+    const cudaError_t err = launch_seg<NW, T, PYR, NJ>(jobs, true, st);
+    return err != cudaSuccess ? err : launch_wta<2 * NW * T, PYR, NJ>(jobs, e, st);
+}
+
+// Shape of the packed kernels for a launch: 8 (the wide shape, one thread
+// per 16 labels, whole chains) when the launch has rows enough for one such
+// warp per SM, else 2 (4 for 64 labels), the segmented shape.
+// packed_words_override() (set through pyrsgm_gb300_set_packed_words) forces
+// one of them.
 inline int packed_nw(int D, long long rows)
 {
     const int force = packed_words_override();
@@ -833,24 +943,24 @@ cudaError_t launch_paths_mode(const Jobs<NJ>& jobs, const LevelExtent& e, cudaSt
             if constexpr (PYR) {
                 if (nw == 8 && fused) return launch_paths_fused16<NJ>(jobs, e, st);
             }
-            return nw == 8 ? launch_paths_packed<8, 1, PYR, NJ>(jobs, e, st)
-                           : launch_paths_packed<2, 4, PYR, NJ>(jobs, e, st);
+            return nw == 8 ? launch_paths_wide<1, PYR, NJ>(jobs, e, st)
+                           : launch_paths_seg<4, 2, PYR, NJ>(jobs, e, st);
         };
         const int nw = packed_choice(key, rows, st, run, err);
         return err != cudaSuccess ? err : run(nw);
     }
     case 10032: {
         auto run = [&](int nw) {
-            return nw == 8 ? launch_paths_packed<8, 2, PYR, NJ>(jobs, e, st)
-                           : launch_paths_packed<2, 8, PYR, NJ>(jobs, e, st);
+            return nw == 8 ? launch_paths_wide<2, PYR, NJ>(jobs, e, st)
+                           : launch_paths_seg<4, 4, PYR, NJ>(jobs, e, st);
         };
         const int nw = packed_choice(key, rows, st, run, err);
         return err != cudaSuccess ? err : run(nw);
     }
     case 10064: {
         auto run = [&](int nw) {
-            return nw == 8 ? launch_paths_packed<8, 4, PYR, NJ>(jobs, e, st)
-                           : launch_paths_packed<4, 8, PYR, NJ>(jobs, e, st);
+            return nw == 8 ? launch_paths_wide<4, PYR, NJ>(jobs, e, st)
+                           : launch_paths_seg<4, 8, PYR, NJ>(jobs, e, st);
         };
         const int nw = packed_choice(key, rows, st, run, err);
         return err != cudaSuccess ? err : run(nw);

@@ -1,9 +1,9 @@
-// k_paths_packed.cuh -- path aggregation for D = 2*NW*T labels (16, 32,
-// 64): the labels of one path chain are packed two per 32-bit word and held
-// by T threads, NW words each.  NW = 8 (a 16-label chain is one thread)
-// spends the fewest instructions per pixel and suits launches with many
-// rows; NW = 2 spreads a chain over more threads, shortening each step, for
-// launches with few rows (one pair, coarse levels).
+// k_paths_packed.cuh -- path aggregation for D = 16, 32 and 64 labels: the
+// labels of one path chain are packed two per 32-bit word and held by T
+// threads, eight words (16 labels) each.  This is the shape for launches
+// with many rows: it spends the fewest instructions per pixel and fills the
+// GPU with whole chains.  Launches with few rows cut their chains into
+// segments (k_paths_seg.cuh).
 //
 // The recurrence of a step (reference: src/sgm_kernels.cu:560-565
 // single-scale, 1230-1252 pyramid) runs on 16-bit pairs with the DPX
@@ -36,8 +36,7 @@
 // step are issued several steps before it without holding registers.  The
 // T->B pass has one slot per step and thread (a warp's 32 columns are
 // adjacent, so its requests are whole lines already); the horizontal pass
-// of the NW = 8 shapes moves 128-byte runs of each chain with the whole
-// warp (chunk_steps), that of the spread shapes streams per lane.
+// moves 128-byte runs of each chain with the whole warp (chunk_steps).
 //
 // Paths: the T->B chains write their costs into V, the L->R and R->L chains
 // of each row into Vl and Vr; the chains never exchange data.  The WTA
@@ -61,12 +60,8 @@ namespace pk {
 
 constexpr uint32_t kMax2 = 0x7fff7fffu;
 constexpr uint32_t kOne2 = 0x00010001u;
-// Warps per block: 4 for the one-thread-per-16-labels shape (throughput on
-// many rows), 2 for the spread shapes (more, smaller blocks for few rows).
-template <int NW>
-__host__ __device__ constexpr int warps_of() { return NW == 8 ? 4 : 2; }
+constexpr int kPackedWarps = 4;  // warps per block
 constexpr int kStagesTb = 8;     // look-ahead of the top->bottom pass
-constexpr int kStagesLane = 6;   // look-ahead of the per-lane horizontal pass
 
 __device__ __forceinline__ uint32_t dup(int v) { return ((uint32_t)v & 0xffffu) * 0x10001u; }
 
@@ -82,10 +77,6 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)
 __device__ __forceinline__ void cp16(void* dst, const void* src)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp8(void* dst, const void* src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp4(void* dst, const void* src)
 {
@@ -113,7 +104,7 @@ struct Grp {
     static constexpr int LENW = PADW + D + 2;   // words a shifted window can touch
     static constexpr int BUFW = LENW * CPW;     // one window buffer of a warp
     static constexpr int NBUF = T == 1 ? 1 : 2;
-    // Ring slot of a thread: its NW cost words.  For NW = 8 the two 16-byte
+    // Ring slot of a thread: its NW cost words.  The two 16-byte
     // halves of a slot are swapped in lanes 4-7 of every 8 (ring_half), so
     // that the 16-byte accesses of 8 lanes at a 32-byte stride hit distinct
     // banks.  The label-base and image words of a slot sit in a separate
@@ -163,18 +154,6 @@ __device__ __forceinline__ void stw(uint32_t* p, const uint32_t (&v)[NW])
             reinterpret_cast<uint4*>(p)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
     }
 }
-// Asynchronous copy of NW words.
-template <int NW>
-__device__ __forceinline__ void cpw(uint32_t* dst, const int16_t* src)
-{
-    if constexpr (NW == 2) {
-        cp8(dst, src);
-    } else {
-#pragma unroll
-        for (int i = 0; i < NW / 4; ++i) cp16(dst + 4 * i, src + 8 * i);
-    }
-}
-
 // Position of half h (0, 1) of an NW = 8 ring slot in lane `lane`'s slot.
 __device__ __forceinline__ int ring_half(int h, int lane) { return 4 * (h ^ ((lane >> 2) & 1)); }
 
@@ -398,19 +377,13 @@ constexpr size_t row_smem()
     constexpr int CH = chunk_steps<G::D>(), SC = chunk_stages<G::D>();
     // per warp: window buffers, SC input chunk slots and one output chunk
     // (32 words per chain each), the label-base / image ring
-    return 256 * 4 + (size_t)warps_of<NW>() * 4 * (G::NBUF * G::BUFW + (SC + 1) * G::CPW * 32 + SC * CH * 64);
-}
-template <int NW, int T>
-constexpr size_t row_lane_smem()
-{
-    using G = Grp<NW, T>;
-    return 256 * 4 + (size_t)warps_of<NW>() * 4 * (G::NBUF * G::BUFW + kStagesLane * 32 * (G::RSW_TB + 2));
+    return 256 * 4 + (size_t)kPackedWarps * 4 * (G::NBUF * G::BUFW + (SC + 1) * G::CPW * 32 + SC * CH * 64);
 }
 template <int NW, int T>
 constexpr size_t tb_smem()
 {
     using G = Grp<NW, T>;
-    return 256 * 4 + (size_t)warps_of<NW>() * 4 * (G::NBUF * G::BUFW + kStagesTb * 32 * (G::RSW_TB + 2));
+    return 256 * 4 + (size_t)kPackedWarps * 4 * (G::NBUF * G::BUFW + kStagesTb * 32 * (G::RSW_TB + 2));
 }
 
 }  // namespace pk
@@ -419,11 +392,11 @@ constexpr size_t tb_smem()
 // Top -> bottom: a warp holds 32/T adjacent columns, T threads each.
 // ---------------------------------------------------------------------------
 template <int NW, int T, bool PYR, int NJ>
-__global__ void __launch_bounds__(pk::warps_of<NW>() * 32) k_gtb(const __grid_constant__ Jobs<NJ> jobs)
+__global__ void __launch_bounds__(pk::kPackedWarps * 32) k_gtb(const __grid_constant__ Jobs<NJ> jobs)
 {
     using namespace pk;
     using G = Grp<NW, T>;
-    constexpr int D = G::D, S = kStagesTb, RS = G::RSW_TB, kWarps = warps_of<NW>();
+    constexpr int D = G::D, S = kStagesTb, RS = G::RSW_TB, kWarps = kPackedWarps;
     const LevelDesc& J = jobs.d[blockIdx.y];
     extern __shared__ __align__(16) uint32_t smem[];
     int* lut = reinterpret_cast<int*>(smem);
@@ -462,12 +435,8 @@ __global__ void __launch_bounds__(pk::warps_of<NW>() * 32) k_gtb(const __grid_co
     auto issue_next = [&](int slot) {
         if (yi < H && PG_IN(oi, 2 * NW, (size_t)W * H * D, 1)) {
             uint32_t* d = ring + slot * 32 * RS;
-            if constexpr (NW == 8) {
-                cp16(d + ring_half(0, lane), Cg + oi);
-                cp16(d + ring_half(1, lane), Cg + oi + 8);
-            } else {
-                cpw<NW>(d, Cg + oi);
-            }
+            cp16(d + ring_half(0, lane), Cg + oi);
+            cp16(d + ring_half(1, lane), Cg + oi + 8);
             if (use_base) cp4(bi + slot * 64, word_of(Bg + pi));
             if (adaptive) cp4(bi + slot * 64 + 32, word_of(Lg + li));
         }
@@ -491,13 +460,11 @@ __global__ void __launch_bounds__(pk::warps_of<NW>() * 32) k_gtb(const __grid_co
         const uint32_t* db = bi + slot * 64;
         slot = slot + 1 == S ? 0 : slot + 1;
         uint32_t cc[NW];
-        if constexpr (NW == 8) {
+        {
             const uint4 a = *reinterpret_cast<const uint4*>(d + ring_half(0, lane));
             const uint4 b = *reinterpret_cast<const uint4*>(d + ring_half(1, lane));
             cc[0] = a.x; cc[1] = a.y; cc[2] = a.z; cc[3] = a.w;
             cc[4] = b.x; cc[5] = b.y; cc[6] = b.z; cc[7] = b.w;
-        } else {
-            ldw<NW>(d, cc);
         }
         const int base = use_base ? (int)(int16_t)(db[0] >> ((pc & 1) * 16)) : J.minD;
         int p2 = J.P2;
@@ -531,11 +498,11 @@ __global__ void __launch_bounds__(pk::warps_of<NW>() * 32) k_gtb(const __grid_co
 // conflicts.
 // ---------------------------------------------------------------------------
 template <int NW, int T, bool PYR, int NJ>
-__global__ void __launch_bounds__(pk::warps_of<NW>() * 32) k_grow(const __grid_constant__ Jobs<NJ> jobs)
+__global__ void __launch_bounds__(pk::kPackedWarps * 32) k_grow(const __grid_constant__ Jobs<NJ> jobs)
 {
     using namespace pk;
     using G = Grp<NW, T>;
-    constexpr int D = G::D, CPW = G::CPW, RPW = CPW / 2, kWarps = warps_of<NW>();
+    constexpr int D = G::D, CPW = G::CPW, RPW = CPW / 2, kWarps = kPackedWarps;
     constexpr int CH = chunk_steps<D>(), SC = chunk_stages<D>();
     constexpr int PPX = D / 8;          // 16-byte pieces per pixel
     constexpr int NCOP = CPW / 4;       // pieces a lane moves per chunk
@@ -655,15 +622,10 @@ __global__ void __launch_bounds__(pk::warps_of<NW>() * 32) k_grow(const __grid_c
             const int q = dir ? CH - 1 - s : s;
             const int w0 = q * (D / 2) + k * NW;
             uint32_t cc[NW];
-            if constexpr (NW == 2) {
-                const uint2 a = *reinterpret_cast<const uint2*>(cin + piece_col(c, w0 >> 2) + (w0 & 3));
-                cc[0] = a.x; cc[1] = a.y;
-            } else {
 #pragma unroll
-                for (int i = 0; i < NW / 4; ++i) {
-                    const uint4 a = *reinterpret_cast<const uint4*>(cin + piece_col(c, (w0 >> 2) + i));
-                    cc[4 * i] = a.x; cc[4 * i + 1] = a.y; cc[4 * i + 2] = a.z; cc[4 * i + 3] = a.w;
-                }
+            for (int i = 0; i < NW / 4; ++i) {
+                const uint4 a = *reinterpret_cast<const uint4*>(cin + piece_col(c, (w0 >> 2) + i));
+                cc[4 * i] = a.x; cc[4 * i + 1] = a.y; cc[4 * i + 2] = a.z; cc[4 * i + 3] = a.w;
             }
             const int x = xs + dx * t;
             int base = minD;
@@ -683,14 +645,10 @@ __global__ void __launch_bounds__(pk::warps_of<NW>() * 32) k_grow(const __grid_c
                 mask_labels<NW>(cc, lo, hi, k);
             }
             gstep<NW, T, PYR>(st, cc, base, p2, p12, chain + (G::NBUF == 2 ? (t & 1) * G::BUFW : 0), k);
-            if constexpr (NW == 2) {
-                *reinterpret_cast<uint2*>(ob + piece_col(c, w0 >> 2) + (w0 & 3)) = make_uint2(st.L[0], st.L[1]);
-            } else {
 #pragma unroll
-                for (int i = 0; i < NW / 4; ++i)
-                    *reinterpret_cast<uint4*>(ob + piece_col(c, (w0 >> 2) + i)) =
-                        make_uint4(st.L[4 * i], st.L[4 * i + 1], st.L[4 * i + 2], st.L[4 * i + 3]);
-            }
+            for (int i = 0; i < NW / 4; ++i)
+                *reinterpret_cast<uint4*>(ob + piece_col(c, (w0 >> 2) + i)) =
+                    make_uint4(st.L[4 * i], st.L[4 * i + 1], st.L[4 * i + 2], st.L[4 * i + 3]);
         }
         __syncwarp();
         {
@@ -706,120 +664,6 @@ __global__ void __launch_bounds__(pk::warps_of<NW>() * 32) k_grow(const __grid_c
         }
         __syncwarp();
         slot = slot + 1 == SC ? 0 : slot + 1;
-    }
-    cp_wait<0>();
-}
-
-// ---------------------------------------------------------------------------
-// Horizontal paths, per-lane loads: the same chains as k_grow, each thread
-// streaming its own costs through a ring of kStagesLane steps and storing
-// its path costs directly.  For the spread shapes (NW < 8) on launches with
-// few rows, where the per-step latency of a chain bounds the pass rather
-// than HBM: the warp-wide chunk copies of k_grow add two warp
-// synchronisations and a shared-memory round trip to every chunk.
-// ---------------------------------------------------------------------------
-template <int NW, int T, bool PYR, int NJ>
-__global__ void __launch_bounds__(pk::warps_of<NW>() * 32) k_grow_lane(const __grid_constant__ Jobs<NJ> jobs)
-{
-    using namespace pk;
-    using G = Grp<NW, T>;
-    constexpr int D = G::D, RPW = G::CPW / 2, S = kStagesLane, RS = G::RSW_TB, kWarps = warps_of<NW>();
-    const LevelDesc& J = jobs.d[blockIdx.y];
-    extern __shared__ __align__(16) uint32_t smem[];
-    int* lut = reinterpret_cast<int*>(smem);
-    uint32_t* cbuf = smem + 256;
-    uint32_t* rbuf = cbuf + kWarps * G::NBUF * G::BUFW;
-    uint32_t* bibuf = rbuf + kWarps * S * 32 * RS;
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = J.adaptive ? J.p2lut[i] : 0;
-    for (int i = threadIdx.x; i < kWarps * G::NBUF * G::BUFW; i += blockDim.x) cbuf[i] = kMax2;
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = lane / T, k = lane % T, r = c >> 1, dir = c & 1;
-    const int row0 = (blockIdx.x * kWarps + warp) * RPW;
-    if (row0 >= J.h) return;   // the whole warp is past the image
-    const int y = row0 + r;
-    const bool row_ok = y < J.h;
-    const int yy = imin(y, J.h - 1);
-    const int W = J.w;
-    uint32_t* chain = cbuf + warp * G::NBUF * G::BUFW + c;
-    uint32_t* ring = rbuf + (warp * S * 32 + lane) * RS;
-    uint32_t* bi = bibuf + warp * S * 64 + lane;   // [slot][base, image][lane]
-
-    // path extents (single-scale: kernel_AggregateLR/RL ranges)
-    int lr_x0 = 0, lr_n, rl_n;
-    if (PYR) {
-        lr_n = J.paths >= 2 ? W : 0;
-        rl_n = W;
-    } else {
-        const int minX1 = imax(J.minD + D, 0), maxX1 = W + imin(J.minD, 0);
-        lr_x0 = minX1;
-        lr_n = J.paths >= 2 ? imax(0, maxX1 - minX1) : 0;
-        rl_n = imax(0, W - minX1);
-    }
-    const int n_mine = dir == 0 ? lr_n : rl_n;
-    const int Tn = imax(lr_n, rl_n);
-    const int dx = dir == 0 ? 1 : -1;
-    const int xs = dir == 0 ? lr_x0 : W - 1;   // step t of this chain is at x = xs + dx * t
-    const int16_t* const Cg = J.C;
-    int16_t* const Og = dir == 0 ? J.Vl : J.Vr;
-    const int16_t* const Bg = J.base;
-    const uint8_t* const Lg = J.left;
-    const bool use_base = PYR && J.refine, adaptive = J.adaptive != 0;
-    const int P2c = J.P2, minD = J.minD;
-    const size_t prow = (size_t)yy * W;
-    const size_t lrow = (size_t)yy * J.lstep;
-    const long long dxD = (long long)dx * D;
-    // issue cursor (step ti) and consume cursor (step t): voxel offset, pixel index, image index
-    size_t oi = (prow + xs) * D + 2 * NW * k, pi = prow + xs, li = lrow + xs;
-    size_t oc = oi, pc = pi, lc = li;
-    int ti = 0;
-    auto issue_next = [&](int slot) {
-        if (ti < n_mine && PG_IN(oi, 2 * NW, (size_t)W * J.h * D, 5)) {
-            cpw<NW>(ring + slot * 32 * RS, Cg + oi);
-            if (use_base) cp4(bi + slot * 64, word_of(Bg + pi));
-            if (adaptive) cp4(bi + slot * 64 + 32, word_of(Lg + li));
-        }
-        cp_commit();
-        ++ti;
-        oi += dxD;
-        pi += dx;
-        li += dx;
-    };
-
-    const uint32_t p12 = dup(imin(J.P1, 0x8000));
-    GChain<NW> s;
-    gchain_init(s, minD);
-#pragma unroll
-    for (int j = 0; j < S - 1; ++j) issue_next(j);
-    int img_prev = 0, slot = 0, islot = S - 1;
-#pragma unroll 2
-    for (int t = 0; t < Tn; ++t) {
-        issue_next(islot);
-        islot = islot + 1 == S ? 0 : islot + 1;
-        cp_wait<S - 1>();
-        const uint32_t* d = ring + slot * 32 * RS;
-        const uint32_t* db = bi + slot * 64;
-        slot = slot + 1 == S ? 0 : slot + 1;
-        uint32_t cc[NW];
-        ldw<NW>(d, cc);
-        const int base = use_base ? (int)(int16_t)(db[0] >> ((pc & 1) * 16)) : minD;
-        int p2 = P2c;
-        if (adaptive) {
-            const int img = (int)((db[32] >> byte_shift(Lg + lc)) & 255u);
-            p2 = lut[abs(img - img_prev) & 255];
-            img_prev = img;
-        }
-        if (PYR && !J.refine) {
-            int lo, hi;
-            label_range(J, xs + dx * t, minD, lo, hi);
-            mask_labels<NW>(cc, lo, hi, k);
-        }
-        gstep<NW, T, PYR>(s, cc, base, p2, p12, chain + (G::NBUF == 2 ? (t & 1) * G::BUFW : 0), k);
-        if (t < n_mine && row_ok && PG_IN(oc, 2 * NW, (size_t)W * J.h * D, 6))
-            stw<NW>(reinterpret_cast<uint32_t*>(Og + oc), s.L);
-        oc += dxD;
-        pc += dx;
-        lc += dx;
     }
     cp_wait<0>();
 }
@@ -1047,124 +891,6 @@ __global__ void __launch_bounds__(128, 4) k_gtbw(const __grid_constant__ Jobs<NJ
         lc += lstep;
     }
     cp_wait<0>();
-}
-
-
-
-template <int NW, int T, bool PYR, int NJ>
-cudaError_t launch_paths_packed(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
-{
-    using G = pk::Grp<NW, T>;
-    cudaError_t err;
-    bool any_tb = false;
-    for (int i = 0; i < jobs.n; ++i) any_tb = any_tb || jobs.d[i].paths >= 3;
-    // T->B and the horizontal paths only share the cost volume.  In the
-    // spread shapes (launches with few rows, which leave most SMs idle) T->B
-    // runs on a second stream beside the row pass, joined before the WTA;
-    // launches that fill the GPU run them one after the other (side by side
-    // they only contend).
-    // 16-label pyramid levels, wide shape, three paths everywhere, and
-    // columns for at least kTbwMinWarpsPerSm warps per SM: the row pass
-    // first, then T->B with the winner-take-all (k_gtbw).  Its serial chain
-    // step carries the winner's work, so with few warps per SM it loses to
-    // k_gtb + k_wta: per launch, 16 pairs of 1080p, 1165 against 1031 us
-    // at 6.3 warps per SM and 467 against 308 us at 3.2; at 12.6 warps per
-    // SM (32 pairs) it is about 15 % faster.
-    bool tbw = false;
-    if constexpr (PYR && NW == 8 && T == 1) {
-        long long cols = 0;
-        tbw = tbw_mode() != 0;
-        for (int i = 0; i < jobs.n; ++i) {
-            tbw = tbw && jobs.d[i].paths >= 3;
-            cols += jobs.d[i].w;
-        }
-        tbw = tbw && (tbw_mode() == 2 || cols >= 32LL * pk::kTbwMinWarpsPerSm * sm_count());
-    }
-    ForkStreams& fk = fork_streams(st);
-    const bool fork = NW != 8 && any_tb && fk.aux != nullptr;
-    cudaStream_t tbst = st;
-    if (tbw) any_tb = false;
-    if (fork) {
-        if ((err = cudaEventRecord(fk.fork, st)) != cudaSuccess) return err;
-        if ((err = cudaStreamWaitEvent(fk.aux, fk.fork, 0)) != cudaSuccess) return err;
-        tbst = fk.aux;
-    }
-    if (any_tb) {
-        Jobs<NJ> tbj = jobs;
-        int n = 0;
-        for (int i = 0; i < jobs.n; ++i)
-            if (jobs.d[i].paths >= 3) tbj.d[n++] = jobs.d[i];
-        tbj.n = n;
-        constexpr size_t smem = pk::tb_smem<NW, T>();
-        if ((err = cudaFuncSetAttribute(k_gtb<NW, T, PYR, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem)) != cudaSuccess)
-            return err;
-        constexpr int kWarps = pk::warps_of<NW>();
-        const int cols = kWarps * G::CPW;
-        dim3 g((e.max_w + cols - 1) / cols, n);
-        prof_begin(tbst);
-        k_gtb<NW, T, PYR, NJ><<<g, kWarps * 32, smem, tbst>>>(tbj);
-        count_launch();
-        prof_end(PK_PATH_TB, jobs_vox(tbj) * 4 + jobs_px(tbj) * ((tbj.d[0].refine ? 2 : 0) + (tbj.d[0].adaptive ? 1 : 0)), tbst);
-        if ((err = launched(tbst, "k_gtb")) != cudaSuccess) return err;
-    }
-    constexpr int kWarps = pk::warps_of<NW>();
-    const int rows = kWarps * G::CPW / 2;
-    dim3 g((e.max_h + rows - 1) / rows, jobs.n);
-    // NW == 8 (many rows): warp-wide 128-byte chunk I/O; spread shapes: per-lane streams
-    if constexpr (NW == 8) {
-        constexpr size_t smem = pk::row_smem<NW, T>();
-        if ((err = cudaFuncSetAttribute(k_grow<NW, T, PYR, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem)) != cudaSuccess)
-            return err;
-        prof_begin(st);
-        k_grow<NW, T, PYR, NJ><<<g, kWarps * 32, smem, st>>>(jobs);
-    } else {
-        constexpr size_t smem = pk::row_lane_smem<NW, T>();
-        if ((err = cudaFuncSetAttribute(k_grow_lane<NW, T, PYR, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem)) != cudaSuccess)
-            return err;
-        prof_begin(st);
-        k_grow_lane<NW, T, PYR, NJ><<<g, kWarps * 32, smem, st>>>(jobs);
-    }
-    count_launch();
-    if (prof_enabled()) {
-        // algorithmic bytes: each horizontal path reads the cost volume and
-        // writes its costs once
-        double by = 0;
-        for (int i = 0; i < jobs.n; ++i) {
-            const LevelDesc& d = jobs.d[i];
-            const double px = (double)d.w * d.h;
-            by += px * d.D * 2 * (d.paths >= 2 ? 4 : 2) + px * 2 * ((d.refine ? 2 : 0) + (d.adaptive ? 1 : 0));
-        }
-        prof_end(PK_PATH_ROW, by, st);
-    }
-    if ((err = launched(st, NW == 8 ? "k_grow" : "k_grow_lane")) != cudaSuccess) return err;
-    if (fork) {
-        if ((err = cudaEventRecord(fk.join, fk.aux)) != cudaSuccess) return err;
-        if ((err = cudaStreamWaitEvent(st, fk.join, 0)) != cudaSuccess) return err;
-    }
-    if constexpr (PYR && NW == 8 && T == 1) {
-        if (tbw) {
-            constexpr size_t smem = pk::tbw_smem();
-            if ((err = cudaFuncSetAttribute(k_gtbw<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-                cudaSuccess)
-                return err;
-            dim3 gt((e.max_w + 127) / 128, jobs.n);
-            prof_begin(st);
-            k_gtbw<NJ><<<gt, 128, smem, st>>>(jobs);
-            count_launch();
-            prof_end(PK_TBW, jobs_vox(jobs) * 6 + jobs_px(jobs) * ((jobs.d[0].refine ? 2 : 0) + (jobs.d[0].adaptive ? 1 : 0) + 10),
-                     st);
-            return launched(st, "k_gtbw");
-        }
-    }
-    dim3 gw((e.max_w + 31) / 32, (e.max_h + 7) / 8, jobs.n);
-    prof_begin(st);
-    k_wta<G::D, PYR, NJ><<<gw, 256, 0, st>>>(jobs);
-    count_launch();
-    prof_end(PK_WTA, jobs_vox(jobs) * 2 * (jobs.d[0].paths >= 3 ? 3 : jobs.d[0].paths) + jobs_px(jobs) * (2 + 6 + 4), st);
-    return launched(st, "k_wta");
 }
 
 }  // namespace pg
