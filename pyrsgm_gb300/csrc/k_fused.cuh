@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(fz::kRlwWarps * 32) k_rlw(const __grid_constan
                 c0 = d == bestD - 1 ? v : c0;
                 c2 = d == bestD + 1 ? v : c2;
             }
-            pk::wta_out<16, true>(J, y, x, base, minCost, bestD, (int)(a >> 7), c0, minCost, c2);
+            pk::wta_out<true>(J, 16, y, x, base, minCost, bestD, (int)(a >> 7), c0, minCost, c2);
         }
         __syncwarp();
         slot = slot + 1 == SC ? 0 : slot + 1;

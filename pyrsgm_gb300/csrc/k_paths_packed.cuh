@@ -297,8 +297,8 @@ __device__ __forceinline__ void wta16(const uint32_t (&t)[8], int& minCost, int&
 // pyramid kernel_PyramidWTA, src/sgm_kernels.cu:1290-1370): minimum cost,
 // first label reaching it, the minimum over labels farther than one from
 // it, and the costs next to it (c0, c2; 0 outside the range).
-template <int D, bool PYR>
-__device__ __forceinline__ void wta_out(const LevelDesc& J, int y, int x, int base, int minCost, int bestD, int alt,
+template <bool PYR>
+__device__ __forceinline__ void wta_out(const LevelDesc& J, int D, int y, int x, int base, int minCost, int bestD, int alt,
                                         int c0, int c1, int c2)
 {
     const int16_t inv = (int16_t)((J.minD - 1) * 16);
@@ -759,7 +759,7 @@ __global__ void __launch_bounds__(256) k_wta(const __grid_constant__ Jobs<NJ> jo
     const int c0 = bestD > 0 ? half(bestD - 1) : 0;
     const int c2 = bestD + 1 < D ? half(bestD + 1) : 0;
     const int base = (PYR && J.refine) ? (int)J.base[p] : J.minD;
-    wta_out<D, PYR>(J, y, x, base, minCost, bestD, alt, c0, minCost, c2);
+    wta_out<PYR>(J, D, y, x, base, minCost, bestD, alt, c0, minCost, c2);
 }
 
 // ---------------------------------------------------------------------------
@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(128, 4) k_gtbw(const __grid_constant__ Jobs<NJ
             }
             int minCost, bestD, alt, c0, c2;
             wta16(t, minCost, bestD, alt, c0, c2);
-            wta_out<D, true>(J, y, x, base, minCost, bestD, alt, c0, minCost, c2);
+            wta_out<true>(J, D, y, x, base, minCost, bestD, alt, c0, minCost, c2);
         }
         pc += W;
         lc += lstep;

@@ -47,11 +47,18 @@ using pk::kOne2;
 
 // Level semantics of a walk.
 enum { kSingle = 0, kCoarse = 1, kRefine = 2 };
+// What a walk does with the path costs: store them; store them until they
+// equal the stored ones; add them to the sum in V (rows of both directions
+// in step).
+enum { kStore = 0, kAgain = 1, kAdd = 2 };
 
 constexpr int kCH = 4;       // steps per chunk
 constexpr int kSC = 3;       // chunk slots per warp
 constexpr int kAhead = 3;    // chunks of look-ahead of the per-pixel inputs
-constexpr int kMaxSeg = 16;  // segments (warps) per block
+constexpr int kMaxSeg = 16;  // segments (warps) per block at most
+// ... for NW words a thread: shared memory for the rings, and registers.
+template <int NW>
+__host__ __device__ constexpr int max_seg() { return NW >= 32 ? 4 : NW >= 16 ? 8 : kMaxSeg; }
 
 template <int NW, int T>
 struct Geo {
@@ -74,11 +81,16 @@ struct Geo {
 };
 
 template <int NW, int T, int MODE>
-__host__ __device__ constexpr int warp_words()
+__host__ __device__ constexpr int warp_words(int rings = 1)
 {
     using G = Geo<NW, T>;
     static_assert(G::CSTR % 4 == 0 && G::BUFW % 4 == 0, "cp.async writes 16-byte pieces");
-    return kSC * G::SLOTW + (MODE == kRefine ? 2 * G::BUFW : 0);
+    return rings * kSC * G::SLOTW + (MODE == kRefine ? 2 * G::BUFW : 0);
+}
+template <int NW, int T, int MODE>
+constexpr size_t add_smem()
+{
+    return 4 * (256 + (size_t)warp_words<NW, T, MODE>(2));
 }
 template <int NW, int T, int MODE>
 constexpr size_t seg_smem(int segs)
@@ -108,6 +120,20 @@ __device__ __forceinline__ void load_words(const int16_t* p, int d0, int Dr, uin
             if (d0 + 8 * i >= Dr) break;
             const uint4 a = __ldcg(reinterpret_cast<const uint4*>(p) + i);
             v[4 * i] = a.x; v[4 * i + 1] = a.y; v[4 * i + 2] = a.z; v[4 * i + 3] = a.w;
+        }
+    }
+}
+
+template <int NW>
+__device__ __forceinline__ void store_words(int16_t* p, int d0, int Dr, const uint32_t (&v)[NW])
+{
+    if constexpr (NW == 2) {
+        *reinterpret_cast<uint2*>(p) = make_uint2(v[0], v[1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < NW / 4; ++i) {
+            if (d0 + 8 * i >= Dr) break;
+            reinterpret_cast<uint4*>(p)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
         }
     }
 }
@@ -259,6 +285,22 @@ __device__ __forceinline__ void seg_step(State<NW, T>& s, const uint32_t (&c)[NW
     s.mp2 = chain_min_dup<NW, T>(s.L);
 }
 
+// The block's adaptive-P2 table; returns whether an active chain's best may
+// reach SHRT_MAX.  It does only where minPrev + P2 does; path costs are at
+// most cost + P2, so with costs of at most cmax that takes cmax + 2 P2 >=
+// SHRT_MAX.
+__device__ __forceinline__ bool load_penalties(const LevelDesc& J, int* lut)
+{
+    const int side = imin(J.bs | 1, 127);
+    const int cmax = J.cost == COST_CENSUS ? 24 : imin(kMax, 255 * side * side);
+    bool high = cmax + 2 * imin(J.P2, kMax) >= kMax;
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+        lut[i] = J.adaptive ? J.p2lut[i] : 0;
+        high = high || cmax + 2 * imin(lut[i], kMax) >= kMax;
+    }
+    return high;
+}
+
 // What a walk needs beside its state.
 template <int NW, int T, int MODE>
 struct Ctx {
@@ -282,12 +324,13 @@ struct Ctx {
 // chains with `act` set are walked, the state of step t0 - 1 is in `s`, a
 // chain stops at the first step whose costs equal the stored ones; returns
 // whether it reached te without one.
-template <int NW, int T, int MODE, bool FIX>
+template <int NW, int T, int MODE, int KIND>
 __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>& s, int t0, int ts, int te, int nch,
                                          int segs, int b, int wch, bool act, uint32_t (&spec)[NW])
 {
     using G = Geo<NW, T>;
     constexpr int D = G::D;
+    constexpr bool FIX = KIND == kAgain, ADD = KIND == kAdd;
     const LevelDesc& J = X.J;
     const int lane = X.lane, k = X.k;
     const int Dr = labels_of<D>(J);
@@ -332,8 +375,12 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
             const int doff = G::PPX <= 32 ? 0 : 256 * (jj % (G::PPX > 32 ? G::PPX / 32 : 1));
             const bool in = kCH * ci_issue + dq < lim[i] && (kApart ? j < jmax : off0 + doff < Dr);
             const int16_t* p = src[i] + (kApart ? j * apart : (long long)dq * advD[i] + doff);
-            if (in && PG_IN(p - J.C, 8, (size_t)J.w * J.h * Dr, 5))
-                cp16s(dst0 + 4 * (slot * G::SLOTW + (kApart ? j * kStep : i) * G::CSTR + dq * (D / 2) + doff / 2), p);
+            const uint32_t dst =
+                dst0 + 4 * (slot * G::SLOTW + (kApart ? j * kStep : i) * G::CSTR + dq * (D / 2) + doff / 2);
+            if (in && PG_IN(p - J.C, 8, (size_t)J.w * J.h * Dr, 5)) {
+                cp16s(dst, p);
+                if (ADD) cp16s(dst + 4 * kSC * G::SLOTW, J.V + (p - J.C));
+            }
         }
 #pragma unroll
         for (int i = 0; i < kChains; ++i) src[i] += (long long)kCH * advD[i];
@@ -421,7 +468,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
         }
         pk::cp_wait<kSC - 1>();
         __syncwarp();
-        if constexpr (!FIX) {
+        if constexpr (KIND == kStore) {
             if (ci == wch) {
 #pragma unroll
                 for (int i = 0; i < NW; ++i) spec[i] = s.L[i];
@@ -447,17 +494,35 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
             seg_step<NW, T, MODE>(s, cc, at, p22, X.p12, X.win + (q & 1) * G::BUFW, k, X.guard);
             bool put = (unsigned)(t + q - ts) < span;
             if constexpr (FIX) put = put && act;
-            if (put && PG_IN(op - X.out, 2 * NW, (size_t)J.w * J.h * Dr, 6)) {
-                if constexpr (NW <= 4) {
-                    if (2 * NW * k < Dr) pk::stw<NW>(reinterpret_cast<uint32_t*>(op), s.L);
-                } else {
+            uint32_t res[NW];
 #pragma unroll
-                    for (int i = 0; i < NW / 4; ++i)
-                        if (2 * NW * k + 8 * i < Dr)
-                            reinterpret_cast<uint4*>(op)[i] =
-                                make_uint4(s.L[4 * i], s.L[4 * i + 1], s.L[4 * i + 2], s.L[4 * i + 3]);
+            for (int i = 0; i < NW; ++i) res[i] = s.L[i];
+            if constexpr (ADD) {
+                const int both = X.e.rl_n - 1 - 2 * (t + q);   // steps until the other direction gets here
+                uint32_t v[NW];
+                bool sum = J.paths >= 3 || (J.paths == 2 && both < 0);
+                pk::ldw<NW>(cin + kSC * G::SLOTW + q * (D / 2), v);
+                if (J.paths >= 2 && both <= 0 && both > -2 * kCH * kSC) {
+                    if (both == 0) {   // the same pixel: L->R first
+                        if (put && !(X.c & 1)) {
+#pragma unroll
+                            for (int i = 0; i < NW; ++i)
+                                if (sum) res[i] = pk::gcombine<MODE != kSingle>(v[i], res[i]);
+                            store_words<NW>(op, 2 * NW * k, Dr, res);
+                        }
+                        put = put && (X.c & 1);
+                        sum = true;
+                    }
+                    __syncwarp();
+                    if (put) load_words<NW>(op, 2 * NW * k, Dr, v);
+                }
+                if (sum) {
+#pragma unroll
+                    for (int i = 0; i < NW; ++i) res[i] = pk::gcombine<MODE != kSingle>(v[i], res[i]);
                 }
             }
+            if (put && PG_IN(op - X.out, imin(2 * NW, Dr - 2 * NW * k), (size_t)J.w * J.h * Dr, 6))
+                store_words<NW>(op, 2 * NW * k, Dr, res);
             op += ostep;
         }
         if constexpr (FIX) {
@@ -470,7 +535,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
             if (t + kCH <= te && mine == 0) act = false;
         }
         // segments followed by another hold whole chunks
-        if (segs > 1 && t + kCH == te && (!FIX || act)) {
+        if (!ADD && segs > 1 && t + kCH == te && (!FIX || act)) {
 #pragma unroll
             for (int i = 0; i < NW; ++i) X.edge[(b * 32 + lane) * NW + i] = s.L[i];
         }
@@ -495,7 +560,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
 // the following ones columns; `rows_too` 0 launches the columns alone (their
 // path costs are all that is written, into V).
 template <int NW, int T, int MODE, int NJ>
-__global__ void __launch_bounds__(sg::kMaxSeg * 32) k_seg(const __grid_constant__ Jobs<NJ> jobs, int rows_too, int warm)
+__global__ void __launch_bounds__(sg::max_seg<NW>() * 32) k_seg(const __grid_constant__ Jobs<NJ> jobs, int rows_too, int warm)
 {
     using namespace sg;
     using G = Geo<NW, T>;
@@ -512,15 +577,7 @@ __global__ void __launch_bounds__(sg::kMaxSeg * 32) k_seg(const __grid_constant_
     int* marked = reinterpret_cast<int*>(smem + 256);   // [segment][chain]: walk it (again)
     uint32_t* mine = smem + 256 + (kMaxSeg + 1) * 32 + b * warp_words<NW, T, MODE>();
     uint32_t* edge = smem + 256 + (kMaxSeg + 1) * 32 + segs * warp_words<NW, T, MODE>();
-    // An active chain's best reaches SHRT_MAX only where minPrev + P2 does;
-    // path costs are at most cost + P2, so with costs of at most cmax that
-    // takes cmax + 2 P2 >= SHRT_MAX.
-    const int cmax = J.cost == COST_CENSUS ? 24 : imin(kMax, 255 * imin(J.bs | 1, 127) * imin(J.bs | 1, 127));
-    bool high = cmax + 2 * imin(J.P2, kMax) >= kMax;
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-        lut[i] = J.adaptive ? J.p2lut[i] : 0;
-        high = high || cmax + 2 * imin(lut[i], kMax) >= kMax;
-    }
+    const bool high = load_penalties(J, lut);
     for (int i = lane; i < warp_words<NW, T, MODE>(); i += 32) mine[i] = kMax2;
     const bool guard = __syncthreads_or(high);
 
@@ -543,7 +600,7 @@ __global__ void __launch_bounds__(sg::kMaxSeg * 32) k_seg(const __grid_constant_
 #pragma unroll
     for (int i = 0; i < NW; ++i) s.L[i] = spec[i] = kMax2;
     s.mp2 = kMax2;
-    seg_walk<NW, T, MODE, false>(X, s, ts - wch * kCH, ts, te, wch + nch, segs, b, wch, true, spec);
+    seg_walk<NW, T, MODE, kStore>(X, s, ts - wch * kCH, ts, te, wch + nch, segs, b, wch, true, spec);
     if (segs == 1) return;
 
     const bool has = b > 0 && ts < te;
@@ -570,7 +627,7 @@ __global__ void __launch_bounds__(sg::kMaxSeg * 32) k_seg(const __grid_constant_
         marked[b * 32 + lane] = 0;
         if (!__syncthreads_or(go)) break;   // also: every start state has been read
         if (__any_sync(0xffffffffu, go)) {
-            const bool past = seg_walk<NW, T, MODE, true>(X, s, ts, ts, te, nch, segs, b, 0, go, spec);
+            const bool past = seg_walk<NW, T, MODE, kAgain>(X, s, ts, ts, te, nch, segs, b, 0, go, spec);
             if (past && X.k == 0) marked[(b + 1) * 32 + X.c] = 1;
         }
         __syncthreads();
@@ -587,13 +644,15 @@ __global__ void __launch_bounds__(sg::kMaxSeg * 32) k_seg(const __grid_constant_
 // second walks outlast what the first ones save (960x540: 38-40 us from 32
 // to 64 steps, 160x96: 42 us of a whole call at 32, 46 at 64).
 constexpr int kMinSeg = 40;
+constexpr int kMaxRefineLabels = 256;   // pyrsgm_compute_level takes no more on a refinement level
+constexpr size_t kSmemPerBlock = 227 * 1024;
 constexpr int kWarmSteps = 16;   // 0 to 32 measured within 5 % of each other, 64 10 % slower
 
-inline int segments_for(long long blocks, int n)
+inline int segments_for(long long blocks, int n, int most)
 {
     const long long per_sm = (blocks + sm_count() - 1) / sm_count();
     const long long want = std::max<long long>(1, 16 / std::max<long long>(1, per_sm));
-    return (int)std::max<long long>(1, std::min<long long>(std::min<long long>(want, sg::kMaxSeg), n / kMinSeg));
+    return (int)std::max<long long>(1, std::min<long long>(std::min<long long>(want, most), n / kMinSeg));
 }
 
 template <int NW, int T, int MODE, int NJ>
@@ -611,7 +670,8 @@ cudaError_t launch_seg_mode(const Jobs<NJ>& jobs, bool rows_too, cudaStream_t st
         n = std::max(n, rows_too ? std::max(d.w, d.h) : d.h);
     }
     if (grid == 0) return cudaSuccess;
-    const int segs = segments_for(blocks, n);
+    int segs = segments_for(blocks, n, sg::max_seg<NW>());
+    while (segs > 1 && sg::seg_smem<NW, T, MODE>(segs) > kSmemPerBlock) --segs;
     const size_t smem = sg::seg_smem<NW, T, MODE>(segs);
     const cudaError_t err =
         cudaFuncSetAttribute(k_seg<NW, T, MODE, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -642,18 +702,21 @@ cudaError_t launch_seg(const Jobs<NJ>& jobs, bool rows_too, cudaStream_t st)
     } else {
         int nref = 0;
         for (int i = 0; i < jobs.n; ++i) nref += jobs.d[i].refine != 0;
-        if (nref == jobs.n) return launch_seg_mode<NW, T, sg::kRefine, NJ>(jobs, rows_too, st);
         if (nref == 0) return launch_seg_mode<NW, T, sg::kCoarse, NJ>(jobs, rows_too, st);
-        Jobs<NJ> part;
-        for (int ref = 0; ref < 2; ++ref) {
-            part.n = 0;
-            for (int i = 0; i < jobs.n; ++i)
-                if ((jobs.d[i].refine != 0) == (ref != 0)) part.d[part.n++] = jobs.d[i];
-            const cudaError_t err = ref ? launch_seg_mode<NW, T, sg::kRefine, NJ>(part, rows_too, st)
-                                        : launch_seg_mode<NW, T, sg::kCoarse, NJ>(part, rows_too, st);
-            if (err != cudaSuccess) return err;
+        if constexpr (2 * NW * T <= kMaxRefineLabels) {
+            if (nref == jobs.n) return launch_seg_mode<NW, T, sg::kRefine, NJ>(jobs, rows_too, st);
+            Jobs<NJ> part;
+            for (int ref = 0; ref < 2; ++ref) {
+                part.n = 0;
+                for (int i = 0; i < jobs.n; ++i)
+                    if ((jobs.d[i].refine != 0) == (ref != 0)) part.d[part.n++] = jobs.d[i];
+                const cudaError_t err = ref ? launch_seg_mode<NW, T, sg::kRefine, NJ>(part, rows_too, st)
+                                            : launch_seg_mode<NW, T, sg::kCoarse, NJ>(part, rows_too, st);
+                if (err != cudaSuccess) return err;
+            }
+            return cudaSuccess;
         }
-        return cudaSuccess;
+        return cudaErrorInvalidValue;
     }
 }
 

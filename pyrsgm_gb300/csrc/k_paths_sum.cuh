@@ -1,0 +1,189 @@
+// k_paths_sum.cuh -- aggregation of the label counts that keep one path
+// volume (every multiple of 16 but 16, 32 and 64, up to 1024): the columns
+// write V (segmented, k_paths_seg.cuh), the rows of both directions add to
+// it, and the winner is read from it.  One volume and the costs are all the
+// memory such a level has; the sums move 16 bytes per label in all.
+#pragma once
+
+#include "k_paths_seg.cuh"
+
+namespace pg {
+
+// Rows of both directions added to V, for the label counts that keep one
+// path volume (every one but 16, 32 and 64): a warp walks both directions of
+// 16 / T rows in step.  10 bytes per label move (costs twice, V in and out
+// once per direction but the first without T->B), no pass needs the sums of
+// another, and the rows alone fill the GPU.
+template <int NW, int T, int MODE, int NJ>
+__global__ void __launch_bounds__(32) k_rowadd(const __grid_constant__ Jobs<NJ> jobs)
+{
+    using namespace sg;
+    using G = Geo<NW, T>;
+    const LevelDesc& J = jobs.d[blockIdx.y];
+    extern __shared__ __align__(16) uint32_t smem[];
+    const int lane = threadIdx.x, g0 = blockIdx.x * G::CPW;
+    if (g0 >= 2 * J.h) return;
+    const Extent<MODE> e(J);
+    int* lut = reinterpret_cast<int*>(smem);
+    uint32_t* mine = smem + 256;
+    const bool guard = __any_sync(0xffffffffu, load_penalties(J, lut));
+    for (int i = lane; i < warp_words<NW, T, MODE>(2); i += 32) mine[i] = kMax2;
+    __syncwarp();
+    const int k = lane % T;
+    Ctx<NW, T, MODE> X{J, lut, mine, mine + 2 * kSC * G::SLOTW + lane / T + NW * k * G::WST, nullptr, lane, lane / T, k,
+                       e, true, J.adaptive != 0, guard, g0, {}, J.V, pk::dup(imin(J.P1, 0x8000))};
+    X.w = walk_of<MODE>(J, e, true, g0 + X.c);
+    const int n = X.w.n, nch = (imax(e.lr_n, e.rl_n) + kCH - 1) / kCH;
+    State<NW, T> s;
+    uint32_t spec[NW];
+#pragma unroll
+    for (int i = 0; i < NW; ++i) s.L[i] = spec[i] = kMax2;
+    s.mp2 = kMax2;
+    seg_walk<NW, T, MODE, kAdd>(X, s, 0, 0, n > 0 ? n : -(1 << 30), nch, 1, 0, 0, true, spec);
+}
+
+// Winner-take-all over the sums in V.  G lanes read a pixel's labels, 16 R
+// each, and reduce; after G pixels every lane has one winner of its own, and
+// the rules and outputs run on full warps.
+template <int G, int R, bool PYR, int NJ>
+__global__ void __launch_bounds__(256) k_wta_sum(const __grid_constant__ Jobs<NJ> jobs)
+{
+    const LevelDesc& J = jobs.d[blockIdx.z];
+    const int W = J.w, D = J.D, lane = threadIdx.x & 31, gl = lane % G;
+    const int y = blockIdx.y * 8 + (threadIdx.x >> 5), x0 = blockIdx.x * 32;
+    if (x0 >= W || y >= J.h) return;
+    int xlo = 0, xhi = W;
+    if (!PYR) {
+        xlo = imax(J.minD + D, 0);
+        xhi = imin(W + imin(J.minD, 0), W - 1);   // the last column has no winner
+    }
+    const int16_t* row = J.V + (size_t)y * W * D;
+    unsigned myBest = 0;
+    int myAlt = 0;
+#pragma unroll 2
+    for (int i = 0; i < G; ++i) {
+        const int x = imin(x0 + lane - gl + i, W - 1);
+        uint32_t t[8 * R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int d0 = 16 * (gl + G * r);
+            uint4 a = make_uint4(pk::kMax2, pk::kMax2, pk::kMax2, pk::kMax2), b = a;
+            if (d0 < D) {
+                const uint4* p = reinterpret_cast<const uint4*>(row + (size_t)x * D + d0);
+                a = __ldg(p);
+                b = __ldg(p + 1);
+            }
+            t[8 * r] = a.x; t[8 * r + 1] = a.y; t[8 * r + 2] = a.z; t[8 * r + 3] = a.w;
+            t[8 * r + 4] = b.x; t[8 * r + 5] = b.y; t[8 * r + 6] = b.z; t[8 * r + 7] = b.w;
+        }
+        unsigned best = 0xffffffffu;
+#pragma unroll
+        for (int j = 0; j < 8 * R; ++j) {
+            const unsigned d = 16u * (gl + G * (j / 8)) + 2 * (j % 8);
+            best = __vimin3_u32(best, (t[j] << 16) | d, (t[j] & 0xffff0000u) | (d + 1));
+        }
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) best = umin(best, __shfl_xor_sync(0xffffffffu, best, o));
+        const int bd = (int)(best & 0xffffu);
+        unsigned far = kMax;
+#pragma unroll
+        for (int j = 0; j < 8 * R; ++j) {
+            const int d = 16 * (gl + G * (j / 8)) + 2 * (j % 8);
+            const unsigned u0 = (unsigned)(d - bd + 1) <= 2u ? (unsigned)kMax : (t[j] & 0xffffu);
+            const unsigned u1 = (unsigned)(d - bd + 2) <= 2u ? (unsigned)kMax : (t[j] >> 16);
+            far = __vimin3_u32(far, u0, u1);
+        }
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) far = umin(far, __shfl_xor_sync(0xffffffffu, far, o));
+        if (gl == i) {
+            myBest = best;
+            myAlt = (int)far;
+        }
+    }
+    const int x = x0 + lane;
+    if (x >= W) return;
+    const size_t p = (size_t)y * W + x;
+    if (x < xlo || x >= xhi) {
+        J.disp_raw[p] = (int16_t)((J.minD - 1) * 16);
+        J.conf_raw[p] = 0.0f;
+        return;
+    }
+    const int minCost = (int)(myBest >> 16), bd = (int)(myBest & 0xffffu);
+    const int c0 = bd > 0 ? (int)__ldg(row + (size_t)x * D + bd - 1) : 0;
+    const int c2 = bd + 1 < D ? (int)__ldg(row + (size_t)x * D + bd + 1) : 0;
+    const int base = (PYR && J.refine) ? (int)J.base[p] : J.minD;
+    pk::wta_out<PYR>(J, D, y, x, base, minCost, bd, myAlt, c0, minCost, c2);
+}
+
+template <int NW, int T, int MODE, int NJ>
+cudaError_t launch_rowadd_mode(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
+{
+    using G = sg::Geo<NW, T>;
+    constexpr size_t smem = sg::add_smem<NW, T, MODE>();
+    const cudaError_t err =
+        cudaFuncSetAttribute(k_rowadd<NW, T, MODE, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return err;
+    prof_begin(st);
+    k_rowadd<NW, T, MODE, NJ><<<dim3((2 * e.max_h + G::CPW - 1) / G::CPW, jobs.n), 32, smem, st>>>(jobs);
+    count_launch();
+    if (prof_enabled()) {
+        // each direction reads the cost volume; V is read (T->B or the first
+        // direction's sum) and written once per direction
+        double by = 0;
+        for (int i = 0; i < jobs.n; ++i) {
+            const LevelDesc& d = jobs.d[i];
+            const int dirs = d.paths >= 2 ? 2 : 1;
+            by += (double)d.w * d.h * (d.D * (4.0 * dirs + 2.0 * (dirs - 1) + (d.paths >= 3 ? 2 : 0)) +
+                                       dirs * ((d.refine ? 2 : 0) + (d.adaptive ? 1 : 0)));
+        }
+        prof_end(PK_PATH_ROW, by, st);
+    }
+    return launched(st, "k_rowadd");
+}
+
+// Columns into V, rows added to it, the winner from it.
+template <int NW, int T, int G, int R, bool PYR, int NJ>
+cudaError_t launch_sum(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
+{
+    cudaError_t err = launch_seg<NW, T, PYR, NJ>(jobs, false, st);
+    if (err != cudaSuccess) return err;
+    if constexpr (!PYR) {
+        err = launch_rowadd_mode<NW, T, sg::kSingle, NJ>(jobs, e, st);
+    } else {
+        Jobs<NJ> part;
+        for (int ref = 0; ref < 2 && err == cudaSuccess; ++ref) {
+            part.n = 0;
+            for (int i = 0; i < jobs.n; ++i)
+                if ((jobs.d[i].refine != 0) == (ref != 0)) part.d[part.n++] = jobs.d[i];
+            if (part.n == 0) continue;
+            if constexpr (2 * NW * T <= kMaxRefineLabels) {
+                err = ref ? launch_rowadd_mode<NW, T, sg::kRefine, NJ>(part, e, st)
+                          : launch_rowadd_mode<NW, T, sg::kCoarse, NJ>(part, e, st);
+            } else {
+                err = ref ? cudaErrorInvalidValue : launch_rowadd_mode<NW, T, sg::kCoarse, NJ>(part, e, st);
+            }
+        }
+    }
+    if (err != cudaSuccess) return err;
+    dim3 gw((e.max_w + 31) / 32, (e.max_h + 7) / 8, jobs.n);
+    prof_begin(st);
+    k_wta_sum<G, R, PYR, NJ><<<gw, 256, 0, st>>>(jobs);
+    count_launch();
+    prof_end(PK_WTA, jobs_vox(jobs) * 2 + jobs_px(jobs) * (2 + 6 + 4), st);
+    return launched(st, "k_wta_sum");
+}
+
+template <bool PYR, int NJ>
+cudaError_t launch_paths_sum(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
+{
+    switch (path_variant(jobs.d[0].D)) {
+    case 64: return launch_sum<4, 8, 4, 1, PYR, NJ>(jobs, e, st);
+    case 128: return launch_sum<4, 16, 8, 1, PYR, NJ>(jobs, e, st);
+    case 256: return launch_sum<8, 16, 16, 1, PYR, NJ>(jobs, e, st);
+    case 512: return launch_sum<16, 16, 32, 1, PYR, NJ>(jobs, e, st);
+    case 1024: return launch_sum<32, 16, 32, 2, PYR, NJ>(jobs, e, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace pg

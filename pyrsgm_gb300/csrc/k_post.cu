@@ -14,15 +14,6 @@ namespace pg {
 template <bool PYR, int NJ>
 cudaError_t launch_paths_mode(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st);
 
-PathShape path_shape(int D)
-{
-    if (D <= 16) return {16, 1};
-    if (D <= 32) return {32, 1};
-    int k = 2;
-    while (32 * k < D) k *= 2;
-    return {32, k};
-}
-
 template <int NJ>
 cudaError_t launch_paths(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
 {
@@ -64,10 +55,9 @@ __global__ void __launch_bounds__(256) k_post(const __grid_constant__ Jobs<NJ> j
     if (x0 >= J.w || y0 >= J.h) return;
     const int W = J.w, H = J.h;
     const int16_t inv = (int16_t)((J.minD - 1) * 16);
-    // Levels aggregated by the packed kernels leave the LR check to this
-    // pass (kernel_StrictPyramidLRCheck / kernel_PseudoLRCheck,
+    // The LR check (kernel_StrictPyramidLRCheck / kernel_PseudoLRCheck,
     // src/sgm_kernels.cu:825-889).
-    const bool check = uses_packed(J.D) && (J.post & POST_LRCHECK);
+    const bool check = (J.post & POST_LRCHECK) != 0;
     const bool med = (J.post & POST_MEDIAN) != 0;
     // The LR-checked disparities of the tile and its halo, staged in three
     // rounds so that each thread's loads are in flight together: its raw

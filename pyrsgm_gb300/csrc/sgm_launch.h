@@ -69,20 +69,15 @@ double jobs_vox(const Jobs<NJ>& j)
     return s;
 }
 
-// Aggregation kernel variant: G lanes per path chain, K labels per lane,
-// G*K >= D (padding labels behave as permanently invalid).
-struct PathShape {
-    int G, K;
-};
-PathShape path_shape(int D);
-// Kernel family of a label count: 10000 + D for the thread-per-chain packed
-// kernels, else G * 100 + K of the lane-parallel ones.  Jobs of one
-// aggregation launch share it.
+// Kernel family of a label count: 10000 + D for 16, 32 and 64 labels, which
+// keep a volume per path, else the labels a chain of the one-volume kernels
+// holds (64, 128, 256, 512, 1024).  Jobs of one aggregation launch share it.
 inline int path_variant(int D)
 {
     if (uses_packed(D)) return 10000 + D;
-    const PathShape s = path_shape(D);
-    return s.G * 100 + s.K;
+    int cap = 64;
+    while (cap < D) cap *= 2;
+    return cap;
 }
 
 // Multiprocessor count of the current device (cached per device).

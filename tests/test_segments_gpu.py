@@ -69,3 +69,33 @@ def test_coarse_level_segments_match_the_oracle(kind, w, h, D, cost, paths):
                                        (64, cases.BT, None), (16, cases.BT, 20000)])
 def test_refinement_segments_match_the_oracle(w, h, D, cost, P2):
     _check(cases._lvl("seg", w, h, D, cost, True, P2=P2, adaptive=P2 is None, seed=w))
+
+
+# Label counts that keep one path volume (k_paths_sum.cuh): the middle of a
+# row, where the two directions meet, at even and odd widths.
+@pytest.mark.parametrize("kind", ["band", "texture"])
+@pytest.mark.parametrize("w,h", [(301, 43), (190, 66)])
+@pytest.mark.parametrize("paths,minD", [(1, 0), (2, 0), (3, 0), (3, -9), (3, 5)])
+@pytest.mark.parametrize("D,cost", [(48, cases.CENSUS), (96, cases.BT), (128, cases.BT), (160, cases.CENSUS)])
+def test_one_volume_single_scale_matches_the_oracle(kind, w, h, paths, minD, D, cost):
+    case = cases._ss("sum", w, h, D, cost, paths=paths, minD=minD, adaptive=paths == 3)
+    case["pair"] = _images(kind, w, h)
+    _check(case)
+
+
+@pytest.mark.parametrize("w,h,D", [(700, 19, 272), (1100, 17, 512), (1100, 9, 1008), (1500, 130, 1024)])
+def test_one_volume_large_label_counts_match_the_oracle(w, h, D):
+    case = cases._ss("sum", w, h, D, cases.CENSUS)
+    case["pair"] = _images("texture", w, h)
+    _check(case)
+    case = cases._lvl("sum", w, h, D, cases.CENSUS, False, paths=3)
+    case["pair"] = _images("band", w, h)
+    _check(case)
+
+
+@pytest.mark.parametrize("refine", [False, True])
+@pytest.mark.parametrize("paths", [1, 2, 3])
+@pytest.mark.parametrize("w,h,D", [(301, 131, 48), (202, 57, 112), (330, 40, 256)])
+def test_one_volume_pyramid_levels_match_the_oracle(refine, paths, w, h, D):
+    _check(cases._lvl("sum", w, h, D, cases.BT if D == 48 else cases.CENSUS, refine, paths=paths, adaptive=paths != 2,
+                      maxD=min(w - 1, 2 * D), seed=w))
