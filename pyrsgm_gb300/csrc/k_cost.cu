@@ -401,6 +401,17 @@ __device__ __forceinline__ uint32_t bt_pixel_off(const uint4 l, const uint4 r)
     return __viaddmin_u16x2(m, m >> 18, kBtOffClamp);
 }
 
+__device__ __forceinline__ void tile_cp16(void* dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void tile_commit_wait()
+{
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------
 // BT coarse / single-scale cost: kernel_BTCost followed by kernel_BoxFilterH
 // and kernel_BoxFilterV (src/sgm_kernels.cu:139-239, 354-416), fused.  The
@@ -463,6 +474,186 @@ __global__ void __launch_bounds__(256) k_cost_bt_box(const __grid_constant__ Job
 }
 
 // ---------------------------------------------------------------------------
+// The same for windows of 3 to 7 pixels, whose sums cannot reach either
+// saturation point (49 * 255 < SHRT_MAX), so that they may be taken in any
+// grouping.  A block owns 64 (label, 32-column segment) units of 4 labels x
+// 8 window rows: db labels (16, 32, 48 or 64) by 32 * nseg columns, and walks
+// down a strip of rows, 8 window rows at a time:
+//   staging: the features of the 8 rows (cp.async); right pixel p of a row
+//            lies at [p & 3][p >> 2], so that the threads of a row, four
+//            pixels apart, read adjacent 16-byte words;
+//   phase 1: a thread per (row, 4 labels, segment) walks the 32 + 2 HW
+//            window columns; label d + 1 needs at a column the right feature
+//            that d needed one column before, so one left and one right
+//            feature are loaded per column for four costs; running sums of
+//            the last 2 HW + 1 costs, two labels per word (offset costs, see
+//            bt_pixel_off), go to a ring of 8 + 2 HW rows in shared memory;
+//   phase 2: a thread per (4 columns, 4 labels) keeps the running column
+//            sums in registers across the strip: adds a row, stores the
+//            costs, takes off the row 2 HW before.
+// About 16 instructions a label; arithmetic and the shared-memory pipe bound
+// it alike.  720p, 128 labels, 5x5: 884 us in k_cost_bt_box.
+// ---------------------------------------------------------------------------
+constexpr int kBsThreads = 128, kBsRows = 8, kBsSeg = 32;
+__host__ __device__ constexpr int bs_segments(int db) { return db <= 16 ? 4 : db <= 32 ? 2 : 1; }
+// staged features of one row: left, right (a multiple of 4)
+template <int HW>
+__host__ __device__ constexpr int bs_left(int db) { return kBsSeg * bs_segments(db) + 2 * HW; }
+template <int HW>
+__host__ __device__ constexpr int bs_right(int db) { return (bs_left<HW>(db) + db - 1 + 3) / 4 * 4; }
+template <int HW>
+__host__ __device__ constexpr size_t bs_smem(int db)
+{
+    return (size_t)(kBsRows + 2 * HW) * kBsSeg * bs_segments(db) * db * 2 +
+           (size_t)kBsRows * (bs_left<HW>(db) + bs_right<HW>(db)) * 16 + 256;   // (a turn reads past the window)
+}
+
+// A right feature whose cost against any left one is 255 (no difference of
+// its halves borrows): right pixels outside the image.
+__device__ __forceinline__ uint4 bt_outside() { return make_uint4(0x40004000u, 0u, 0x40004000u, 0u); }
+
+template <int HW, int NJ>
+__global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_constant__ Jobs<NJ> jobs, int strip)
+{
+    constexpr int RING = kBsRows + 2 * HW, SW = kBsSeg + 2 * HW;
+    constexpr int U = HW == 3 ? 12 : 4;   // columns per turn: a multiple of 4 right features and 2 HW costs kept
+    const LevelDesc& J = jobs.d[blockIdx.z];
+    const int W = J.w, H = J.h, D = J.D;
+    const int nblk = (D + 63) / 64, db = ((D + nblk - 1) / nblk + 15) / 16 * 16;
+    const int nseg = bs_segments(db), TX = kBsSeg * nseg, ntx = (W + TX - 1) / TX;
+    const int bd = blockIdx.x / ntx, x0 = (blockIdx.x - bd * ntx) * TX, y0 = blockIdx.y * strip;
+    const int d0 = bd * db;
+    if (d0 >= D || y0 >= H) return;
+    const int nd = imin(db, D - d0), DQ = nd / 4;   // labels and label quads of this block
+    extern __shared__ __align__(16) unsigned char smb[];
+    uint16_t* ring = reinterpret_cast<uint16_t*>(smb);                   // [RING][TX][db]
+    uint4* sl = reinterpret_cast<uint4*>(smb + (size_t)RING * TX * db * 2);   // [rows][nsl]
+    const int nsl = TX + 2 * HW, nsr = nsl + nd - 1, srs = (nsr + 3) / 4;
+    uint4* sr = sl + kBsRows * nsl;                                      // [rows][4][srs]
+    const int xrs = x0 - HW - (d0 + J.minD + nd - 1);                    // image column of right pixel 0
+    // no window column is clamped
+    const bool interior = x0 - HW >= 0 && x0 + TX - 1 + HW < W;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    // phase 1 unit
+    const int q = t % DQ, rs = t / DQ, r1 = rs % kBsRows, seg = rs / kBsRows;
+    const bool unit = seg < nseg;
+    // phase 2 items: columns xq + step * i, label quad q
+    const int step = kBsThreads / DQ, xq = rs;
+    constexpr int kItems = kBsSeg * 16 / kBsThreads;   // columns per thread at 16 quads per segment
+    const int items = t < step * DQ ? (TX - xq + step - 1) / step : 0;
+    const uint32_t off2 = (kBtOff * (uint32_t)((2 * HW + 1) * (2 * HW + 1))) * 0x10001u;
+    uint2 run[kItems];
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) run[i] = make_uint2(0u - off2, 0u - off2);
+    const int y1 = imin(y0 + strip, H);
+    const int nrow = y1 - y0 + 2 * HW;                 // window rows of the strip
+    auto stage = [&](int w0) {                         // a warp per row
+        for (int r = warp; r < imin(kBsRows, nrow - w0); r += kBsThreads / 32) {
+            const size_t grow = (size_t)iclamp(y0 - HW + w0 + r, 0, H - 1) * W;
+            for (int j = lane; j < nsl; j += 32)
+                tile_cp16(sl + r * nsl + j, J.featL + grow + iclamp(x0 - HW + j, 0, W - 1));
+            uint4* o = sr + (size_t)r * 4 * srs + (lane & 3) * srs + (lane >> 2);
+            for (int p = lane; p < nsr; p += 32, o += 8) {
+                const int xx = xrs + p;
+                if (xx >= 0 && xx < W) tile_cp16(o, J.featR + grow + xx);
+                else *o = bt_outside();
+            }
+        }
+    };
+    stage(0);
+    int slot = 0;                                      // ring row of window row w0
+    for (int w0 = 0; w0 < nrow; w0 += kBsRows) {
+        const int rows = imin(kBsRows, nrow - w0);
+        tile_commit_wait();
+        __syncthreads();
+        if (unit && r1 < rows) {
+            const uint4* lrow = sl + r1 * nsl + seg * kBsSeg;
+            const uint4* rrow = sr + r1 * 4 * srs;
+            const int wr = slot + r1 >= RING ? slot + r1 - RING : slot + r1;
+            uint16_t* out = ring + ((size_t)wr * TX + seg * kBsSeg) * db + 4 * q;
+            uint32_t h0[2 * HW], h1[2 * HW], s0 = 0, s1 = 0;
+#pragma unroll
+            for (int i = 0; i < 2 * HW; ++i) h0[i] = h1[i] = 0;
+            // add the four labels' costs of column j (u: its place in the turn)
+            auto column = [&](int j, int u, const uint32_t (&e)[4]) {
+                const uint32_t p0 = e[0] | (e[1] << 16), p1 = e[2] | (e[3] << 16);
+                s0 += p0;
+                s1 += p1;
+                if (j >= 2 * HW && j < SW)
+                    *reinterpret_cast<uint2*>(out + (size_t)(j - 2 * HW) * db) = make_uint2(s0, s1);
+                s0 -= h0[u % (2 * HW)];
+                s1 -= h1[u % (2 * HW)];
+                h0[u % (2 * HW)] = p0;
+                h1[u % (2 * HW)] = p1;
+            };
+            if (interior) {
+                // label d0 + 4 q + i needs right pixel top + j - i at window
+                // column j; top is 3 modulo 4
+                const int top = seg * kBsSeg + nd - 1 - 4 * q;
+                const uint4* rp = rrow + (top >> 2);
+                uint4 win[4];   // right pixel p at p & 3
+#pragma unroll
+                for (int i = 1; i < 4; ++i) win[(3 - i) & 3] = rp[((3 - i) & 3) * srs];
+#pragma unroll 1
+                for (int j0 = 0; j0 < SW; j0 += U) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const uint4 l = lrow[j0 + u];
+                        win[(3 + u) & 3] = rp[((3 + u) & 3) * srs + ((3 + u) >> 2)];
+                        uint32_t e[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) e[i] = bt_pixel_off(l, win[(3 + u - i) & 3]);
+                        column(j0 + u, u, e);
+                    }
+                    rp += U / 4;
+                }
+            } else {
+#pragma unroll 1
+                for (int j0 = 0; j0 < SW; j0 += 2 * HW) {
+#pragma unroll
+                    for (int u = 0; u < 2 * HW; ++u) {
+                        const int gx = iclamp(x0 - HW + seg * kBsSeg + j0 + u, 0, W - 1);
+                        const int p = gx - (d0 + J.minD + 4 * q) - xrs;
+                        const uint4 l = lrow[j0 + u];
+                        uint32_t e[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) e[i] = bt_pixel_off(l, rrow[((p - i) & 3) * srs + ((p - i) >> 2)]);
+                        column(j0 + u, u, e);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        if (w0 + kBsRows < nrow) stage(w0 + kBsRows);   // its copies run beside phase 2
+        int wr = slot, wo = slot + kBsRows >= RING ? slot + kBsRows - RING : slot + kBsRows;   // rows w, w - 2 HW
+        for (int r = 0; r < rows; ++r) {
+            const uint16_t* add = ring + ((size_t)wr * TX + xq) * db + 4 * q;
+            const uint16_t* sub = ring + ((size_t)wo * TX + xq) * db + 4 * q;
+            const int y = y0 + w0 + r - 2 * HW;
+            const bool full = w0 + r >= 2 * HW;
+            int16_t* out = J.C + ((size_t)(full ? y : 0) * W + x0 + xq) * D + d0 + 4 * q;
+#pragma unroll
+            for (int i = 0; i < kItems; ++i) {
+                if (i < items) {
+                    const uint2 a = *reinterpret_cast<const uint2*>(add + step * i * db);
+                    run[i].x += a.x;
+                    run[i].y += a.y;
+                    if (full) {
+                        if (x0 + xq + step * i < W) *reinterpret_cast<uint2*>(out + (size_t)(step * i) * D) = run[i];
+                        const uint2 b = *reinterpret_cast<const uint2*>(sub + step * i * db);
+                        run[i].x -= b.x;
+                        run[i].y -= b.y;
+                    }
+                }
+            }
+            wr = wr + 1 == RING ? 0 : wr + 1;
+            wo = wo + 1 == RING ? 0 : wo + 1;
+        }
+        slot = wr;
+    }
+}
+
+// ---------------------------------------------------------------------------
 // BT refine cost: kernel_BTWindowCostLocal, src/sgm_kernels.cu:1075-1110.
 // For label d of pixel p the reference sums, over the blockSize^2 window of
 // clamped pixels q, the BT cost of q at the real disparity base_p + d (255
@@ -501,17 +692,6 @@ constexpr int kTiSL = kTiX + 2 * kTiMaxHalf;        // staged left features per 
 constexpr int kTiSR = kTiSL + kTiRn - 1;            // staged right features per window row
 constexpr size_t kTiHs = (size_t)kTiRows * kTiX * kTiRs * 2;
 constexpr size_t kTiSmem = kTiHs + (size_t)kTiRows * (kTiSL + kTiSR) * 16;
-
-__device__ __forceinline__ void tile_cp16(void* dst, const void* src)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                 "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void tile_commit_wait()
-{
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
 
 // Sums along x, for a cluster of real disparities rmin .. rmin + rn - 1,
 // of every window row of the tile (see above).
@@ -805,6 +985,83 @@ cudaError_t launch_prepare(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStrea
     return launched(st, "k_features");
 }
 
+template <int HW, int NJ>
+cudaError_t launch_bt_strip(const Jobs<NJ>& jobs, cudaStream_t st)
+{
+    size_t smem = 0;
+    int gx = 0, max_h = 0;
+    long long tiles = 0;
+    for (int i = 0; i < jobs.n; ++i) {
+        const LevelDesc& d = jobs.d[i];
+        const int nblk = (d.D + 63) / 64, db = ((d.D + nblk - 1) / nblk + 15) / 16 * 16;
+        const int tx = kBsSeg * bs_segments(db), n = (d.w + tx - 1) / tx * nblk;
+        gx = std::max(gx, n);
+        max_h = std::max(max_h, d.h);
+        tiles += n;
+        smem = std::max(smem, bs_smem<HW>(db));
+    }
+    // strips of 8 k window rows: the k whose waves of blocks (3 per SM) take
+    // the fewest turns of 8 rows
+    int strip = 0;
+    long long best = 0;
+    for (int k = 2; k <= 16; ++k) {
+        const int rows = k * kBsRows - 2 * HW;
+        const long long blocks = tiles * ((max_h + rows - 1) / rows), slots = 3LL * sm_count();
+        const long long turns = (blocks + slots - 1) / slots * k;
+        if (strip == 0 || turns < best) {
+            strip = rows;
+            best = turns;
+        }
+    }
+    const cudaError_t err =
+        cudaFuncSetAttribute(k_cost_bt_strip<HW, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return err;
+    k_cost_bt_strip<HW, NJ><<<dim3(gx, (max_h + strip - 1) / strip, jobs.n), kBsThreads, smem, st>>>(jobs, strip);
+    return cudaGetLastError();
+}
+
+// BT cost of fixed disparities: by window size, 3 to 7 pixels in strips, any
+// other through k_cost_bt_box.
+template <int NJ>
+cudaError_t launch_bt_fixed(const Jobs<NJ>& jobs, cudaStream_t st)
+{
+    Jobs<NJ> part;
+    int launches = 0;
+    for (int half = 0; half <= 3; ++half) {
+        part.n = 0;
+        int maxHalf = 0, max_w = 0, max_h = 0, max_D = 0;
+        for (int i = 0; i < jobs.n; ++i) {
+            const LevelDesc& d = jobs.d[i];
+            const int h = d.bs / 2;
+            if ((h >= 1 && h <= 3 ? h : 0) != half) continue;
+            part.d[part.n++] = d;
+            maxHalf = std::max(maxHalf, h);
+            max_w = std::max(max_w, d.w);
+            max_h = std::max(max_h, d.h);
+            max_D = std::max(max_D, d.D);
+        }
+        if (part.n == 0) continue;
+        if (launches++ > 0) count_launch();   // launch_cost counts one
+        cudaError_t err = cudaSuccess;
+        if (half == 1) err = launch_bt_strip<1, NJ>(part, st);
+        else if (half == 2) err = launch_bt_strip<2, NJ>(part, st);
+        else if (half == 3) err = launch_bt_strip<3, NJ>(part, st);
+        else {
+            const int SW = kBxX + 2 * maxHalf, SH = kBxY + 2 * maxHalf;
+            const size_t smem = ((SH * SW * kBxD + 15) & ~15) + (size_t)SH * kBxX * kBxD * 2;
+            if (smem > 48 * 1024)
+                err = cudaFuncSetAttribute(k_cost_bt_box<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (err != cudaSuccess) return err;
+            const int nxt = (max_w + kBxX - 1) / kBxX;
+            dim3 g(nxt * ((max_D + kBxD - 1) / kBxD), (max_h + kBxY - 1) / kBxY, part.n);
+            k_cost_bt_box<NJ><<<g, 256, smem, st>>>(part, maxHalf, nxt);
+            err = cudaGetLastError();
+        }
+        if (err != cudaSuccess) return err;
+    }
+    return cudaSuccess;
+}
+
 // All jobs in `jobs` share the cost mode and the refine flag.
 template <int NJ>
 cudaError_t launch_cost(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
@@ -821,23 +1078,13 @@ cudaError_t launch_cost(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t
         dim3 g((e.max_w + kTiX - 1) / kTiX, (e.max_h + kTiY - 1) / kTiY, jobs.n);
         k_cost_bt_tiled<NJ><<<g, 256, kTiSmem, st>>>(jobs);
     } else {
-        int maxHalf = 0;
-        for (int j = 0; j < jobs.n; ++j) maxHalf = std::max(maxHalf, jobs.d[j].bs / 2);
-        const int SW = kBxX + 2 * maxHalf, SH = kBxY + 2 * maxHalf;
-        const size_t smem = ((SH * SW * kBxD + 15) & ~15) + (size_t)SH * kBxX * kBxD * 2;
-        if (smem > 48 * 1024) {
-            cudaError_t err = cudaFuncSetAttribute(k_cost_bt_box<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)smem);
-            if (err != cudaSuccess) return err;
-        }
-        const int nxt = (e.max_w + kBxX - 1) / kBxX;
-        dim3 g(nxt * ((e.max_D + kBxD - 1) / kBxD), (e.max_h + kBxY - 1) / kBxY, jobs.n);
-        k_cost_bt_box<NJ><<<g, 256, smem, st>>>(jobs, maxHalf, nxt);
+        const cudaError_t err = launch_bt_fixed(jobs, st);
+        if (err != cudaSuccess) return err;
     }
     count_launch();
     // write the int16 volume, read both views' features (and the label base)
     prof_end(PK_COST, jobs_vox(jobs) * 2 + jobs_px(jobs) * ((J0.cost == COST_CENSUS ? 8 : 32) + (J0.refine ? 2 : 0)), st);
-    return launched(st, J0.cost == COST_CENSUS ? "k_cost_census" : J0.refine ? "k_cost_bt_tiled" : "k_cost_bt_box");
+    return launched(st, J0.cost == COST_CENSUS ? "k_cost_census" : J0.refine ? "k_cost_bt_tiled" : "BT cost of fixed disparities");
 }
 
 #define PG_INST(NJ)                                                                          \
