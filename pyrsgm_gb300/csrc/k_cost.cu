@@ -10,8 +10,6 @@
 
 namespace pg {
 
-constexpr uint32_t kBtBias2 = 0x01000100u;   // 256 in each 16-bit half
-
 // ---------------------------------------------------------------------------
 // pyrDown: 5x5 [1 4 6 4 1]^2 / 256, BORDER_REFLECT_101, (sum+128)>>8.
 // Reference: src/pyrdown.cu:16-52.
@@ -105,8 +103,8 @@ __global__ void __launch_bounds__(256) k_pyrdown(const __grid_constant__ PyrDown
 // channels the half-sample interval [lo, hi] of dev_bt_channel_cost
 // (src/sgm_kernels.cu:1002-1028) with clamped neighbours.  Census pixels
 // store their 25-bit descriptor as one word per pixel; BT pixels store four
-// words of 16-bit pairs (gradient low half, intensity high half):
-// value + 256, value, lo + 256, hi — the operands of bt_pixel().
+// words of signed 16-bit pairs (gradient low half, intensity high half):
+// value, -value, lo, -hi -- the operands of bt_pixel().
 //
 // The view-0 blocks also start the level: every pixel's disp2 key is
 // cleared, and on refine levels the label base is derived from the parent
@@ -260,8 +258,8 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
                 uint32_t glo, ghi, ilo, ihi;
                 interval(gv, hl ? g[j] : gv, hr ? g[j + 2] : gv, glo, ghi);
                 interval(iv, hl ? (int)r2[j + 1] : iv, hr ? (int)r2[j + 3] : iv, ilo, ihi);
-                const uint32_t X = (uint32_t)gv | ((uint32_t)iv << 16), X0 = glo | (ilo << 16), X1 = ghi | (ihi << 16);
-                f[j] = make_uint4(X + kBtBias2, X, X0 + kBtBias2, X1);
+                auto pair = [](uint32_t g, uint32_t i) { return (g & 0xffffu) | (i << 16); };
+                f[j] = make_uint4(pair(gv, iv), pair(0u - gv, 0u - iv), pair(glo, ilo), pair(0u - ghi, 0u - ihi));
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j)
@@ -376,30 +374,20 @@ __global__ void __launch_bounds__(256) k_cost_census(const __grid_constant__ Job
 // BT cost of one (left pixel, right pixel) pair: dev_bt_pixel_cost,
 // src/sgm_kernels.cu:1030-1043, i.e. min(255, bt(gradient) + bt(intensity)
 // >> 2) with bt(u, v) = min(max(0, u - v.hi, v.lo - u), max(0, v - u.hi,
-// u.lo - v)), on both channels at once as 16-bit pairs.  The +256 bias in
-// the features keeps every difference positive (no borrow between halves)
-// and is the floor of the maxima, subtracted once at the end.
-__device__ __forceinline__ int bt_pixel(const uint4 l, const uint4 r)
+// u.lo - v)), on both channels at once as 16-bit pairs: the features hold
+// the negated operands, so each difference and maximum is one instruction.
+// Seven in all.
+__device__ __forceinline__ uint32_t bt_pixel(const uint4 l, const uint4 r)
 {
-    const uint32_t c0 = __vimax3_u16x2(kBtBias2, l.x - r.w, r.z - l.y);   // 256 + max(0, u - v.hi, v.lo - u)
-    const uint32_t c1 = __vimax3_u16x2(kBtBias2, r.x - l.w, l.z - r.y);   // 256 + max(0, v - u.hi, u.lo - v)
-    const uint32_t t = __vminu2(c0, c1) - kBtBias2;
-    return imin(255, (int)(t & 0xffffu) + (int)(t >> 18));
+    const uint32_t c0 = __viaddmax_s16x2(l.x, r.w, __viaddmax_s16x2(r.z, l.y, 0u));
+    const uint32_t c1 = __viaddmax_s16x2(r.x, l.w, __viaddmax_s16x2(l.z, r.y, 0u));
+    const uint32_t m = __vminu2(c0, c1);
+    return __viaddmin_u16x2(m, m >> 18, 255u);   // the high half comes out 0
 }
 
-// The same cost plus kBtOff, for the tiled window sums.  With m = min(c0, c1)
-// (256 + bt in each half), m >> 18 = 64 + (bt(intensity) >> 2) lies in the
-// low half alone, so one __viaddmin_u16x2 adds it to 256 + bt(gradient),
-// clamps at 255 + kBtOff and zeroes the high half.  Sums of these carry
-// kBtOff per term, taken off once per label.
-constexpr uint32_t kBtOff = 320, kBtOffClamp = 255 + kBtOff;
-__device__ __forceinline__ uint32_t bt_pixel_off(const uint4 l, const uint4 r)
-{
-    const uint32_t c0 = __vimax3_u16x2(kBtBias2, l.x - r.w, r.z - l.y);
-    const uint32_t c1 = __vimax3_u16x2(kBtBias2, r.x - l.w, l.z - r.y);
-    const uint32_t m = __vminu2(c0, c1);
-    return __viaddmin_u16x2(m, m >> 18, kBtOffClamp);
-}
+// A right feature whose cost against any left one is 255: right pixels
+// outside the image.
+__device__ __forceinline__ uint4 bt_outside() { return make_uint4(0x30003000u, 0u, 0x30003000u, 0u); }
 
 __device__ __forceinline__ void tile_cp16(void* dst, const void* src)
 {
@@ -444,7 +432,7 @@ __global__ void __launch_bounds__(256) k_cost_bt_box(const __grid_constant__ Job
         const int gy = iclamp(y0 - h + r, 0, H - 1), gx = iclamp(x0 - h + j, 0, W - 1);
         const int x2 = gx - (d0 + dd + J.minD);
         int v = 255;
-        if (x2 >= 0 && x2 < W) v = bt_pixel(J.featL[(size_t)gy * W + gx], J.featR[(size_t)gy * W + x2]);
+        if (x2 >= 0 && x2 < W) v = (int)bt_pixel(J.featL[(size_t)gy * W + gx], J.featR[(size_t)gy * W + x2]);
         bt[(r * SW + j) * kBxD + dd] = (uint8_t)v;
     }
     __syncthreads();
@@ -486,13 +474,16 @@ __global__ void __launch_bounds__(256) k_cost_bt_box(const __grid_constant__ Job
 //            window columns; label d + 1 needs at a column the right feature
 //            that d needed one column before, so one left and one right
 //            feature are loaded per column for four costs; running sums of
-//            the last 2 HW + 1 costs, two labels per word (offset costs, see
-//            bt_pixel_off), go to a ring of 8 + 2 HW rows in shared memory;
+//            the last 2 HW + 1 costs, two labels per word, go to shared
+//            memory;
 //   phase 2: a thread per (4 columns, 4 labels) keeps the running column
-//            sums in registers across the strip: adds a row, stores the
-//            costs, takes off the row 2 HW before.
-// About 16 instructions a label; arithmetic and the shared-memory pipe bound
-// it alike.  720p, 128 labels, 5x5: 884 us in k_cost_bt_box.
+//            sums and the last 2 HW rows of its sums in registers across the
+//            strip: adds a row, stores the costs, takes off the row 2 HW
+//            before.  The next rows' features are copied meanwhile.
+// The ALU pipe bounds it (half of its instructions): 133 us for 720p with
+// 128 labels and 5x5 windows (884 in k_cost_bt_box); four blocks per SM at
+// 128 registers were slower than three at 168 (153 us), and so were the old
+// rows' sums read back from shared memory (162 us).
 // ---------------------------------------------------------------------------
 constexpr int kBsThreads = 128, kBsRows = 8, kBsSeg = 32;
 __host__ __device__ constexpr int bs_segments(int db) { return db <= 16 ? 4 : db <= 32 ? 2 : 1; }
@@ -504,18 +495,14 @@ __host__ __device__ constexpr int bs_right(int db) { return (bs_left<HW>(db) + d
 template <int HW>
 __host__ __device__ constexpr size_t bs_smem(int db)
 {
-    return (size_t)(kBsRows + 2 * HW) * kBsSeg * bs_segments(db) * db * 2 +
+    return (size_t)kBsRows * kBsSeg * bs_segments(db) * db * 2 +
            (size_t)kBsRows * (bs_left<HW>(db) + bs_right<HW>(db)) * 16 + 256;   // (a turn reads past the window)
 }
-
-// A right feature whose cost against any left one is 255 (no difference of
-// its halves borrows): right pixels outside the image.
-__device__ __forceinline__ uint4 bt_outside() { return make_uint4(0x40004000u, 0u, 0x40004000u, 0u); }
 
 template <int HW, int NJ>
 __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_constant__ Jobs<NJ> jobs, int strip)
 {
-    constexpr int RING = kBsRows + 2 * HW, SW = kBsSeg + 2 * HW;
+    constexpr int SW = kBsSeg + 2 * HW;
     constexpr int U = HW == 3 ? 12 : 4;   // columns per turn: a multiple of 4 right features and 2 HW costs kept
     const LevelDesc& J = jobs.d[blockIdx.z];
     const int W = J.w, H = J.h, D = J.D;
@@ -526,8 +513,8 @@ __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_const
     if (d0 >= D || y0 >= H) return;
     const int nd = imin(db, D - d0), DQ = nd / 4;   // labels and label quads of this block
     extern __shared__ __align__(16) unsigned char smb[];
-    uint16_t* ring = reinterpret_cast<uint16_t*>(smb);                   // [RING][TX][db]
-    uint4* sl = reinterpret_cast<uint4*>(smb + (size_t)RING * TX * db * 2);   // [rows][nsl]
+    uint16_t* sums = reinterpret_cast<uint16_t*>(smb);                   // [rows][TX][db]
+    uint4* sl = reinterpret_cast<uint4*>(smb + (size_t)kBsRows * TX * db * 2);   // [rows][nsl]
     const int nsl = TX + 2 * HW, nsr = nsl + nd - 1, srs = (nsr + 3) / 4;
     uint4* sr = sl + kBsRows * nsl;                                      // [rows][4][srs]
     const int xrs = x0 - HW - (d0 + J.minD + nd - 1);                    // image column of right pixel 0
@@ -541,14 +528,17 @@ __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_const
     const int step = kBsThreads / DQ, xq = rs;
     constexpr int kItems = kBsSeg * 16 / kBsThreads;   // columns per thread at 16 quads per segment
     const int items = t < step * DQ ? (TX - xq + step - 1) / step : 0;
-    const uint32_t off2 = (kBtOff * (uint32_t)((2 * HW + 1) * (2 * HW + 1))) * 0x10001u;
-    uint2 run[kItems];
+    uint2 run[kItems], before[kItems][2 * HW];
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) run[i] = make_uint2(0u - off2, 0u - off2);
+    for (int i = 0; i < kItems; ++i) {
+        run[i] = make_uint2(0u, 0u);
+#pragma unroll
+        for (int k = 0; k < 2 * HW; ++k) before[i][k] = make_uint2(0u, 0u);
+    }
     const int y1 = imin(y0 + strip, H);
-    const int nrow = y1 - y0 + 2 * HW;                 // window rows of the strip
+    const int nrow = y1 - y0 + 2 * HW;                 // window rows of the strip; whole turns of 8 are walked
     auto stage = [&](int w0) {                         // a warp per row
-        for (int r = warp; r < imin(kBsRows, nrow - w0); r += kBsThreads / 32) {
+        for (int r = warp; r < kBsRows; r += kBsThreads / 32) {
             const size_t grow = (size_t)iclamp(y0 - HW + w0 + r, 0, H - 1) * W;
             for (int j = lane; j < nsl; j += 32)
                 tile_cp16(sl + r * nsl + j, J.featL + grow + iclamp(x0 - HW + j, 0, W - 1));
@@ -560,17 +550,15 @@ __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_const
             }
         }
     };
+    int16_t* orow = J.C + ((long long)(y0 - 2 * HW) * W + x0 + xq) * D + d0 + 4 * q;   // of window row w0
     stage(0);
-    int slot = 0;                                      // ring row of window row w0
     for (int w0 = 0; w0 < nrow; w0 += kBsRows) {
-        const int rows = imin(kBsRows, nrow - w0);
         tile_commit_wait();
         __syncthreads();
-        if (unit && r1 < rows) {
+        if (unit) {
             const uint4* lrow = sl + r1 * nsl + seg * kBsSeg;
             const uint4* rrow = sr + r1 * 4 * srs;
-            const int wr = slot + r1 >= RING ? slot + r1 - RING : slot + r1;
-            uint16_t* out = ring + ((size_t)wr * TX + seg * kBsSeg) * db + 4 * q;
+            uint16_t* out = sums + (r1 * TX + seg * kBsSeg) * db + 4 * q;
             uint32_t h0[2 * HW], h1[2 * HW], s0 = 0, s1 = 0;
 #pragma unroll
             for (int i = 0; i < 2 * HW; ++i) h0[i] = h1[i] = 0;
@@ -602,7 +590,7 @@ __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_const
                         win[(3 + u) & 3] = rp[((3 + u) & 3) * srs + ((3 + u) >> 2)];
                         uint32_t e[4];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) e[i] = bt_pixel_off(l, win[(3 + u - i) & 3]);
+                        for (int i = 0; i < 4; ++i) e[i] = bt_pixel(l, win[(3 + u - i) & 3]);
                         column(j0 + u, u, e);
                     }
                     rp += U / 4;
@@ -617,7 +605,7 @@ __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_const
                         const uint4 l = lrow[j0 + u];
                         uint32_t e[4];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) e[i] = bt_pixel_off(l, rrow[((p - i) & 3) * srs + ((p - i) >> 2)]);
+                        for (int i = 0; i < 4; ++i) e[i] = bt_pixel(l, rrow[((p - i) & 3) * srs + ((p - i) >> 2)]);
                         column(j0 + u, u, e);
                     }
                 }
@@ -625,31 +613,28 @@ __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_const
         }
         __syncthreads();
         if (w0 + kBsRows < nrow) stage(w0 + kBsRows);   // its copies run beside phase 2
-        int wr = slot, wo = slot + kBsRows >= RING ? slot + kBsRows - RING : slot + kBsRows;   // rows w, w - 2 HW
-        for (int r = 0; r < rows; ++r) {
-            const uint16_t* add = ring + ((size_t)wr * TX + xq) * db + 4 * q;
-            const uint16_t* sub = ring + ((size_t)wo * TX + xq) * db + 4 * q;
-            const int y = y0 + w0 + r - 2 * HW;
-            const bool full = w0 + r >= 2 * HW;
-            int16_t* out = J.C + ((size_t)(full ? y : 0) * W + x0 + xq) * D + d0 + 4 * q;
+        const uint16_t* add = sums + xq * db + 4 * q;
+#pragma unroll
+        for (int r = 0; r < kBsRows; ++r) {
+            const int wr = w0 + r;
+            const bool put = wr >= 2 * HW && wr < nrow;
 #pragma unroll
             for (int i = 0; i < kItems; ++i) {
                 if (i < items) {
-                    const uint2 a = *reinterpret_cast<const uint2*>(add + step * i * db);
+                    const uint2 a = *reinterpret_cast<const uint2*>(add + (r * TX + step * i) * db);
                     run[i].x += a.x;
                     run[i].y += a.y;
-                    if (full) {
-                        if (x0 + xq + step * i < W) *reinterpret_cast<uint2*>(out + (size_t)(step * i) * D) = run[i];
-                        const uint2 b = *reinterpret_cast<const uint2*>(sub + step * i * db);
-                        run[i].x -= b.x;
-                        run[i].y -= b.y;
-                    }
+                    if (put && x0 + xq + step * i < W)
+                        *reinterpret_cast<uint2*>(orow + (size_t)(step * i) * D) = run[i];
+                    run[i].x -= before[i][0].x;
+                    run[i].y -= before[i][0].y;
+#pragma unroll
+                    for (int k = 0; k + 1 < 2 * HW; ++k) before[i][k] = before[i][k + 1];
+                    before[i][2 * HW - 1] = a;
                 }
             }
-            wr = wr + 1 == RING ? 0 : wr + 1;
-            wo = wo + 1 == RING ? 0 : wo + 1;
+            orow += (size_t)W * D;
         }
-        slot = wr;
     }
 }
 
@@ -664,28 +649,28 @@ __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_const
 // its pixels need, [min base, max base + D - 1], span at most kTiRn:
 //   staging: the features of every window row of the tile (left: one per
 //            window column, clamped; right: the ones its disparities reach)
-//            are copied once into shared memory with cp.async;
-//   phase 1: the (window row, two adjacent real disparities) units of a
-//            half row of 16 output columns are numbered row-major and cut
-//            into groups of 32, one unit per lane, dealt to the 8 warps in
-//            turn; a lane walks its half row left to right and keeps the
-//            running sums of the last blockSize costs of both disparities
-//            (sums along x, into shared memory), loading each left and
-//            right feature once for the two.  A tile usually needs 17 real
-//            disparities, so numbering the units this way keeps nearly
-//            every lane busy;
-//   phase 2: a thread per pixel adds blockSize rows of those sums, two
-//            labels per 32-bit add, from its own real-disparity offset.
+//            are copied once into shared memory with cp.async, a warp per
+//            row; right pixels outside the image get a feature of cost 255;
+//   phase 1: the (window row, two adjacent real disparities) units are
+//            numbered row-major and cut into groups of 32, one unit per
+//            lane, dealt to the 8 warps in turn; a lane walks the window
+//            columns left to right and keeps the running sums of the last
+//            blockSize costs of both disparities (sums along x, into shared
+//            memory), loading each left and right feature once for the two.
+//            A tile usually needs 17 real disparities, so numbering the
+//            units this way keeps nearly every lane busy;
+//   phase 2: a thread per two vertical neighbours adds blockSize rows of
+//            those sums for each, two labels per 32-bit add, from their
+//            real-disparity offset.  The two have one parent and so one
+//            offset, and share all but two of their window rows.
 // Window sums are exact integers (at most 25 * 255 here, no intermediate
-// clamp in the reference); the terms carry kBtOff each (bt_pixel_off), at
-// most 25 * 575 per 16-bit half, removed after the column sums.  Tiles
-// whose parents disagree more widely are
-// split into two base clusters (a pass each); pixels in neither, or a
-// wider window, evaluate each window directly.
+// clamp in the reference).  Tiles whose parents disagree more widely take a
+// pass per cluster of bases; what is left after kTiClusters of them, wider
+// windows and more than kTiRn labels evaluate each window directly.
 // ---------------------------------------------------------------------------
 constexpr int kTiX = 32, kTiY = 16, kTiRn = 32, kTiMaxHalf = 2;
 constexpr int kTiWarps = 8;
-constexpr int kTiSeg = 16;                          // output columns of a half row
+constexpr int kTiClusters = 8;   // passes of a tile
 constexpr int kTiRows = kTiY + 2 * kTiMaxHalf;      // window rows at most
 constexpr int kTiRs = kTiRn + 2;   // halves per (row, column): 17 words, odd, so columns hit distinct banks
 constexpr int kTiSL = kTiX + 2 * kTiMaxHalf;        // staged left features per window row
@@ -700,91 +685,78 @@ __device__ __forceinline__ void bt_row_sums(const LevelDesc& J, uint16_t* hs, ui
                                             int rn, int warp, int lane)
 {
     constexpr int R = kTiY + 2 * HW;     // window rows
-    constexpr int SW = kTiSeg + 2 * HW;  // window columns of a half row
+    constexpr int SW = kTiX + 2 * HW;    // window columns
+    constexpr int Q = HW > 0 ? 2 * HW : 1;
     const int W = J.w, H = J.h;
     uint4* sl = st;                      // [R][kTiSL]  left, columns x0 - HW + j (clamped)
-    uint4* sr = st + kTiRows * kTiSL;    // [R][kTiSR]  right, columns xrs + k (inside the image only)
+    uint4* sr = st + kTiRows * kTiSL;    // [R][kTiSR]  right, columns xrs + k
     const int xrs = x0 - HW - (rmin + rn - 1);
-    const int nsl = kTiX + 2 * HW, nsr = nsl + rn - 1;
-    // staging (the block's threads, one pass of copies)
-    for (int i = threadIdx.x; i < R * nsl; i += blockDim.x) {
-        const int r = i / nsl, j = i - r * nsl;
-        const int gy = iclamp(y0 - HW + r, 0, H - 1);
-        tile_cp16(sl + r * kTiSL + j, J.featL + (size_t)gy * W + iclamp(x0 - HW + j, 0, W - 1));
-    }
-    for (int i = threadIdx.x; i < R * nsr; i += blockDim.x) {
-        const int r = i / nsr, k = i - r * nsr;
-        const int gy = iclamp(y0 - HW + r, 0, H - 1);
-        const int xx = xrs + k;
-        if (xx >= 0 && xx < W) tile_cp16(sr + r * kTiSR + k, J.featR + (size_t)gy * W + xx);
+    const int nsr = SW + rn - 1;
+    for (int r = warp; r < R; r += kTiWarps) {
+        const size_t grow = (size_t)iclamp(y0 - HW + r, 0, H - 1) * W;
+        for (int j = lane; j < SW; j += 32)
+            tile_cp16(sl + r * kTiSL + j, J.featL + grow + iclamp(x0 - HW + j, 0, W - 1));
+        for (int k = lane; k < nsr; k += 32) {
+            const int xx = xrs + k;
+            if (xx >= 0 && xx < W) tile_cp16(sr + r * kTiSR + k, J.featR + grow + xx);
+            else sr[r * kTiSR + k] = bt_outside();
+        }
     }
     tile_commit_wait();
     __syncthreads();
-    // every window column of the tile inside the image, and every right pixel too
-    const bool interior = x0 - HW >= 0 && x0 + kTiX - 1 + HW < W && xrs >= 0 && xrs + nsr - 1 < W;
-    // Units: (window row, real-disparity pair ri, ri + 1) of a half row,
-    // numbered row-major, one per lane.  Real disparity ri + 1 needs at
-    // window column j the right feature that ri needed at column j - 1, so
-    // a lane loads one left and one right feature per column for two sums
-    // and stores both as one word.  With rn odd the last pair's second
-    // half is past the cluster: computed, never read.
+    // no window column is clamped
+    const bool interior = x0 - HW >= 0 && x0 + kTiX - 1 + HW < W;
+    // Units: (window row, real-disparity pair ri, ri + 1), numbered
+    // row-major, one per lane.  Real disparity ri + 1 needs at window column
+    // j the right feature that ri needed at column j - 1, so a lane loads
+    // one left and one right feature per column for two sums and stores both
+    // as one word.  With rn odd the last pair's second half is past the
+    // cluster: computed, never read.
     const int rp = (rn + 1) >> 1;
     const int pairs = R * rp;
-    const int chunks = (pairs + 31) >> 5;
-    for (int u = warp; u < 2 * chunks; u += kTiWarps) {
-        const int seg = u & 1, f = (u >> 1) * 32 + lane;
+    for (int f0 = warp * 32; f0 < pairs; f0 += kTiWarps * 32) {
+        const int f = f0 + lane;
         const bool on = f < pairs;
         const int fr = on ? f : pairs - 1;
         const int row = fr / rp, ri = 2 * (fr - row * rp);
-        const int real = rmin + ri;
-        const int c0 = seg * kTiSeg;               // first window column of the half row (tile-relative)
-        const uint4* lrow = sl + row * kTiSL + c0;
+        const uint4* lrow = sl + row * kTiSL;
         const uint4* rrow = sr + row * kTiSR;
-        uint32_t* out = reinterpret_cast<uint32_t*>(hs + ((size_t)row * kTiX + c0) * kTiRs + ri);
-        auto walk = [&](auto inner) {
-            constexpr bool IN = decltype(inner)::value;
-            // right feature of window column j for ri: srl[j]; for ri + 1: srl[j - 1] (interior)
-            const uint4* srl = rrow + c0 - ri + rn - 1;
-            uint4 rprev = IN ? srl[-1] : make_uint4(0u, 0u, 0u, 0u);
-            uint32_t q0[2 * HW + 1], q1[2 * HW + 1];
+        uint32_t* out = reinterpret_cast<uint32_t*>(hs + (size_t)row * kTiX * kTiRs + ri);
+        uint32_t h[Q], s = 0;   // the last 2 HW costs; their sum
 #pragma unroll
-            for (int i = 0; i < 2 * HW + 1; ++i) q0[i] = q1[i] = 0;
-            uint32_t s0 = 0, s1 = 0;
+        for (int i = 0; i < Q; ++i) h[i] = 0;
+        auto column = [&](int j, int u, uint32_t e0, uint32_t e1) {
+            const uint32_t p = e0 | (e1 << 16);
+            s += p;
+            if (j >= 2 * HW && on) out[(j - 2 * HW) * (kTiRs / 2)] = s;
+            s -= HW > 0 ? h[u % Q] : p;
+            h[u % Q] = p;
+        };
+        if (interior) {
+            // right feature of window column j for ri: srl[j]; for ri + 1: srl[j - 1]
+            const uint4* srl = rrow - ri + rn - 1;
+            uint4 rprev = ri + 1 < rn ? srl[-1] : bt_outside();
+#pragma unroll 1
+            for (int j0 = 0; j0 < SW; j0 += 4) {
 #pragma unroll
-            for (int j = 0; j < SW; ++j) {
-                uint32_t e0, e1;   // costs + kBtOff at real disparities ri, ri + 1
-                if (IN) {
-                    const uint4 l = lrow[j], r = srl[j];
-                    e0 = bt_pixel_off(l, r);
-                    e1 = bt_pixel_off(l, rprev);
+                for (int u = 0; u < 4; ++u) {
+                    if (SW % 4 != 0 && j0 + u >= SW) break;
+                    const uint4 l = lrow[j0 + u], r = srl[j0 + u];
+                    column(j0 + u, u, bt_pixel(l, r), bt_pixel(l, rprev));
                     rprev = r;
-                } else {
-                    const int gx = iclamp(x0 - HW + c0 + j, 0, W - 1);
-                    const int x2 = gx - real, x3 = x2 - 1;
-                    const uint4 l = lrow[j];
-                    e0 = (x2 >= 0 && x2 < W) ? bt_pixel_off(l, rrow[x2 - xrs]) : kBtOffClamp;
-                    e1 = (x3 >= 0 && x3 < W) ? bt_pixel_off(l, rrow[x3 - xrs]) : kBtOffClamp;
-                }
-                s0 += e0;
-                s1 += e1;
-                if (j >= 2 * HW && on) out[(j - 2 * HW) * (kTiRs / 2)] = s0 | (s1 << 16);
-                if (HW > 0) {
-                    s0 -= q0[0];
-                    s1 -= q1[0];
-#pragma unroll
-                    for (int i = 0; i + 1 < 2 * HW; ++i) {
-                        q0[i] = q0[i + 1];
-                        q1[i] = q1[i + 1];
-                    }
-                    q0[2 * HW - 1 < 0 ? 0 : 2 * HW - 1] = e0;
-                    q1[2 * HW - 1 < 0 ? 0 : 2 * HW - 1] = e1;
-                } else {
-                    s0 = s1 = 0;
                 }
             }
-        };
-        if (interior) walk(std::true_type{});
-        else walk(std::false_type{});
+        } else {
+#pragma unroll 1
+            for (int j0 = 0; j0 < SW; j0 += Q) {
+#pragma unroll
+                for (int u = 0; u < Q; ++u) {
+                    const int k = iclamp(x0 - HW + j0 + u, 0, W - 1) - (rmin + ri) - xrs;
+                    const uint4 l = lrow[j0 + u];
+                    column(j0 + u, u, bt_pixel(l, rrow[k]), bt_pixel(l, rrow[imax(k - 1, 0)]));
+                }
+            }
+        }
     }
 }
 
@@ -799,13 +771,13 @@ __global__ void __launch_bounds__(256, 3) k_cost_bt_tiled(const __grid_constant_
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint4* stg = reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(hs) + kTiHs);
     __shared__ int wred[2][kTiWarps];
-    // a thread's two pixels: (x0 + lane, y0 + warp) and (x0 + lane, y0 + warp + 8)
+    // a thread's two pixels: (x0 + lane, y0 + 2 warp) and the one below
     const int x = x0 + lane;
     int yq[2], bq[2];
     bool inq[2], hasq[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        yq[i] = y0 + warp + 8 * i;
+        yq[i] = y0 + 2 * warp + i;
         inq[i] = x < W && yq[i] < H;
         bq[i] = inq[i] ? (int)J.base[(size_t)yq[i] * W + x] : (int)kNoParent;
         hasq[i] = inq[i] && bq[i] != kNoParent;
@@ -821,79 +793,111 @@ __global__ void __launch_bounds__(256, 3) k_cost_bt_tiled(const __grid_constant_
 #pragma unroll
         for (int i = 0; i < kTiWarps; ++i) { mn = imin(mn, wred[0][i]); mx = imax(mx, wred[1][i]); }
     };
-    // Real disparities the tile needs: [min base, max base + D - 1].  When
-    // they span more than kTiRn (a depth edge through the tile), the bases
-    // are split at the midpoint of their range into two clusters, each
-    // handled by its own pass when it fits.
-    int bmin, bmax;
-    block_minmax(hasq[0], hasq[1], bmin, bmax);
-    int ncl = 0, cut = INT_MAX;
-    int cmin[2] = {bmin, 0}, cmax[2] = {bmax, 0};
-    if (bmax != INT_MIN && h <= kTiMaxHalf) {
-        if (bmax + D - bmin <= kTiRn) {
-            ncl = 1;
-        } else {
-            cut = bmin + ((bmax - bmin) >> 1);
-            int a0, a1, b0, b1;
-            block_minmax(hasq[0] && bq[0] <= cut, hasq[1] && bq[1] <= cut, a0, a1);
-            block_minmax(hasq[0] && bq[0] > cut, hasq[1] && bq[1] > cut, b0, b1);
-            if (a1 + D - a0 <= kTiRn && b1 + D - b0 <= kTiRn) {
-                ncl = 2;
-                cmin[0] = a0; cmax[0] = a1; cmin[1] = b0; cmax[1] = b1;
-            }
-        }
-    }
     const bool vec = (D & 7) == 0;
-    for (int c = 0; c < ncl; ++c) {
-        const int rmin = cmin[c], rn = cmax[c] + D - cmin[c];
+    // Clusters of bases, lowest first: the pixels whose real disparities lie
+    // within kTiRn of the lowest one left.  11-26 % of the tiles of a 1080p
+    // scene hold a depth edge or a wild parent and need more than one; a
+    // pass costs less than the window sums of a few pixels, and two passes
+    // at most left 1-2 % of the pixels to those (a seventh of the kernel's
+    // instructions, in blocks that outlasted the others).
+    bool todo[2] = {hasq[0] && h <= kTiMaxHalf && D <= kTiRn, hasq[1] && h <= kTiMaxHalf && D <= kTiRn};
+    for (int c = 0; c < kTiClusters; ++c) {
+        int rmin, top;
+        block_minmax(todo[0], todo[1], rmin, top);
+        if (top == INT_MIN) break;
+        if (top + D - rmin > kTiRn) {
+            const int last = rmin + kTiRn - D;
+            int lowest;
+            block_minmax(todo[0] && bq[0] <= last, todo[1] && bq[1] <= last, lowest, top);
+        }
+        const int rn = top + D - rmin;
+        const bool mine[2] = {todo[0] && bq[0] <= top, todo[1] && bq[1] <= top};
         if (h == 2) bt_row_sums<2>(J, hs, stg, x0, y0, rmin, rn, warp, lane);
         else if (h == 1) bt_row_sums<1>(J, hs, stg, x0, y0, rmin, rn, warp, lane);
         else bt_row_sums<0>(J, hs, stg, x0, y0, rmin, rn, warp, lane);
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            if (!(hasq[i] && (ncl == 1 || (c == 0) == (bq[i] <= cut)))) continue;
-            const int ty = warp + 8 * i;
-            if (!PG_IN(((size_t)yq[i] * W + x) * D, D, (size_t)W * H * D, 11)) continue;
-            int lo, hi;
-            label_range(J, x, bq[i], lo, hi);
+        // packed pair sums of 2h+1 rows from offset ri0 = b - rmin (halves),
+        // 8 labels per chunk
+        auto put = [&](int i, int d0, const uint32_t (&acc)[5], uint32_t sh, int lo, int hi) {
             int16_t* out = J.C + ((size_t)yq[i] * W + x) * D;
-            // packed pair sums of 2h+1 rows from offset ri0 = b - rmin (halves), 8 labels per chunk;
-            // each half carries kBtOff per window pixel
-            const int ri0 = bq[i] - rmin;
-            const uint32_t sh = (uint32_t)(ri0 & 1) * 16;
-            const uint32_t off2 = (kBtOff * (uint32_t)((2 * h + 1) * (2 * h + 1))) * 0x10001u;
-            for (int d0 = 0; d0 < D; d0 += 8) {
-                uint32_t acc[5] = {0u, 0u, 0u, 0u, 0u};
-                for (int k = 0; k <= 2 * h; ++k) {
-                    const uint32_t* row =
-                        reinterpret_cast<const uint32_t*>(hs + ((ty + k) * kTiX + lane) * kTiRs) + ((ri0 + d0) >> 1);
+            if (!PG_IN(((size_t)yq[i] * W + x) * D, D, (size_t)W * H * D, 11)) return;
+            uint32_t w[4];
 #pragma unroll
-                    for (int j = 0; j < 5; ++j) acc[j] += row[j];
-                }
-                uint32_t w[4];
+            for (int q = 0; q < 4; ++q) w[q] = __funnelshift_r(acc[q], acc[q + 1], sh);
+            if (lo > d0 || hi < d0 + 7) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    w[q] = __funnelshift_r(acc[q], acc[q + 1], sh) - off2;
                     const int d = d0 + 2 * q;
                     if (d < lo || d > hi) w[q] = (w[q] & 0xffff0000u) | (uint32_t)kMax;
                     if (d + 1 < lo || d + 1 > hi) w[q] = (w[q] & 0xffffu) | ((uint32_t)kMax << 16);
                 }
-                if (vec) {
-                    reinterpret_cast<uint4*>(out + d0)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                } else {
-                    for (int q = 0; q < 8 && d0 + q < D; ++q)
-                        out[d0 + q] = (int16_t)((w[q >> 1] >> ((q & 1) * 16)) & 0xffffu);
+            }
+            if (vec) {
+                reinterpret_cast<uint4*>(out + d0)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            } else {
+                for (int q = 0; q < 8 && d0 + q < D; ++q)
+                    out[d0 + q] = (int16_t)((w[q >> 1] >> ((q & 1) * 16)) & 0xffffu);
+            }
+        };
+        auto rowsum = [&](int k, int col) {   // window row k, words from half `col`
+            return reinterpret_cast<const uint32_t*>(hs + (k * kTiX + lane) * kTiRs) + (col >> 1);
+        };
+        if (mine[0] && mine[1] && bq[0] == bq[1]) {
+            int lo, hi;
+            label_range(J, x, bq[0], lo, hi);
+            const int ri0 = bq[0] - rmin;
+            const uint32_t sh = (uint32_t)(ri0 & 1) * 16;
+            for (int d0 = 0; d0 < D; d0 += 8) {
+                uint32_t top[5], bot[5];
+                const uint32_t* r0 = rowsum(2 * warp, ri0 + d0);
+                const uint32_t* r1 = rowsum(2 * warp + 2 * h + 1, ri0 + d0);
+#pragma unroll
+                for (int j = 0; j < 5; ++j) {
+                    top[j] = r0[j];
+                    bot[j] = r1[j];
+                }
+                for (int k = 1; k <= 2 * h; ++k) {   // the rows both windows hold
+                    const uint32_t* row = rowsum(2 * warp + k, ri0 + d0);
+#pragma unroll
+                    for (int j = 0; j < 5; ++j) {
+                        const uint32_t v = row[j];
+                        top[j] += v;
+                        bot[j] += v;
+                    }
+                }
+                put(0, d0, top, sh, lo, hi);
+                put(1, d0, bot, sh, lo, hi);
+            }
+        } else {
+#pragma unroll 1
+            for (int i = 0; i < 2; ++i) {
+                if (!(i ? mine[1] : mine[0])) continue;
+                const int bb = i ? bq[1] : bq[0];
+                int lo, hi;
+                label_range(J, x, bb, lo, hi);
+                const uint32_t sh = (uint32_t)((bb - rmin) & 1) * 16;
+                for (int d0 = 0; d0 < D; d0 += 8) {
+                    uint32_t acc[5] = {0u, 0u, 0u, 0u, 0u};
+                    for (int k = 0; k <= 2 * h; ++k) {
+                        const uint32_t* row = rowsum(2 * warp + i + k, bb - rmin + d0);
+#pragma unroll
+                        for (int j = 0; j < 5; ++j) acc[j] += row[j];
+                    }
+                    if (i) put(1, d0, acc, sh, lo, hi);
+                    else put(0, d0, acc, sh, lo, hi);
                 }
             }
         }
-        __syncthreads();   // the next cluster's row sums overwrite hs
+        todo[0] = todo[0] && !mine[0];
+        todo[1] = todo[1] && !mine[1];
+        // (the next cluster's reductions come before its row sums overwrite hs)
     }
-    // direct window per pixel (no parent, or not in a cluster)
+    // direct window per pixel (no parent, or in no cluster)
 #pragma unroll 1
     for (int i = 0; i < 2; ++i) {
-        const bool in = i ? inq[1] : inq[0], has = i ? hasq[1] : hasq[0];
-        if (!in || (ncl > 0 && has)) continue;
+        const bool in = i ? inq[1] : inq[0], has = i ? hasq[1] : hasq[0], left = i ? todo[1] : todo[0];
+        const bool wide = h > kTiMaxHalf || D > kTiRn;   // no clusters at all
+        if (!in || (has && !left && !wide)) continue;
         const int y = i ? yq[1] : yq[0], b = i ? bq[1] : bq[0];
         int lo, hi;
         label_range(J, x, b, lo, hi);
@@ -911,7 +915,7 @@ __global__ void __launch_bounds__(256, 3) k_cost_bt_tiled(const __grid_constant_
 #pragma unroll
                         for (int q = 0; q < 8; ++q) {
                             const int x2 = gx - (b + d0 + q);
-                            sum[q] += (x2 >= 0 && x2 < W) ? bt_pixel(lf, __ldg(&rrow[x2])) : 255;
+                            sum[q] += (x2 >= 0 && x2 < W) ? (int)bt_pixel(lf, __ldg(&rrow[x2])) : 255;
                         }
                     }
                 }

@@ -5,8 +5,8 @@
 //   images            u8, caller-pitched (bytes)
 //   features          16 bytes per pixel and view: the census descriptor
 //                     (one word per pixel, dense) for the Census cost, or
-//                     the Birchfield-Tomasi operands (value + 256, value,
-//                     lo + 256, hi; gradient and intensity as 16-bit pairs)
+//                     the Birchfield-Tomasi operands (value, -value, lo,
+//                     -hi; gradient and intensity as signed 16-bit pairs)
 //   label base        int16 per pixel (refine levels); kNoParent marks pixels
 //                     whose parent was rejected (no valid label)
 //   cost volume C     int16 [y][x][D], d innermost
