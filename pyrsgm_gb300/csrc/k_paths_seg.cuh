@@ -69,13 +69,14 @@ struct Geo {
     static constexpr int NCOP = CPW * PPC / 32;
     // words of one chain's chunk: padded so that the reads of a step (T
     // lanes x NW words per chain) hit distinct banks
-    static constexpr int CSTR = kCH * D / 2 + (D == 16 ? 8 : D == 32 ? 16 : 0);
+    static constexpr int CSTR = kCH * D / 2 + (NW == 8 ? 4 : D == 16 ? 8 : D == 32 ? 16 : 0);
     static constexpr int SLOTW = CPW * CSTR;
     static constexpr int PADW = D / 2 + 1;   // guard words before label 0
     static constexpr int LENW = PADW + D + 2;
     // Word w of chain c lies at w * WST + c: the stride makes the windows of
     // a chain's lanes (NW words apart) fall into distinct banks.
-    static constexpr int WST = T == 2 ? 20 : T == 4 ? 10 : T == 8 ? 9 : CPW;
+    static constexpr int WST = NW == 8 ? (T == 2 ? 18 : T == 4 ? 9 : T == 8 ? 5 : CPW)
+                                       : (T == 2 ? 20 : T == 4 ? 10 : T == 8 ? 9 : CPW);
     static constexpr int BUFW = (LENW * WST + 3) / 4 * 4;   // (the rings between the windows stay 16-byte aligned)
     static constexpr int QL = kCH > T ? kCH / T : 1;   // pixels of a chunk a lane prepares
 };
@@ -301,6 +302,17 @@ __device__ __forceinline__ bool load_penalties(const LevelDesc& J, int* lut)
     return high;
 }
 
+// SHRT_MAX at the lane's labels (from d0 on) that label_range rules out for
+// pixel x of a coarse level.
+template <int NW>
+__device__ __forceinline__ void invalid_labels(int x, int minD, int maxD, int wLast, int d0, uint32_t (&mask)[NW])
+{
+    const int lo = imax(0, x - wLast - minD) - d0, hi = imin(maxD, x) - minD - d0;   // relative to d0
+#pragma unroll
+    for (int i = 0; i < NW; ++i)
+        mask[i] = (2 * i < lo || 2 * i > hi ? 0x7fffu : 0u) | (2 * i + 1 < lo || 2 * i + 1 > hi ? 0x7fff0000u : 0u);
+}
+
 // What a walk needs beside its state.
 template <int NW, int T, int MODE>
 struct Ctx {
@@ -334,6 +346,12 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
     const LevelDesc& J = X.J;
     const int lane = X.lane, k = X.k;
     const int Dr = labels_of<D>(J);
+    // the descriptor's fields that the loop reads, in registers
+    const int minD = J.minD, maxD = J.maxD, wLast = J.w - 1, paths = J.paths, rl_n = X.e.rl_n, P2 = J.P2;
+    const int16_t* const Bg = J.base;
+    const uint8_t* const Lg = J.left;
+    int16_t* const Vg = J.V;
+    const int16_t* const Cg = J.C;
     // Copies of a chunk: piece i = lane + 32 j of the warp's CPW * PPC.
     // Below 64 labels a lane copies one piece each of NCOP chains a fixed
     // number apart (of the same direction); from 64 on the chain of copy j
@@ -379,7 +397,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
                 dst0 + 4 * (slot * G::SLOTW + (kApart ? j * kStep : i) * G::CSTR + dq * (D / 2) + doff / 2);
             if (in && PG_IN(p - J.C, 8, (size_t)J.w * J.h * Dr, 5)) {
                 cp16s(dst, p);
-                if (ADD) cp16s(dst + 4 * kSC * G::SLOTW, J.V + (p - J.C));
+                if (ADD) cp16s(dst + 4 * kSC * G::SLOTW, Vg + (p - Cg));
             }
         }
 #pragma unroll
@@ -392,14 +410,14 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
     // misses L2 takes several chunks of steps, and nothing may touch the
     // loaded values before
     const bool need = MODE == kRefine || X.adaptive;
-    const uint32_t p2const = pk::dup(imin(J.P2, 0x7fff));
+    const uint32_t p2const = pk::dup(imin(P2, 0x7fff));
     const unsigned span = te > ts ? te - ts : 0;
     struct Pixel {
         uint32_t base, img;
     };
     auto load_pixel = [&](int t, Pixel& v) {
-        if (MODE == kRefine) v.base = (uint32_t)(uint16_t)__ldg(J.base + X.w.p0 + (long long)X.w.dp * t);
-        if (X.adaptive) v.img = __ldg(J.left + X.w.l0 + (long long)X.w.dl * t);
+        if (MODE == kRefine) v.base = (uint32_t)(uint16_t)__ldg(Bg + X.w.p0 + (long long)X.w.dp * t);
+        if (X.adaptive) v.img = __ldg(Lg + X.w.l0 + (long long)X.w.dl * t);
     };
     auto load_chunk = [&](int t, Pixel (&v)[G::QL]) {
 #pragma unroll
@@ -427,6 +445,9 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
 #pragma unroll
     for (int j = 0; j < kSC - 1; ++j) issue(j);
     int slot = 0, islot = kSC - 1;
+    uint32_t mask[NW];   // coarse: SHRT_MAX at the pixel's invalid labels (a column's are those of every pixel)
+#pragma unroll
+    for (int i = 0; i < NW; ++i) mask[i] = 0;
     for (int ci = 0; ci < nch; ++ci) {
         if (FIX && !__any_sync(0xffffffffu, act)) break;
         const int t = t0 + kCH * ci;
@@ -459,7 +480,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
             }
 #pragma unroll
             for (int i = 0; i < G::QL; ++i) {
-                int p2 = J.P2;
+                int p2 = P2;
                 if (X.adaptive) p2 = X.lut[abs((int)(cur[i] & 255u) - (int)(prev[i] & 255u))];
                 info[i] = (uint32_t)imin(p2, 0x7fff) << 16;
                 if (MODE == kRefine)
@@ -474,6 +495,13 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
                 for (int i = 0; i < NW; ++i) spec[i] = s.L[i];
             }
         }
+        // coarse levels: does a pixel of the chunk have an invalid label?
+        bool border = false;
+        if (MODE == kCoarse) {
+            const int xa = X.w.xs + X.w.dx * t, xb = xa + X.w.dx * (kCH - 1);
+            border = __any_sync(0xffffffffu, imin(maxD, imin(xa, xb)) - minD < Dr - 1 || imax(xa, xb) - wLast > minD);
+            if (border && (X.rows || ci == 0)) invalid_labels<NW>(xa, minD, maxD, wLast, 2 * NW * k, mask);
+        }
         const uint32_t* cin = X.ring + slot * G::SLOTW + X.c * G::CSTR + k * NW;
         slot = slot + 1 == kSC ? 0 : slot + 1;
 #pragma unroll
@@ -486,10 +514,10 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
                             : __shfl_sync(0xffffffffu, info[T < kCH ? q / T : 0], T < kCH ? q % T : q, T);
                 p22 = __byte_perm(at, 0, 0x3232);
             }
-            if (MODE == kCoarse) {
-                int lo, hi;
-                label_range(J, X.w.xs + X.w.dx * (t + q), J.minD, lo, hi);
-                pk::mask_labels<NW>(cc, lo, hi, k);
+            if (MODE == kCoarse && border) {
+                if (X.rows && q > 0) invalid_labels<NW>(X.w.xs + X.w.dx * (t + q), minD, maxD, wLast, 2 * NW * k, mask);
+#pragma unroll
+                for (int i = 0; i < NW; ++i) cc[i] |= mask[i];
             }
             seg_step<NW, T, MODE>(s, cc, at, p22, X.p12, X.win + (q & 1) * G::BUFW, k, X.guard);
             bool put = (unsigned)(t + q - ts) < span;
@@ -498,11 +526,11 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
 #pragma unroll
             for (int i = 0; i < NW; ++i) res[i] = s.L[i];
             if constexpr (ADD) {
-                const int both = X.e.rl_n - 1 - 2 * (t + q);   // steps until the other direction gets here
+                const int both = rl_n - 1 - 2 * (t + q);   // steps until the other direction gets here
                 uint32_t v[NW];
-                bool sum = J.paths >= 3 || (J.paths == 2 && both < 0);
+                bool sum = paths >= 3 || (paths == 2 && both < 0);
                 pk::ldw<NW>(cin + kSC * G::SLOTW + q * (D / 2), v);
-                if (J.paths >= 2 && both <= 0 && both > -2 * kCH * kSC) {
+                if (paths >= 2 && both <= 0 && both > -2 * kCH * kSC) {
                     if (both == 0) {   // the same pixel: L->R first
                         if (put && !(X.c & 1)) {
 #pragma unroll
@@ -640,10 +668,11 @@ __global__ void __launch_bounds__(sg::max_seg<NW>() * 32) k_seg(const __grid_con
 // steps: as many as keep every block resident at 16 warps per SM (128
 // registers a thread).  A segment more than that makes a second wave: 429
 // groups (2879x1987) took 215 us with 5 segments and 256 with 8, 255 groups
-// (1080p) 86 us with 7 and 106 with 9.  Below kMinSeg steps a segment the
-// second walks outlast what the first ones save (960x540: 38-40 us from 32
-// to 64 steps, 160x96: 42 us of a whole call at 32, 46 at 64).
-constexpr int kMinSeg = 40;
+// (1080p) 86 us with 7 and 106 with 9.  Short segments are walked again for
+// longer than they saved: 64 steps at least (2879x1987 pyramid: 1247 us a
+// call with 64, 1262 with 40, 1270 with 130), 40 for the first four segments
+// of small levels (160x96: 42 us a call, 46 at 64).
+constexpr int kMinSeg = 64, kMinSegSmall = 40;
 constexpr int kMaxRefineLabels = 256;   // pyrsgm_compute_level takes no more on a refinement level
 constexpr size_t kSmemPerBlock = 227 * 1024;
 constexpr int kWarmSteps = 16;   // 0 to 32 measured within 5 % of each other, 64 10 % slower
@@ -652,7 +681,8 @@ inline int segments_for(long long blocks, int n, int most)
 {
     const long long per_sm = (blocks + sm_count() - 1) / sm_count();
     const long long want = std::max<long long>(1, 16 / std::max<long long>(1, per_sm));
-    return (int)std::max<long long>(1, std::min<long long>(std::min<long long>(want, most), n / kMinSeg));
+    const long long fit = std::max(n / kMinSeg, std::min(4, n / kMinSegSmall));
+    return (int)std::max<long long>(1, std::min<long long>(std::min<long long>(want, most), fit));
 }
 
 template <int NW, int T, int MODE, int NJ>
