@@ -140,6 +140,20 @@ cudaError_t launch_paths_seg(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStr
     return err != cudaSuccess ? err : launch_wta<2 * NW * T, PYR, NJ>(jobs, e, st);
 }
 
+// 16 labels: four threads a chain while the launch has at most three such
+// groups of 8 chains per SM -- the step is shorter, and the lone walks that
+// follow the first ones with it (us, two threads against four: 480x270 34
+// and 24, 960x540 52 and 41, 1440x994 92 and 79) --, else two, which take
+// fewer instructions (1080p 86 and 95, 2879x1987 213 and 250).
+template <bool PYR, int NJ>
+cudaError_t launch_paths_seg16(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
+{
+    long long chains = 0;
+    for (int i = 0; i < jobs.n; ++i) chains += 2 * jobs.d[i].h + (jobs.d[i].paths >= 3 ? jobs.d[i].w : 0);
+    return chains <= 3LL * 8 * sm_count() ? launch_paths_seg<2, 4, PYR, NJ>(jobs, e, st)
+                                          : launch_paths_seg<4, 2, PYR, NJ>(jobs, e, st);
+}
+
 // Shape of the packed kernels for a launch: 8 (the wide shape, one thread
 // per 16 labels, whole chains) when the launch has rows enough for one such
 // warp per SM, else 2 (4 for 64 labels), the segmented shape.
@@ -218,7 +232,7 @@ cudaError_t launch_paths_mode(const Jobs<NJ>& jobs, const LevelExtent& e, cudaSt
                 if (nw == 8 && fused) return launch_paths_fused16<NJ>(jobs, e, st);
             }
             return nw == 8 ? launch_paths_wide<1, PYR, NJ>(jobs, e, st)
-                           : launch_paths_seg<4, 2, PYR, NJ>(jobs, e, st);
+                           : launch_paths_seg16<PYR, NJ>(jobs, e, st);
         };
         const int nw = packed_choice(key, rows, st, run, err);
         return err != cudaSuccess ? err : run(nw);

@@ -75,8 +75,9 @@ struct Geo {
     static constexpr int LENW = PADW + D + 2;
     // Word w of chain c lies at w * WST + c: the stride makes the windows of
     // a chain's lanes (NW words apart) fall into distinct banks.
-    static constexpr int WST = NW == 8 ? (T == 2 ? 18 : T == 4 ? 9 : T == 8 ? 5 : CPW)
-                                       : (T == 2 ? 20 : T == 4 ? 10 : T == 8 ? 9 : CPW);
+    static constexpr int WST = NW == 8   ? (T == 2 ? 18 : T == 4 ? 9 : T == 8 ? 5 : CPW)
+                               : NW == 2 ? 20
+                                         : (T == 2 ? 20 : T == 4 ? 10 : T == 8 ? 9 : CPW);
     static constexpr int BUFW = (LENW * WST + 3) / 4 * 4;   // (the rings between the windows stay 16-byte aligned)
     static constexpr int QL = kCH > T ? kCH / T : 1;   // pixels of a chunk a lane prepares
 };
