@@ -6,13 +6,17 @@
 // of at most max_speckle_size pixels is set to new_val.
 //
 // GPU form: connected components by lock-free union-find (roots linked
-// larger index -> smaller with atomicCAS): first inside each 32x8 tile in
-// shared memory, each pixel linking its right and lower neighbour, which
-// leaves every pixel pointing at its tile-local root; then across tile
-// borders in global memory; then root sizes (atomicAdd, one per distinct
-// root and warp) and one pass that clears small regions.  The partition into
-// regions is unique, so the output is exactly that of a sequential flood
-// fill.
+// larger index -> smaller with atomicCAS).  Inside a 32x32 tile a row's runs
+// are found with one ballot, so that a pixel starts at its run's first one,
+// and a link to the row above is needed only where the pixel to the left
+// has not made it already (on a disparity map, at few pixels); the tile
+// leaves every pixel pointing at its tile-local root, and that root's size.
+// Then the same across tile borders in global memory (a sixteenth of the
+// pixels), the sizes of the tile roots added to their global roots, and one
+// pass that clears small regions.  The partition into regions is unique, so
+// the output is exactly that of a sequential flood fill.
+// Bound by the dependent walks of the four launches, not by the 30 bytes a
+// pixel they move.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -64,90 +68,116 @@ struct SpArgs {
     int* size;
 };
 
-__device__ __forceinline__ short sp_at(const SpArgs& A, int x, int y) { return A.d[(size_t)y * A.pitch + x]; }
+__device__ __forceinline__ int sp_at(const SpArgs& A, int x, int y) { return A.d[(size_t)y * A.pitch + x]; }
+__device__ __forceinline__ bool sp_joined(const SpArgs& A, int u, int v)
+{
+    return u != A.new_val && v != A.new_val && abs(u - v) <= A.max_diff;
+}
 
-// Tile pass: components inside one 32x8 tile (shared-memory union-find),
-// then every pixel's global label is its tile-local root's pixel index.
+constexpr int kSpTile = 32, kSpRows = 4;   // tile side; rows of it per warp
+
+// First pixel of a lane's run: the highest clear bit at or below the lane.
+__device__ __forceinline__ int sp_first(unsigned runs, int lane)
+{
+    return 31 - __clz(~runs & (0xffffffffu >> (31 - lane)));
+}
+
+// Tile pass (see above): lab[p] = index of p's tile-local root, size[p] = its
+// pixels in the tile at the root, 0 elsewhere.
 __global__ void __launch_bounds__(256) k_sp_tile(const SpArgs A)
 {
-    __shared__ int lab[256];
-    __shared__ short val[256];
-    const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
-    const int x = blockIdx.x * 32 + tx, y = blockIdx.y * 8 + ty;
-    const bool in = x < A.w && y < A.h;
-    const short v = in ? sp_at(A, x, y) : (short)A.new_val;
-    val[t] = v;
-    lab[t] = v != A.new_val ? t : -1;
-    __syncthreads();
-    if (v != A.new_val) {
-        if (tx + 1 < 32) {
-            const short u = val[t + 1];
-            if (u != A.new_val && abs(u - v) <= A.max_diff) sp_union(lab, t, t + 1, 256);
-        }
-        if (ty + 1 < 8) {
-            const short u = val[t + 32];
-            if (u != A.new_val && abs(u - v) <= A.max_diff) sp_union(lab, t, t + 32, 256);
-        }
+    __shared__ int lab[kSpTile * kSpTile], cnt[kSpTile * kSpTile];
+    __shared__ short val[kSpTile * kSpTile];
+    __shared__ unsigned runs[kSpTile];   // bit x: pixel x continues the run of pixel x - 1
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x = blockIdx.x * kSpTile + lane, y0 = blockIdx.y * kSpTile + warp * kSpRows;
+#pragma unroll
+    for (int k = 0; k < kSpRows; ++k) {
+        const int row = warp * kSpRows + k, i = row * kSpTile + lane, y = y0 + k;
+        const int v = x < A.w && y < A.h ? sp_at(A, x, y) : A.new_val;
+        const int left = __shfl_up_sync(0xffffffffu, v, 1);
+        const bool on = lane > 0 && sp_joined(A, left, v);
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) runs[row] = m;
+        val[i] = (short)v;
+        if (!on) lab[i] = i;   // only the first pixels of runs have a label here
+        cnt[i] = 0;
     }
     __syncthreads();
-    if (!in) return;
-    const int p = y * A.w + x;
-    A.size[p] = 0;
-    if (v == A.new_val) {
-        A.lab[p] = -1;
-        return;
+#pragma unroll
+    for (int k = 0; k < kSpRows; ++k) {
+        const int row = warp * kSpRows + k, i = row * kSpTile + lane;
+        const bool up = row > 0 && sp_joined(A, row > 0 ? val[i - kSpTile] : A.new_val, val[i]);
+        const unsigned ups = __ballot_sync(0xffffffffu, up);
+        // left neighbour joined to this pixel and to its own upper one, that one to ours
+        const unsigned made = runs[row] & (row > 0 ? runs[row - 1] : 0u) & (ups << 1);
+        if (up && !((made >> lane) & 1u))
+            sp_union(lab, row * kSpTile + sp_first(runs[row], lane), (row - 1) * kSpTile + sp_first(runs[row - 1], lane),
+                     kSpTile * kSpTile);
     }
-    const int r = sp_find(lab, t);
-    A.lab[p] = (blockIdx.y * 8 + (r >> 5)) * A.w + blockIdx.x * 32 + (r & 31);
+    __syncthreads();
+    int root[kSpRows];
+#pragma unroll
+    for (int k = 0; k < kSpRows; ++k) {
+        const int row = warp * kSpRows + k, i = row * kSpTile + lane;
+        const unsigned m = runs[row];
+        int r = -1;
+        if (!((m >> lane) & 1u) && val[i] != A.new_val) {   // a run's first pixel finds its root and counts it
+            r = sp_find(lab, i);
+            const unsigned ends = ~m >> lane >> 1;           // clear bits after the lane: the next run
+            atomicAdd(&cnt[r], ends ? __ffs(ends) : 32 - lane);
+        }
+        root[k] = __shfl_sync(0xffffffffu, r, sp_first(m, lane));
+    }
+    __syncthreads();
+    if (x >= A.w) return;
+#pragma unroll
+    for (int k = 0; k < kSpRows; ++k) {
+        const int i = (warp * kSpRows + k) * kSpTile + lane, y = y0 + k;
+        if (y >= A.h) break;
+        const int p = y * A.w + x, r = root[k];
+        A.size[p] = r == i ? cnt[i] : 0;
+        A.lab[p] = r < 0 ? -1 : (blockIdx.y * kSpTile + r / kSpTile) * A.w + blockIdx.x * kSpTile + r % kSpTile;
+    }
 }
 
-// Border pass: links across the right and lower edges of the tiles.
-__global__ void k_sp_link(const SpArgs A)
+// Border pass: links across the left edges of the tiles (thread i < nv: edge
+// i / h, row i % h), then across their upper ones.
+__global__ void __launch_bounds__(256) k_sp_link(const SpArgs A, int nv, int nh)
 {
-    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
-    if (x >= A.w || y >= A.h) return;
-    const bool right = (x & 31) == 31 && x + 1 < A.w, down = (y & 7) == 7 && y + 1 < A.h;
-    if (!right && !down) return;
-    const int v = sp_at(A, x, y);
-    if (v == A.new_val) return;
-    const int p = y * A.w + x, n = A.w * A.h;
-    if (right) {
-        const int u = sp_at(A, x + 1, y);
-        if (u != A.new_val && abs(u - v) <= A.max_diff) sp_union(A.lab, p, p + 1, n);
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= nv + nh) return;
+    const bool side = i < nv;
+    const int e = side ? i : i - nv, len = side ? A.h : A.w;
+    const int x = side ? (e / len + 1) * kSpTile : e % len, y = side ? e % len : (e / len + 1) * kSpTile;
+    const int dx = side ? 1 : 0, dy = side ? 0 : 1;     // towards the other tile: (x - dx, y - dy)
+    const int v = sp_at(A, x, y), u = sp_at(A, x - dx, y - dy);
+    if (!sp_joined(A, u, v)) return;
+    // the pair before along the edge, in the same two tiles, has made it?
+    if ((side ? y : x) % kSpTile != 0) {
+        const int v1 = sp_at(A, x - dy, y - dx), u1 = sp_at(A, x - dx - dy, y - dy - dx);
+        if (sp_joined(A, u1, v1) && sp_joined(A, v1, v) && sp_joined(A, u1, u)) return;
     }
-    if (down) {
-        const int u = sp_at(A, x, y + 1);
-        if (u != A.new_val && abs(u - v) <= A.max_diff) sp_union(A.lab, p, p + A.w, n);
-    }
+    sp_union(A.lab, y * A.w + x, (y - dy) * A.w + x - dx, A.w * A.h);
 }
 
+// The tile roots' sizes to their global roots.
 __global__ void __launch_bounds__(256) k_sp_count(const SpArgs A)
 {
-    const int lane = threadIdx.x & 31;
-    const int x = blockIdx.x * 32 + lane, y = blockIdx.y * 8 + (threadIdx.x >> 5);
-    int r = -1 - lane;   // outside the image or new_val: a key no other lane has
-    if (x < A.w && y < A.h) {
-        const int p = y * A.w + x;
-        if (A.lab[p] >= 0) {
-            r = sp_find(A.lab, p);
-            A.lab[p] = r;
-        }
-    }
-    // one atomic per distinct root in the warp (a large region's pixels
-    // would otherwise queue on a single counter); all 32 lanes take part
-    const unsigned peers = __match_any_sync(0xffffffffu, r);
-    if (r >= 0 && lane == __ffs(peers) - 1) atomicAdd(&A.size[r], __popc(peers));
+    const long long p = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (p >= (long long)A.w * A.h) return;
+    const int n = A.size[p];
+    if (n == 0 || A.lab[p] == (int)p) return;   // (a global root's own pixels are counted)
+    atomicAdd(&A.size[sp_find(A.lab, (int)p)], n);
 }
 
-__global__ void k_sp_apply(const SpArgs A)
+__global__ void __launch_bounds__(256) k_sp_apply(const SpArgs A)
 {
     const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
     if (x >= A.w || y >= A.h) return;
-    const int p = y * A.w + x;
-    if (A.lab[p] < 0) return;
-    // the root again: path halving by other threads of the count pass may
-    // have pointed lab[p] at an ancestor after its own thread stored the root
-    const int r = sp_find(A.lab, p);
+    int r = A.lab[y * A.w + x];
+    if (r < 0) return;
+    for (int q = A.lab[r]; q != r; q = A.lab[r]) r = q;
     if (A.size[r] <= A.max_size) A.d[(size_t)y * A.pitch + x] = (short)A.new_val;
 }
 
@@ -169,22 +199,28 @@ extern "C" int pyrsgm_gb300_filter_speckles(short* d_disp, size_t pitch_bytes, i
     }
     pg::SpArgs A{d_disp, pitch_bytes / sizeof(short), width, height, new_val, max_speckle_size, max_diff,
                  static_cast<int*>(scratch), static_cast<int*>(scratch) + n};
-    const dim3 g((width + 31) / 32, (height + 7) / 8);
+    const int tx = (width + pg::kSpTile - 1) / pg::kSpTile, ty = (height + pg::kSpTile - 1) / pg::kSpTile;
+    const int nv = (tx - 1) * height, nh = (ty - 1) * width;   // border pixels: left edges, upper edges
     cudaError_t e;
-    pg::k_sp_tile<<<g, 256, 0, stream>>>(A);
-    if ((e = pg::launched(stream, "k_sp_tile")) == cudaSuccess) {
-        pg::k_sp_link<<<g, 256, 0, stream>>>(A);
+    int launches = 3;
+    pg::k_sp_tile<<<dim3(tx, ty), 256, 0, stream>>>(A);
+    e = pg::launched(stream, "k_sp_tile");
+    if (e == cudaSuccess && nv + nh > 0) {
+        pg::k_sp_link<<<(nv + nh + 255) / 256, 256, 0, stream>>>(A, nv, nh);
         e = pg::launched(stream, "k_sp_link");
+        ++launches;
+        if (e == cudaSuccess) {
+            pg::k_sp_count<<<(int)((n + 255) / 256), 256, 0, stream>>>(A);
+            e = pg::launched(stream, "k_sp_count");
+        }
+    } else {
+        --launches;   // one tile: its sizes are final
     }
     if (e == cudaSuccess) {
-        pg::k_sp_count<<<g, 256, 0, stream>>>(A);
-        e = pg::launched(stream, "k_sp_count");
-    }
-    if (e == cudaSuccess) {
-        pg::k_sp_apply<<<g, 256, 0, stream>>>(A);
+        pg::k_sp_apply<<<dim3((width + 31) / 32, (height + 7) / 8), 256, 0, stream>>>(A);
         e = pg::launched(stream, "k_sp_apply");
     }
-    pg::count_launches(4);
+    pg::count_launches(launches);
     cudaFreeAsync(scratch, stream);
     return e == cudaSuccess ? 0 : -1;
 }

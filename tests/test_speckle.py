@@ -82,3 +82,33 @@ def test_gpu_speckle_filter_large_and_extreme_maps(kind):
     pg.filter_speckles(d, INV, max_size, max_diff)
     torch.cuda.synchronize()
     np.testing.assert_array_equal(d.cpu().numpy(), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,w", [(1, 1), (1, 70), (70, 1), (32, 32), (33, 32), (32, 65), (31, 97), (129, 63)])
+@pytest.mark.parametrize("kind", ["blocky", "comb", "spiral", "flat"])
+def test_tile_edges_match_the_flood_fill(h, w, kind):
+    """Sizes at the edges of the 32x32 tiles; combs and a spiral wind one
+    region through every tile, so that links and sizes travel far."""
+    import torch
+    import pyrsgm_gb300 as pg
+    img = np.full((h, w), 160, np.int16)
+    if kind == "blocky":
+        img = _blocky(h, w, h * 100 + w)
+    elif kind == "comb":
+        img[1::2, :] = INV
+        img[:, w // 2] = 160
+        img[h // 2:, 0] = INV
+    elif kind == "spiral":
+        y, x = np.mgrid[0:h, 0:w]
+        ring = np.minimum(np.minimum(x, w - 1 - x), np.minimum(y, h - 1 - y))
+        img[ring % 2 == 1] = INV
+        for r in range(0, min(h, w) // 2, 2):
+            if r + 1 < h and r < w:
+                img[min(r + 1, h - 1), min(r + 1, w - 1)] = 160
+    for max_size in (1, 40, 700):
+        want = _oracle.orc_speckles(img, INV, max_size, 8)
+        d = torch.from_numpy(img.copy()).cuda()
+        pg.filter_speckles(d, INV, max_size, 8)
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(d.cpu().numpy(), want)
