@@ -112,16 +112,23 @@ __global__ void __launch_bounds__(256) k_pyrdown(const __grid_constant__ PyrDown
 // rejected parent -- invalid disparity or confidence below the minimum --
 // becomes kNoParent: every label of the pixel is invalid).
 //
-// One block: 128 x 16 pixels of one view, a thread per 4 adjacent pixels
-// of a row.  The image tile with its 2-pixel border (4 columns on each
-// side, so rows stay word aligned) is staged as words when it lies inside
-// the image and the rows are word aligned, else byte by byte with
-// replicated borders.
+// One block: 128 x 8 pixels of one view, a warp per row.  The image tile
+// with its 2-pixel border (4 columns on each side, so rows stay word
+// aligned) is staged as words when it lies inside the image and the rows are
+// word aligned, else byte by byte with replicated borders.  Census: a thread
+// per 4 adjacent pixels, 16-byte stores.  BT: gradients of 4 adjacent pixels
+// per thread on 16-bit pairs, laid down with the intensities as one word per
+// pixel; then a thread per pixel, 32 apart, makes the intervals of both
+// channels at once from three words and stores 16 bytes beside its
+// neighbour's (a thread storing the features of 4 adjacent pixels kept L1
+// busy with quarter-line requests: 26 us for the two views of a 1080p level).
+// The parent's values are loaded before the tile is waited for.
 // ---------------------------------------------------------------------------
-constexpr int kFtX = 128, kFtY = 16;
+constexpr int kFtX = 128, kFtY = 8;
 constexpr int kFtSWB = kFtX + 8;        // staged bytes per row: image columns x0 - 4 .. x0 + 131
 constexpr int kFtSWW = kFtSWB / 4;      // ... as words
-constexpr int kFtSH = kFtY + 4;         // staged rows: y0 - 2 .. y0 + 17
+constexpr int kFtSH = kFtY + 4;         // staged rows: y0 - 2 .. y0 + 9
+constexpr int kFtGW = kFtX + 8;         // gradient words per row: columns x0 - 4 ..
 
 __device__ __forceinline__ uint32_t byte_of(uint32_t w, int k) { return (w >> (8 * k)) & 0xffu; }
 
@@ -154,6 +161,25 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
     const int W = J.w, H = J.h;
 
     __shared__ uint32_t tw[kFtSH][kFtSWW];   // byte c of row r: image pixel (y0 - 2 + r, x0 - 4 + c), clamped
+    __shared__ __align__(16) uint32_t gi[kFtY][kFtGW];   // BT: gradient | intensity << 16 of column x0 - 4 + c
+    const int tx = threadIdx.x & 31, rr = threadIdx.x >> 5;
+    const int xb = x0 + 4 * tx, y = y0 + rr;
+    const int np = y < H ? imin(4, W - xb) : 0;     // pixels of this thread inside the image
+    const bool vec = np == 4 && (W & 3) == 0;       // 16-byte stores of 4 words / 8-byte of 4 int16
+    // the parent's values of this thread's pixels
+    int praw[4];
+    float pcf[4];
+    if (view == 0 && J.refine && np > 0) {
+        const int py = imin(y >> 1, J.ph - 1);
+        const int16_t* prow = J.pdisp + (size_t)py * J.pd_pitch;
+        const float* crow = J.pconf + (size_t)py * J.pc_pitch;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {   // xb is even: pixels 2 j and 2 j + 1 have one parent
+            const int px = imin((xb >> 1) + j, J.pw - 1);
+            praw[2 * j] = praw[2 * j + 1] = __ldg(prow + px);
+            pcf[2 * j] = pcf[2 * j + 1] = __ldg(crow + px);
+        }
+    }
     const bool aligned = ((reinterpret_cast<uintptr_t>(img) | (uintptr_t)step) & 3u) == 0;
     if (aligned && x0 >= 4 && x0 + kFtX + 4 <= W && y0 >= 2 && y0 + kFtY + 2 <= H) {
         for (int i = threadIdx.x; i < kFtSH * kFtSWW; i += 256) {
@@ -168,18 +194,11 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
         }
     }
     __syncthreads();
-    const int tx = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int xb = x0 + 4 * tx;
-    if (xb >= W) return;
-    const int np = imin(4, W - xb);                 // pixels of this thread inside the image
-    const bool vec = np == 4 && (W & 3) == 0;       // 16-byte stores of 4 words / 8-byte of 4 int16
+    if (y >= H) return;
     const int ftzero = imax(J.pfc, 15) | 1;
-#pragma unroll 1
-    for (int rr = warp; rr < kFtY; rr += 8) {
-        const int y = y0 + rr;
-        if (y >= H) break;
+    {
         const size_t p = (size_t)y * W + xb;
-        if (!PG_IN(p, np, (size_t)W * H, 9)) continue;
+        if (!PG_IN((size_t)y * W + x0, imin(kFtX, W - x0), (size_t)W * H, 9)) return;
         if (J.cost == COST_CENSUS) {
             // bit (dy, dx) of the 4 pixels at once: bytes 2 + dx .. 5 + dx of
             // the 12-byte row window, compared with the 4 centre bytes
@@ -208,6 +227,7 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
                 cv[j] = (byte_of(acc[0], j) << 17) | (byte_of(acc[1], j) << 9) | (byte_of(acc[2], j) << 1) |
                         byte_of(acc[3], j);
             uint32_t* out = reinterpret_cast<uint32_t*>(feat) + p;
+            if (np <= 0) return;
             if (vec) {
                 *reinterpret_cast<uint4*>(out) = make_uint4(cv[0], cv[1], cv[2], cv[3]);
             } else {
@@ -216,54 +236,56 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
                     if (j < np) out[j] = cv[j];
             }
         } else {
-            // bytes 2 .. 9 of the window rows rr + 1 .. rr + 3: columns xb - 2 .. xb + 5
-            uint32_t r1[8], r2[8], r3[8];
-            {
-                const uint32_t a0 = tw[rr + 1][tx], a1 = tw[rr + 1][tx + 1], a2 = tw[rr + 1][tx + 2];
-                const uint32_t b0 = tw[rr + 2][tx], b1 = tw[rr + 2][tx + 1], b2 = tw[rr + 2][tx + 2];
-                const uint32_t c0 = tw[rr + 3][tx], c1 = tw[rr + 3][tx + 1], c2 = tw[rr + 3][tx + 2];
+            // columns xb - 1 .. xb + 4 of the three rows as 16-bit pairs
+            // (xb - 1, xb), (xb + 1, xb + 2), (xb + 3, xb + 4)
+            const uint32_t lim = (uint32_t)ftzero * 0x10001u;
+            uint32_t v[3] = {0u, 0u, 0u}, mid[3];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const int bi = k + 2;   // byte index in the 12-byte window
-                    const uint32_t wa = bi < 4 ? a0 : bi < 8 ? a1 : a2;
-                    const uint32_t wb = bi < 4 ? b0 : bi < 8 ? b1 : b2;
-                    const uint32_t wc = bi < 4 ? c0 : bi < 8 ? c1 : c2;
-                    r1[k] = byte_of(wa, bi & 3);
-                    r2[k] = byte_of(wb, bi & 3);
-                    r3[k] = byte_of(wc, bi & 3);
+            for (int k = 0; k < 3; ++k) {
+                const uint32_t a = tw[rr + 1 + k][tx], m = tw[rr + 1 + k][tx + 1], z = tw[rr + 1 + k][tx + 2];
+                const uint32_t q[3] = {__byte_perm(__byte_perm(a, m, 0x0043), 0, 0x4140), __byte_perm(m, 0, 0x4241),
+                                       __byte_perm(__byte_perm(m, z, 0x0043), 0, 0x4140)};
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    v[i] += k == 1 ? 2 * q[i] : q[i];
+                    if (k == 1) mid[i] = q[i];
                 }
             }
-            // g[i]: gradient at pixel column xb - 1 + i (window byte k = i + 1)
-            int g[6];
+            // gradient of column c: v(c + 1) - v(c - 1), clipped and offset
+            uint32_t g[2];
 #pragma unroll
-            for (int i = 0; i < 6; ++i) {
-                const int k = i + 1;
-                int v = ((int)r2[k + 1] - (int)r2[k - 1]) * 2;
-                v += (int)r1[k + 1] - (int)r1[k - 1];
-                v += (int)r3[k + 1] - (int)r3[k - 1];
-                g[i] = iclamp(v, -ftzero, ftzero) + ftzero;
+            for (int i = 0; i < 2; ++i)
+                g[i] = __vadd2(__vmaxs2(__vmins2(__vsub2(v[i + 1], v[i]), lim), __vsub2(0u, lim)), lim);
+            // intensities (xb, xb + 1), (xb + 2, xb + 3)
+            const uint32_t in0 = __byte_perm(mid[0], mid[1], 0x5432), in1 = __byte_perm(mid[1], mid[2], 0x5432);
+            *reinterpret_cast<uint4*>(&gi[rr][4 + 4 * tx]) =
+                make_uint4(__byte_perm(g[0], in0, 0x5410), __byte_perm(g[0], in0, 0x7632), __byte_perm(g[1], in1, 0x5410),
+                           __byte_perm(g[1], in1, 0x7632));
+            if (tx == 0 || tx == 31) {   // the columns beside the tile
+                const uint8_t* tb = reinterpret_cast<const uint8_t*>(&tw[0][0]);
+                const int c = tx == 0 ? 3 : kFtX + 4;   // staged column
+                int d = 0;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const uint8_t* r = tb + (rr + 1 + k) * kFtSWB + c;
+                    d += (k == 1 ? 2 : 1) * ((int)r[1] - (int)r[-1]);
+                }
+                gi[rr][c] = (uint32_t)(iclamp(d, -ftzero, ftzero) + ftzero) | (uint32_t)tb[(rr + 2) * kFtSWB + c] << 16;
             }
-            auto interval = [](int v, int l, int r, uint32_t& lo, uint32_t& hi) {
-                const int vl = (v + l) >> 1, vr = (v + r) >> 1;
-                lo = (uint32_t)imin(imin(vl, vr), v);
-                hi = (uint32_t)imax(imax(vl, vr), v);
-            };
-            uint4 f[4];
+            __syncwarp();
+            uint4* out = feat + (size_t)y * W;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 // the neighbour columns are clamped first (x - 1 -> 0 at the left border)
-                const int x = xb + j;
-                const bool hl = x > 0, hr = x + 1 < W;
-                const int gv = g[j + 1], iv = (int)r2[j + 2];
-                uint32_t glo, ghi, ilo, ihi;
-                interval(gv, hl ? g[j] : gv, hr ? g[j + 2] : gv, glo, ghi);
-                interval(iv, hl ? (int)r2[j + 1] : iv, hr ? (int)r2[j + 3] : iv, ilo, ihi);
-                auto pair = [](uint32_t g, uint32_t i) { return (g & 0xffffu) | (i << 16); };
-                f[j] = make_uint4(pair(gv, iv), pair(0u - gv, 0u - iv), pair(glo, ilo), pair(0u - ghi, 0u - ihi));
+                const int x = x0 + tx + 32 * j, c = 4 + tx + 32 * j;
+                if (x < W) {
+                    const uint32_t u = gi[rr][c], l = gi[rr][x > 0 ? c - 1 : c], r = gi[rr][x + 1 < W ? c + 1 : c];
+                    const uint32_t ul = ((u + l) >> 1) & 0x7fff7fffu, ur = ((u + r) >> 1) & 0x7fff7fffu;
+                    const uint32_t lo = __vimin3_u16x2(ul, ur, u), hi = __vimax3_u16x2(ul, ur, u);
+                    out[x] = make_uint4(u, __vsub2(0u, u), lo, __vsub2(0u, hi));
+                }
             }
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j < np) feat[p + j] = f[j];
+            if (np <= 0) return;
         }
         if (view == 0) {
             if (vec) {
@@ -274,15 +296,9 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
                     if (j < np) J.keys[p + j] = 0xffffffffu;   // no disp2 candidate yet
             }
             if (J.refine) {
-                const int py = imin(y >> 1, J.ph - 1);
-                const int16_t* prow = J.pdisp + (size_t)py * J.pd_pitch;
-                const float* crow = J.pconf + (size_t)py * J.pc_pitch;
                 int16_t b[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int px = imin((xb + j) >> 1, J.pw - 1);
-                    b[j] = j < np ? refine_base(J, xb + j, __ldg(prow + px), __ldg(crow + px)) : (int16_t)0;
-                }
+                for (int j = 0; j < 4; ++j) b[j] = refine_base(J, xb + j, praw[j], pcf[j]);
                 int16_t* bo = J.base + p;
                 if (vec) {
                     *reinterpret_cast<uint2*>(bo) =

@@ -25,27 +25,40 @@ cudaError_t launch_paths(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_
 // the nine is the median of (largest column minimum, median of the column
 // medians, smallest column maximum) -- the structure of the opt_med9
 // network of Paeth / Devillard ("Fast median search: an ANSI C
-// implementation").
-__device__ __forceinline__ int med3(int a, int b, int c) { return imax(imin(a, b), imin(imax(a, b), c)); }
+// implementation") --, two pixels at a time in 16-bit halves.
+__device__ __forceinline__ uint32_t med3(uint32_t a, uint32_t b, uint32_t c)
+{
+    return __vmaxs2(__vmins2(a, b), __vmins2(__vmaxs2(a, b), c));
+}
 
 struct Col3 {
-    int lo, mid, hi;
+    uint32_t lo, mid, hi;
 };
-__device__ __forceinline__ Col3 sort3(int a, int b, int c)
+__device__ __forceinline__ Col3 sort3(uint32_t a, uint32_t b, uint32_t c)
 {
-    const int l = imin(a, b), h = imax(a, b);
-    return {imin(l, c), imax(l, imin(h, c)), imax(h, c)};
+    const uint32_t l = __vmins2(a, b), h = __vmaxs2(a, b);
+    return {__vmins2(l, c), __vmaxs2(l, __vmins2(h, c)), __vmaxs2(h, c)};
 }
-__device__ __forceinline__ int median9(const Col3& a, const Col3& b, const Col3& c)
+// The columns one to the left of the second pair: the high half of a, the low half of b.
+__device__ __forceinline__ Col3 between(const Col3& a, const Col3& b)
 {
-    return med3(imax(imax(a.lo, b.lo), c.lo), med3(a.mid, b.mid, c.mid), imin(imin(a.hi, b.hi), c.hi));
+    return {__funnelshift_r(a.lo, b.lo, 16), __funnelshift_r(a.mid, b.mid, 16), __funnelshift_r(a.hi, b.hi, 16)};
+}
+__device__ __forceinline__ uint32_t median9(const Col3& a, const Col3& b, const Col3& c)
+{
+    return med3(__vimax3_s16x2(a.lo, b.lo, c.lo), med3(a.mid, b.mid, c.mid), __vimin3_s16x2(a.hi, b.hi, c.hi));
 }
 
-// One block: 128 x 16 pixels, a thread per 4 adjacent pixels of a row.  The
-// (LR-checked) disparities of the tile and its one-pixel halo are computed
-// once into shared memory; the median takes the in-image neighbours only
-// (sorted, middle element) at the image border.
-constexpr int kPoX = 128, kPoY = 16;
+// One block: 128 x 8 pixels, a warp per row, a thread per 4 adjacent pixels.
+// The (LR-checked) disparities of the tile and a halo of one row and four
+// columns are computed once into shared memory, four pixels at a time, in
+// three rounds so that a thread's loads overlap: raw disparities, the disp2
+// keys they point at, decisions; the confidences are loaded before all of
+// them.  The median takes the in-image neighbours only (sorted, middle
+// element) at the image border.  Instruction bound before (280 a pixel, 33
+// us on a 1080p level), latency bound below.
+constexpr int kPoX = 128, kPoY = 8;
+constexpr int kPoG = kPoX / 4 + 2;   // groups of 4 pixels per staged row: columns x0 - 4 .. x0 + 131
 
 template <int NJ>
 __global__ void __launch_bounds__(256) k_post(const __grid_constant__ Jobs<NJ> jobs)
@@ -54,183 +67,184 @@ __global__ void __launch_bounds__(256) k_post(const __grid_constant__ Jobs<NJ> j
     const int x0 = blockIdx.x * kPoX, y0 = blockIdx.y * kPoY;
     if (x0 >= J.w || y0 >= J.h) return;
     const int W = J.w, H = J.h;
-    const int16_t inv = (int16_t)((J.minD - 1) * 16);
+    const int inv = (int)(int16_t)((J.minD - 1) * 16);
     // The LR check (kernel_StrictPyramidLRCheck / kernel_PseudoLRCheck,
     // src/sgm_kernels.cu:825-889).
     const bool check = (J.post & POST_LRCHECK) != 0;
     const bool med = (J.post & POST_MEDIAN) != 0;
-    // The LR-checked disparities of the tile and its halo, staged in three
-    // rounds so that each thread's loads are in flight together: its raw
-    // disparities, then the disp2 keys they point at, then the decisions.
-    __shared__ int16_t td[kPoY + 2][kPoX + 2];   // row r, column c: pixel (y0 - 1 + r, x0 - 1 + c)
-    if (check || med) {
-        constexpr int kN = (kPoY + 2) * (kPoX + 2), kPer = (kN + 255) / 256;
-        int dv[kPer], xs[kPer], rowp[kPer];   // (a level has far fewer than 2^31 pixels)
+    const bool quad = (W & 3) == 0;   // rows of raw disparities and confidences start on 4-pixel boundaries
+    const int tx = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int xb = x0 + 4 * tx, y = y0 + warp;
+    const int np = y < H ? imin(4, W - xb) : 0;
+    __shared__ __align__(16) uint2 td[kPoY + 2][kPoG];   // row r, group g: pixels x0 - 4 + 4 g .. of row y0 - 1 + r
+    float cin[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (np > 0) {
+        const float* c = J.conf_raw + (size_t)y * W + xb;
+        if (quad) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(c));
+            cin[0] = v.x; cin[1] = v.y; cin[2] = v.z; cin[3] = v.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j < np) cin[j] = __ldg(c + j);
+        }
+    }
+    {
+        constexpr int kN = (kPoY + 2) * kPoG, kPer = (kN + 255) / 256;
+        int dv[kPer][4], xg[kPer], rowp[kPer];   // (a level has far fewer than 2^31 pixels)
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
             const int i = threadIdx.x + 256 * k;
-            const int r = i / (kPoX + 2), c = i - r * (kPoX + 2);
-            const int yy = y0 - 1 + r, xx = x0 - 1 + c;
-            const bool in = i < kN && yy >= 0 && yy < H && xx >= 0 && xx < W;
-            rowp[k] = in ? yy * W : 0;
-            xs[k] = in ? xx : -1;
-            dv[k] = in ? (int)J.disp_raw[(size_t)rowp[k] + xx] : (int)inv;
+            const int r = i / kPoG, g = i - r * kPoG;
+            const int yy = y0 - 1 + r;
+            xg[k] = x0 - 4 + 4 * g;
+            const bool in = i < kN && yy >= 0 && yy < H && xg[k] >= 0 && xg[k] < W;
+            rowp[k] = in ? yy * W : -1;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dv[k][j] = inv;
+            if (in) {
+                const int16_t* p = J.disp_raw + (size_t)rowp[k] + xg[k];
+                if (quad) {
+                    const uint2 a = __ldg(reinterpret_cast<const uint2*>(p));
+                    dv[k][0] = (int)(int16_t)(a.x & 0xffffu);
+                    dv[k][1] = (int)(int16_t)(a.x >> 16);
+                    dv[k][2] = (int)(int16_t)(a.y & 0xffffu);
+                    dv[k][3] = (int)(int16_t)(a.y >> 16);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (xg[k] + j < W) dv[k][j] = (int)__ldg(p + j);
+                }
+            }
         }
         if (check) {
-            unsigned k0[kPer], k1[kPer];
+            // The key of right pixel rx holds 0xffff - x' of its winner x'
+            // (all ones: none); the winner's disparity there is x' - rx, and
+            // rx + d0 = x, so that disp2 - d0 = x' - x.  A right pixel
+            // without a winner has disparity `inv` in the reference, which
+            // counts where it is not below minD (minD > 1).
+            unsigned k0[kPer][4], k1[kPer][4];
 #pragma unroll
-            for (int k = 0; k < kPer; ++k) {
-                k0[k] = k1[k] = 0xffffffffu;
-                if (xs[k] >= 0 && dv[k] != inv) {
-                    const int r0 = xs[k] - (dv[k] >> 4), r1 = xs[k] - ((dv[k] + 15) >> 4);
-                    if (r0 >= 0 && r0 < W) k0[k] = __ldg(J.keys + (size_t)rowp[k] + r0);
-                    if (r1 >= 0 && r1 < W) k1[k] = __ldg(J.keys + (size_t)rowp[k] + r1);
-                }
-            }
+            for (int k = 0; k < kPer; ++k)
 #pragma unroll
-            for (int k = 0; k < kPer; ++k) {
-                const int d16 = dv[k], xx = xs[k];
-                if (xx < 0 || d16 == inv) continue;
-                const int d0 = d16 >> 4, d1 = (d16 + 15) >> 4;
-                const int r0 = xx - d0, r1 = xx - d1;
-                // disp2 of right pixel rx from its key (cost << 16 | 0xffff - x)
-                auto disp2 = [&](unsigned key, int rx) -> int {
-                    return key == 0xffffffffu ? (int)inv : (int)(0xffffu - (key & 0xffffu)) - rx;
-                };
-                const bool in0 = r0 >= 0 && r0 < W, in1 = r1 >= 0 && r1 < W;
-                const int v0 = in0 ? disp2(k0[k], r0) : 0, v1 = in1 ? disp2(k1[k], r1) : 0;
-                if (J.pyr) {
-                    const bool ok = (in0 && v0 >= J.minD && abs(v0 - d0) <= J.maxdiff) ||
-                                    (in1 && v1 >= J.minD && abs(v1 - d1) <= J.maxdiff);
-                    dv[k] = ok ? d16 : (int)inv;
-                } else {
-                    const bool bad0 = in0 && v0 >= J.minD && abs(v0 - d0) > J.maxdiff;
-                    const bool bad1 = in1 && v1 >= J.minD && abs(v1 - d1) > J.maxdiff;
-                    dv[k] = (bad0 && bad1) ? (int)inv : d16;
+                for (int j = 0; j < 4; ++j) {
+                    k0[k][j] = k1[k][j] = 0xffffffffu;
+                    if (rowp[k] >= 0 && dv[k][j] != inv) {
+                        const int x = xg[k] + j, r0 = x - (dv[k][j] >> 4), r1 = x - ((dv[k][j] + 15) >> 4);
+                        const unsigned* row = J.keys + (size_t)rowp[k];
+                        if ((unsigned)r0 < (unsigned)W) k0[k][j] = __ldg(row + r0);
+                        if ((unsigned)r1 < (unsigned)W) k1[k][j] = __ldg(row + r1);
+                    }
                 }
-            }
+            const bool pyr = J.pyr != 0, none_counts = inv >= J.minD;
+            const int maxdiff = J.maxdiff;
+#pragma unroll
+            for (int k = 0; k < kPer; ++k)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int x = xg[k] + j;
+                    bool on0 = k0[k][j] != 0xffffffffu, on1 = k1[k][j] != 0xffffffffu;
+                    int e0 = abs((int)(~k0[k][j] & 0xffffu) - x), e1 = abs((int)(~k1[k][j] & 0xffffu) - x);
+                    if (none_counts) {
+                        const int d0 = dv[k][j] >> 4, d1 = (dv[k][j] + 15) >> 4;
+                        if (!on0) e0 = abs(inv - d0);
+                        if (!on1) e1 = abs(inv - d1);
+                        on0 = (unsigned)(x - d0) < (unsigned)W;
+                        on1 = (unsigned)(x - d1) < (unsigned)W;
+                    }
+                    const bool bad = pyr ? !((on0 && e0 <= maxdiff) || (on1 && e1 <= maxdiff))
+                                         : (on0 && e0 > maxdiff) && (on1 && e1 > maxdiff);
+                    if (bad) dv[k][j] = inv;
+                }
         }
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
             const int i = threadIdx.x + 256 * k;
-            if (i < kN) (&td[0][0])[i] = (int16_t)dv[k];
+            if (i < kN)
+                (&td[0][0])[i] = make_uint2(__byte_perm(dv[k][0], dv[k][1], 0x5410), __byte_perm(dv[k][2], dv[k][3], 0x5410));
         }
         __syncthreads();
     }
-    const int tx = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int xb = x0 + 4 * tx;
-    if (xb >= W) return;
-    const int np = imin(4, W - xb);
-#pragma unroll 1
-    for (int ty = warp; ty < kPoY; ty += 8) {
-        const int y = y0 + ty;
-        if (y >= H) break;
-        const size_t p = (size_t)y * W + xb;
-        int dv[4], dn[4];
-        float cf[4];
-        int din[4];
-        float cin[4];
-        if (np == 4 && (p & 3) == 0) {   // 8- and 16-byte loads of the four pixels
-            const uint2 a = *reinterpret_cast<const uint2*>(J.disp_raw + p);
-            const float4 c = *reinterpret_cast<const float4*>(J.conf_raw + p);
-            din[0] = (int)(int16_t)(a.x & 0xffffu);
-            din[1] = (int)(int16_t)(a.x >> 16);
-            din[2] = (int)(int16_t)(a.y & 0xffffu);
-            din[3] = (int)(int16_t)(a.y >> 16);
-            cin[0] = c.x; cin[1] = c.y; cin[2] = c.z; cin[3] = c.w;
+    if (np <= 0) return;
+    uint2 d = td[warp + 1][tx + 1], m = d;   // checked disparities, median
+    if (med) {
+        if (xb > 0 && xb + 4 < W && y > 0 && y + 1 < H) {
+            // column pairs (xb - 2, xb - 1) .. (xb + 4, xb + 5)
+            Col3 c[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                uint32_t v[3];
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    const uint2* row = &td[warp + r][tx];
+                    v[r] = i == 0 ? row[0].y : i == 1 ? row[1].x : i == 2 ? row[1].y : row[2].x;
+                }
+                c[i] = sort3(v[0], v[1], v[2]);
+            }
+            const Col3 mid = between(c[1], c[2]);
+            m.x = median9(between(c[0], c[1]), c[1], mid);
+            m.y = median9(mid, c[2], between(c[2], c[3]));
         } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int jj = imin(j, np - 1);
-                din[j] = J.disp_raw[p + jj];
-                cin[j] = J.conf_raw[p + jj];
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int jj = imin(j, np - 1);
-            const int d = (check || med) ? (int)td[ty + 1][4 * tx + 1 + jj] : din[j];
-            dv[j] = d;
-            cf[j] = (d != din[j]) ? 0.0f : cin[j];  // the check zeroes what it rejects
-            dn[j] = d;
-        }
-        if (med) {
-            const bool inner = xb > 0 && xb + 4 < W && y > 0 && y + 1 < H;
-            if (inner) {
-                Col3 c[6];
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    const int cc = 4 * tx + k;   // tile column of pixel column xb - 1 + k
-                    c[k] = sort3(td[ty][cc], td[ty + 1][cc], td[ty + 2][cc]);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) dn[j] = median9(c[j], c[j + 1], c[j + 2]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (j >= np) break;
-                    const int x = xb + j;
-                    int v[9];
-                    int n = 0;
-                    for (int dy = -1; dy <= 1; ++dy) {
-                        if (y + dy < 0 || y + dy >= H) continue;
-                        for (int dx = -1; dx <= 1; ++dx) {
-                            if (x + dx < 0 || x + dx >= W) continue;
-                            v[n++] = td[ty + 1 + dy][4 * tx + 1 + j + dx];
-                        }
+            int16_t o[4] = {0, 0, 0, 0};
+            for (int j = 0; j < np; ++j) {
+                const int x = xb + j;
+                int v[9];
+                int n = 0;
+                for (int dy = -1; dy <= 1; ++dy) {
+                    if (y + dy < 0 || y + dy >= H) continue;
+                    const int16_t* row = reinterpret_cast<const int16_t*>(td[warp + 1 + dy]);
+                    for (int dx = -1; dx <= 1; ++dx) {
+                        if (x + dx < 0 || x + dx >= W) continue;
+                        v[n++] = row[4 * tx + 4 + j + dx];
                     }
-                    for (int i = 1; i < n; ++i) {
-                        const int key = v[i];
-                        int q = i - 1;
-                        while (q >= 0 && v[q] > key) { v[q + 1] = v[q]; --q; }
-                        v[q + 1] = key;
-                    }
-                    dn[j] = v[n / 2];
                 }
+                for (int i = 1; i < n; ++i) {
+                    const int key = v[i];
+                    int q = i - 1;
+                    while (q >= 0 && v[q] > key) { v[q + 1] = v[q]; --q; }
+                    v[q + 1] = key;
+                }
+                o[j] = (int16_t)v[n / 2];
             }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (dn[j] != dv[j]) cf[j] = 0.0f;
-            }
-        }
-        const bool vec = np == 4;
-        if (J.out16 && PG_IN((size_t)y * J.out16_pitch + xb, np, (size_t)J.out16_pitch * H, 8)) {
-            int16_t* o = J.out16 + (size_t)y * J.out16_pitch + xb;
-            if (vec && ((reinterpret_cast<uintptr_t>(o) & 7) == 0)) {
-                *reinterpret_cast<uint2*>(o) =
-                    make_uint2((uint32_t)(uint16_t)dn[0] | ((uint32_t)(uint16_t)dn[1] << 16),
-                               (uint32_t)(uint16_t)dn[2] | ((uint32_t)(uint16_t)dn[3] << 16));
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (j < np) o[j] = (int16_t)dn[j];
-            }
-        }
-        float f32[4], fc[4];
-        const bool conv = J.out32 && J.outc;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float f = (int16_t)dn[j] / 16.0f;
-            const bool ok = (int16_t)dn[j] != inv && f > 0.0f;
-            f32[j] = ok ? f : 0.0f;
-            fc[j] = conv ? (ok ? cf[j] : 0.0f) : cf[j];
-        }
-        auto store4 = [&](float* o, const float (&v)[4]) {
-            if (vec && ((reinterpret_cast<uintptr_t>(o) & 15) == 0)) {
-                *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (j < np) o[j] = v[j];
-            }
-        };
-        if (conv) {
-            store4(J.out32 + (size_t)y * J.out32_pitch + xb, f32);
-            store4(J.outc + (size_t)y * J.outc_pitch + xb, fc);
-        } else if (J.outc && J.conf_only_copy) {
-            store4(J.outc + (size_t)y * J.outc_pitch + xb, fc);
+            m = make_uint2((uint32_t)(uint16_t)o[0] | ((uint32_t)(uint16_t)o[1] << 16),
+                           (uint32_t)(uint16_t)o[2] | ((uint32_t)(uint16_t)o[3] << 16));
         }
     }
+    const bool vec = np == 4;
+    if (J.out16 && PG_IN((size_t)y * J.out16_pitch + xb, np, (size_t)J.out16_pitch * H, 8)) {
+        int16_t* o = J.out16 + (size_t)y * J.out16_pitch + xb;
+        if (vec && ((reinterpret_cast<uintptr_t>(o) & 7) == 0)) {
+            *reinterpret_cast<uint2*>(o) = m;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j < np) o[j] = (int16_t)(j < 2 ? m.x >> (16 * j) : m.y >> (16 * (j - 2)));
+        }
+    }
+    const bool conv = J.out32 && J.outc;
+    if (!conv && !(J.outc && J.conf_only_copy)) return;
+    // the confidence stays where neither the check (which leaves `inv`) nor
+    // the median changed the disparity; invalid pixels have 0
+    float f32[4], fc[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int dn = (int)(int16_t)(j < 2 ? m.x >> (16 * j) : m.y >> (16 * (j - 2)));
+        const int dc = (int)(int16_t)(j < 2 ? d.x >> (16 * j) : d.y >> (16 * (j - 2)));
+        const bool ok = dn != inv && dn > 0;
+        f32[j] = ok ? dn / 16.0f : 0.0f;
+        fc[j] = dn == dc && dc != inv && (ok || !conv) ? cin[j] : 0.0f;
+    }
+    auto store4 = [&](float* o, const float (&v)[4]) {
+        if (vec && ((reinterpret_cast<uintptr_t>(o) & 15) == 0)) {
+            *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j < np) o[j] = v[j];
+        }
+    };
+    if (conv) store4(J.out32 + (size_t)y * J.out32_pitch + xb, f32);
+    store4(J.outc + (size_t)y * J.outc_pitch + xb, fc);
 }
 
 template <int NJ>
