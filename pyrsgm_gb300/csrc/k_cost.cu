@@ -35,6 +35,8 @@ constexpr int kPdSH = 2 * kPdY + 3;     // staged source rows
 template <int NB>
 __global__ void __launch_bounds__(256) k_pyrdown(const __grid_constant__ PyrDownBatch<NB> b)
 {
+    let_next_in();
+    after_previous();
     const PyrDownDesc& P = b.d[blockIdx.z];
     const int x0 = blockIdx.x * kPdX, y0 = blockIdx.y * kPdY;
     if (x0 >= P.dw || y0 >= P.dh) return;
@@ -151,6 +153,9 @@ __device__ __forceinline__ int16_t refine_base(const LevelDesc& J, int x, int ra
 template <int NJ>
 __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<NJ> jobs)
 {
+    // (the strips of a BT level of fixed disparities are a few even waves)
+    if (jobs.d[0].refine || jobs.d[0].cost == COST_CENSUS) let_next_in();
+    after_previous();
     const LevelDesc& J = jobs.d[blockIdx.z >> 1];
     const int view = blockIdx.z & 1;
     const int x0 = blockIdx.x * kFtX, y0 = blockIdx.y * kFtY;
@@ -335,6 +340,8 @@ __device__ __noinline__ int adaptive_p2_value(int P2, int cur, int prev, float a
 
 __global__ void k_p2_table(int* lut, int P2, float alpha, float beta, float lower, float upper)
 {
+    let_next_in();
+    after_previous();
     const int i = threadIdx.x;
     if (i < 256) lut[i] = adaptive_p2_value(P2, i, 0, alpha, beta, lower, upper);
 }
@@ -350,6 +357,7 @@ __global__ void k_p2_table(int* lut, int P2, float alpha, float beta, float lowe
 template <int NJ>
 __global__ void __launch_bounds__(256) k_cost_census(const __grid_constant__ Jobs<NJ> jobs)
 {
+    after_previous();
     const LevelDesc& J = jobs.d[blockIdx.z];
     const int x = blockIdx.x * 32 + (threadIdx.x & 31);
     const int y = blockIdx.y * 8 + (threadIdx.x >> 5);
@@ -429,6 +437,7 @@ constexpr int kBxX = 32, kBxY = 8, kBxD = 16;
 template <int NJ>
 __global__ void __launch_bounds__(256) k_cost_bt_box(const __grid_constant__ Jobs<NJ> jobs, int maxHalf, int nxt)
 {
+    after_previous();
     const LevelDesc& J = jobs.d[blockIdx.z];
     const int x0 = (blockIdx.x % nxt) * kBxX;
     const int d0 = (blockIdx.x / nxt) * kBxD;
@@ -518,6 +527,7 @@ __host__ __device__ constexpr size_t bs_smem(int db)
 template <int HW, int NJ>
 __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_constant__ Jobs<NJ> jobs, int strip)
 {
+    after_previous();
     constexpr int SW = kBsSeg + 2 * HW;
     constexpr int U = HW == 3 ? 12 : 4;   // columns per turn: a multiple of 4 right features and 2 HW costs kept
     const LevelDesc& J = jobs.d[blockIdx.z];
@@ -779,6 +789,7 @@ __device__ __forceinline__ void bt_row_sums(const LevelDesc& J, uint16_t* hs, ui
 template <int NJ>
 __global__ void __launch_bounds__(256, 3) k_cost_bt_tiled(const __grid_constant__ Jobs<NJ> jobs)
 {
+    after_previous();
     const LevelDesc& J = jobs.d[blockIdx.z];
     const int x0 = blockIdx.x * kTiX, y0 = blockIdx.y * kTiY;
     if (x0 >= J.w || y0 >= J.h) return;
@@ -962,7 +973,7 @@ cudaError_t launch_pyrdown(const PyrDownBatch<NB>& b, int max_dw, int max_dh, cu
 {
     dim3 grid((max_dw + kPdX - 1) / kPdX, (max_dh + kPdY - 1) / kPdY, b.n);
     prof_begin(st);
-    k_pyrdown<NB><<<grid, 256, 0, st>>>(b);
+    launch_after(k_pyrdown<NB>, grid, 256, 0, st, b);
     count_launch();
     if (prof_enabled()) {
         double by = 0;
@@ -978,7 +989,7 @@ template cudaError_t launch_pyrdown<kBatchPyr>(const PyrDownBatch<kBatchPyr>&, i
 cudaError_t launch_p2_table(int* lut, int P2, float alpha, float beta, float lower, float upper, cudaStream_t st)
 {
     prof_begin(st);
-    k_p2_table<<<1, 256, 0, st>>>(lut, P2, alpha, beta, lower, upper);
+    launch_after(k_p2_table, 1, 256, 0, st, lut, P2, alpha, beta, lower, upper);
     count_launch();
     prof_end(PK_P2TABLE, 1024.0, st);
     return launched(st, "k_p2_table");
@@ -989,7 +1000,7 @@ cudaError_t launch_prepare(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStrea
 {
     dim3 gf((e.max_w + kFtX - 1) / kFtX, (e.max_h + kFtY - 1) / kFtY, 2 * jobs.n);
     prof_begin(st);
-    k_features<NJ><<<gf, 256, 0, st>>>(jobs);
+    launch_after(k_features<NJ>, gf, 256, 0, st, jobs);
     count_launch();
     if (prof_enabled()) {
         // read u8 and write features of both views, write the keys; refine
@@ -1036,7 +1047,7 @@ cudaError_t launch_bt_strip(const Jobs<NJ>& jobs, cudaStream_t st)
     const cudaError_t err =
         cudaFuncSetAttribute(k_cost_bt_strip<HW, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
-    k_cost_bt_strip<HW, NJ><<<dim3(gx, (max_h + strip - 1) / strip, jobs.n), kBsThreads, smem, st>>>(jobs, strip);
+    launch_after(k_cost_bt_strip<HW, NJ>, dim3(gx, (max_h + strip - 1) / strip, jobs.n), kBsThreads, smem, st, jobs, strip);
     return cudaGetLastError();
 }
 
@@ -1074,7 +1085,7 @@ cudaError_t launch_bt_fixed(const Jobs<NJ>& jobs, cudaStream_t st)
             if (err != cudaSuccess) return err;
             const int nxt = (max_w + kBxX - 1) / kBxX;
             dim3 g(nxt * ((max_D + kBxD - 1) / kBxD), (max_h + kBxY - 1) / kBxY, part.n);
-            k_cost_bt_box<NJ><<<g, 256, smem, st>>>(part, maxHalf, nxt);
+            launch_after(k_cost_bt_box<NJ>, g, 256, smem, st, part, maxHalf, nxt);
             err = cudaGetLastError();
         }
         if (err != cudaSuccess) return err;
@@ -1090,13 +1101,13 @@ cudaError_t launch_cost(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t
     prof_begin(st);
     if (J0.cost == COST_CENSUS) {
         dim3 g((e.max_w + 31) / 32, (e.max_h + 7) / 8, jobs.n);
-        k_cost_census<NJ><<<g, 256, 0, st>>>(jobs);
+        launch_after(k_cost_census<NJ>, g, 256, 0, st, jobs);
     } else if (J0.refine) {
         cudaError_t err = cudaFuncSetAttribute(k_cost_bt_tiled<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)kTiSmem);
         if (err != cudaSuccess) return err;
         dim3 g((e.max_w + kTiX - 1) / kTiX, (e.max_h + kTiY - 1) / kTiY, jobs.n);
-        k_cost_bt_tiled<NJ><<<g, 256, kTiSmem, st>>>(jobs);
+        launch_after(k_cost_bt_tiled<NJ>, g, 256, kTiSmem, st, jobs);
     } else {
         const cudaError_t err = launch_bt_fixed(jobs, st);
         if (err != cudaSuccess) return err;

@@ -37,7 +37,7 @@ cudaError_t launch_wta(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t 
 {
     dim3 gw((e.max_w + 31) / 32, (e.max_h + 7) / 8, jobs.n);
     prof_begin(st);
-    k_wta<D, PYR, NJ><<<gw, 256, 0, st>>>(jobs);
+    launch_after(k_wta<D, PYR, NJ>, gw, 256, 0, st, jobs);
     count_launch();
     prof_end(PK_WTA, jobs_vox(jobs) * 2 * (jobs.d[0].paths >= 3 ? 3 : jobs.d[0].paths) + jobs_px(jobs) * (2 + 6 + 4), st);
     return launched(st, "k_wta");
@@ -86,7 +86,7 @@ cudaError_t launch_paths_wide(const Jobs<NJ>& jobs, const LevelExtent& e, cudaSt
         const int cols = kWarps * G::CPW;
         dim3 g((e.max_w + cols - 1) / cols, n);
         prof_begin(st);
-        k_gtb<NW, T, PYR, NJ><<<g, kWarps * 32, smem, st>>>(tbj);
+        launch_after(k_gtb<NW, T, PYR, NJ>, g, kWarps * 32, smem, st, tbj);
         count_launch();
         prof_end(PK_PATH_TB, jobs_vox(tbj) * 4 + jobs_px(tbj) * ((tbj.d[0].refine ? 2 : 0) + (tbj.d[0].adaptive ? 1 : 0)), st);
         if ((err = launched(st, "k_gtb")) != cudaSuccess) return err;
@@ -99,7 +99,7 @@ cudaError_t launch_paths_wide(const Jobs<NJ>& jobs, const LevelExtent& e, cudaSt
         cudaSuccess)
         return err;
     prof_begin(st);
-    k_grow<NW, T, PYR, NJ><<<g, kWarps * 32, smem, st>>>(jobs);
+    launch_after(k_grow<NW, T, PYR, NJ>, g, kWarps * 32, smem, st, jobs);
     count_launch();
     if (prof_enabled()) {
         // algorithmic bytes: each horizontal path reads the cost volume and
@@ -121,7 +121,7 @@ cudaError_t launch_paths_wide(const Jobs<NJ>& jobs, const LevelExtent& e, cudaSt
                 return err;
             dim3 gt((e.max_w + 127) / 128, jobs.n);
             prof_begin(st);
-            k_gtbw<NJ><<<gt, 128, smem, st>>>(jobs);
+            launch_after(k_gtbw<NJ>, gt, 128, smem, st, jobs);
             count_launch();
             prof_end(PK_TBW, jobs_vox(jobs) * 6 + jobs_px(jobs) * ((jobs.d[0].refine ? 2 : 0) + (jobs.d[0].adaptive ? 1 : 0) + 10),
                      st);

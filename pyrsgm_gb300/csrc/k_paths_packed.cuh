@@ -394,6 +394,7 @@ constexpr size_t tb_smem()
 template <int NW, int T, bool PYR, int NJ>
 __global__ void __launch_bounds__(pk::kPackedWarps * 32) k_gtb(const __grid_constant__ Jobs<NJ> jobs)
 {
+    after_previous();
     using namespace pk;
     using G = Grp<NW, T>;
     constexpr int D = G::D, S = kStagesTb, RS = G::RSW_TB, kWarps = kPackedWarps;
@@ -500,6 +501,7 @@ __global__ void __launch_bounds__(pk::kPackedWarps * 32) k_gtb(const __grid_cons
 template <int NW, int T, bool PYR, int NJ>
 __global__ void __launch_bounds__(pk::kPackedWarps * 32) k_grow(const __grid_constant__ Jobs<NJ> jobs)
 {
+    after_previous();
     using namespace pk;
     using G = Grp<NW, T>;
     constexpr int D = G::D, CPW = G::CPW, RPW = CPW / 2, kWarps = kPackedWarps;
@@ -680,6 +682,8 @@ __global__ void __launch_bounds__(pk::kPackedWarps * 32) k_grow(const __grid_con
 template <int D, bool PYR, int NJ>
 __global__ void __launch_bounds__(256) k_wta(const __grid_constant__ Jobs<NJ> jobs)
 {
+    if (NJ == 1) let_next_in();   // (in a batch the next label count's chains may follow)
+    after_previous();
     using namespace pk;
     constexpr int DW = D / 2;
     const LevelDesc& J = jobs.d[blockIdx.z];
@@ -787,6 +791,7 @@ __host__ __device__ constexpr size_t tbw_smem()
 template <int NJ>
 __global__ void __launch_bounds__(128, 4) k_gtbw(const __grid_constant__ Jobs<NJ> jobs)
 {
+    after_previous();
     using namespace pk;
     using G = Grp<8, 1>;
     constexpr int D = 16, S = kStagesTbw, kWarps = 4, SLOT = 3 * 256;   // words: costs, Vl, Vr of 32 lanes

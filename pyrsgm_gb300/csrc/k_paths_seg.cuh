@@ -601,13 +601,18 @@ __global__ void __launch_bounds__(sg::max_seg<NW>() * 32) k_seg(const __grid_con
     const int rgroups = rows_too ? (2 * J.h + G::CPW - 1) / G::CPW : 0;
     const bool rows = (int)blockIdx.x < rgroups;
     const int g0 = (rows ? (int)blockIdx.x : (int)blockIdx.x - rgroups) * G::CPW;
-    if (!rows && g0 >= e.ncol) return;   // the whole block is past the level
+    if (!rows && g0 >= e.ncol) {   // the whole block is past the level
+        after_previous();
+        return;
+    }
     int* lut = reinterpret_cast<int*>(smem);
     int* marked = reinterpret_cast<int*>(smem + 256);   // [segment][chain]: walk it (again)
     uint32_t* mine = smem + 256 + (kMaxSeg + 1) * 32 + b * warp_words<NW, T, MODE>();
     uint32_t* edge = smem + 256 + (kMaxSeg + 1) * 32 + segs * warp_words<NW, T, MODE>();
-    const bool high = load_penalties(J, lut);
     for (int i = lane; i < warp_words<NW, T, MODE>(); i += 32) mine[i] = kMax2;
+    if (rows_too) let_next_in();   // (columns alone: k_rowadd is next)
+    after_previous();
+    const bool high = load_penalties(J, lut);
     const bool guard = __syncthreads_or(high);
 
     const int k = lane % T;
@@ -708,7 +713,7 @@ cudaError_t launch_seg_mode(const Jobs<NJ>& jobs, bool rows_too, cudaStream_t st
         cudaFuncSetAttribute(k_seg<NW, T, MODE, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     prof_begin(st);
-    k_seg<NW, T, MODE, NJ><<<dim3(grid, jobs.n), segs * 32, smem, st>>>(jobs, rows_too ? 1 : 0, kWarmSteps);
+    launch_after(k_seg<NW, T, MODE, NJ>, dim3(grid, jobs.n), segs * 32, smem, st, jobs, rows_too ? 1 : 0, kWarmSteps);
     count_launch();
     if (prof_enabled()) {
         // each path reads the cost volume and writes its costs once

@@ -22,12 +22,17 @@ __global__ void __launch_bounds__(32) k_rowadd(const __grid_constant__ Jobs<NJ> 
     const LevelDesc& J = jobs.d[blockIdx.y];
     extern __shared__ __align__(16) uint32_t smem[];
     const int lane = threadIdx.x, g0 = blockIdx.x * G::CPW;
-    if (g0 >= 2 * J.h) return;
+    if (g0 >= 2 * J.h) {
+        after_previous();
+        return;
+    }
     const Extent<MODE> e(J);
     int* lut = reinterpret_cast<int*>(smem);
     uint32_t* mine = smem + 256;
-    const bool guard = __any_sync(0xffffffffu, load_penalties(J, lut));
     for (int i = lane; i < warp_words<NW, T, MODE>(2); i += 32) mine[i] = kMax2;
+    let_next_in();
+    after_previous();
+    const bool guard = __any_sync(0xffffffffu, load_penalties(J, lut));
     __syncwarp();
     const int k = lane % T;
     Ctx<NW, T, MODE> X{J, lut, mine, mine + 2 * kSC * G::SLOTW + lane / T + NW * k * G::WST, nullptr, lane, lane / T, k,
@@ -48,6 +53,8 @@ __global__ void __launch_bounds__(32) k_rowadd(const __grid_constant__ Jobs<NJ> 
 template <int G, int R, bool PYR, int NJ>
 __global__ void __launch_bounds__(256) k_wta_sum(const __grid_constant__ Jobs<NJ> jobs)
 {
+    if (NJ == 1) let_next_in();   // (in a batch the next label count's chains may follow)
+    after_previous();
     const LevelDesc& J = jobs.d[blockIdx.z];
     const int W = J.w, D = J.D, lane = threadIdx.x & 31, gl = lane % G;
     const int y = blockIdx.y * 8 + (threadIdx.x >> 5), x0 = blockIdx.x * 32;
@@ -124,7 +131,7 @@ cudaError_t launch_rowadd_mode(const Jobs<NJ>& jobs, const LevelExtent& e, cudaS
         cudaFuncSetAttribute(k_rowadd<NW, T, MODE, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     prof_begin(st);
-    k_rowadd<NW, T, MODE, NJ><<<dim3((2 * e.max_h + G::CPW - 1) / G::CPW, jobs.n), 32, smem, st>>>(jobs);
+    launch_after(k_rowadd<NW, T, MODE, NJ>, dim3((2 * e.max_h + G::CPW - 1) / G::CPW, jobs.n), 32, smem, st, jobs);
     count_launch();
     if (prof_enabled()) {
         // each direction reads the cost volume; V is read (T->B or the first
@@ -167,7 +174,7 @@ cudaError_t launch_sum(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t 
     if (err != cudaSuccess) return err;
     dim3 gw((e.max_w + 31) / 32, (e.max_h + 7) / 8, jobs.n);
     prof_begin(st);
-    k_wta_sum<G, R, PYR, NJ><<<gw, 256, 0, st>>>(jobs);
+    launch_after(k_wta_sum<G, R, PYR, NJ>, gw, 256, 0, st, jobs);
     count_launch();
     prof_end(PK_WTA, jobs_vox(jobs) * 2 + jobs_px(jobs) * (2 + 6 + 4), st);
     return launched(st, "k_wta_sum");

@@ -63,6 +63,8 @@ constexpr int kPoG = kPoX / 4 + 2;   // groups of 4 pixels per staged row: colum
 template <int NJ>
 __global__ void __launch_bounds__(256) k_post(const __grid_constant__ Jobs<NJ> jobs)
 {
+    let_next_in();
+    after_previous();
     const LevelDesc& J = jobs.d[blockIdx.z];
     const int x0 = blockIdx.x * kPoX, y0 = blockIdx.y * kPoY;
     if (x0 >= J.w || y0 >= J.h) return;
@@ -252,7 +254,7 @@ cudaError_t launch_post(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t
 {
     dim3 g((e.max_w + kPoX - 1) / kPoX, (e.max_h + kPoY - 1) / kPoY, jobs.n);
     prof_begin(st);
-    k_post<NJ><<<g, 256, 0, st>>>(jobs);
+    launch_after(k_post<NJ>, g, 256, 0, st, jobs);
     count_launch();
     if (prof_enabled()) {
         double by = 0;

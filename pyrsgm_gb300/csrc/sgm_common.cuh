@@ -79,6 +79,19 @@ struct Jobs {
 // (k_paths_packed.cuh); their LR check runs in the post kernel.
 __host__ __device__ __forceinline__ bool uses_packed(int D) { return D == 16 || D == 32 || D == 64; }
 
+// Kernels are launched with launch_after(): a grid may be let in before the
+// one ahead of it in the stream is complete, and begins with
+// after_previous(), which waits until that one is complete and its writes
+// are visible.  It is let in when every block of the one ahead has called
+// let_next_in() or ended.  Kernels ahead of one that counts on an even
+// spread of its blocks over the SMs (a single wave: k_seg, k_rowadd, k_grow,
+// k_gtbw, k_cost_bt_strip) do not call it: blocks let in early pile up on
+// the SMs that finish first (with it in every kernel the rows of a 720p level
+// with 128 labels took half as long again, and 32 pairs 9.8 instead of 9.0
+// ms).
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ int imin(int a, int b) { return a < b ? a : b; }
 __device__ __forceinline__ int imax(int a, int b) { return a > b ? a : b; }
 __device__ __forceinline__ int iclamp(int v, int lo, int hi) { return imin(imax(v, lo), hi); }

@@ -124,6 +124,34 @@ struct TuningScope {
 bool tune_lookup(const TuneKey& k, TuneEntry& out);
 void tune_store(const TuneKey& k, const TuneEntry& e);
 
+// Launch a kernel that begins with after_previous() (sgm_common.cuh): its
+// blocks may become resident while the previous kernel of the stream
+// finishes.  Every kernel waits for the whole one before it, so the order of
+// the stream is kept.  Hides the launch and the start of the blocks, 1 to 2
+// us a kernel (160x96 level, five kernels: 34 -> 27 us a call).  The launch
+// error is left for cudaGetLastError().
+template <class T>
+struct LaunchArg {
+    using type = T;
+};
+template <class... P>
+void launch_after(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t st,
+                  const typename LaunchArg<P>::type&... args)
+{
+    cudaLaunchAttribute a;
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    void* p[] = {const_cast<void*>(static_cast<const void*>(&args))...};
+    cudaLaunchKernelExC(&c, reinterpret_cast<const void*>(kernel), p);
+}
+
 // Count of kernel launches issued by this library (process-wide); a CUDA
 // graph replay counts the kernels it contains.
 void count_launch();

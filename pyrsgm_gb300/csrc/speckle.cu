@@ -86,6 +86,8 @@ __device__ __forceinline__ int sp_first(unsigned runs, int lane)
 // pixels in the tile at the root, 0 elsewhere.
 __global__ void __launch_bounds__(256) k_sp_tile(const SpArgs A)
 {
+    let_next_in();
+    after_previous();
     __shared__ int lab[kSpTile * kSpTile], cnt[kSpTile * kSpTile];
     __shared__ short val[kSpTile * kSpTile];
     __shared__ unsigned runs[kSpTile];   // bit x: pixel x continues the run of pixel x - 1
@@ -145,6 +147,8 @@ __global__ void __launch_bounds__(256) k_sp_tile(const SpArgs A)
 // i / h, row i % h), then across their upper ones.
 __global__ void __launch_bounds__(256) k_sp_link(const SpArgs A, int nv, int nh)
 {
+    let_next_in();
+    after_previous();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= nv + nh) return;
     const bool side = i < nv;
@@ -164,6 +168,8 @@ __global__ void __launch_bounds__(256) k_sp_link(const SpArgs A, int nv, int nh)
 // The tile roots' sizes to their global roots.
 __global__ void __launch_bounds__(256) k_sp_count(const SpArgs A)
 {
+    let_next_in();
+    after_previous();
     const long long p = (long long)blockIdx.x * 256 + threadIdx.x;
     if (p >= (long long)A.w * A.h) return;
     const int n = A.size[p];
@@ -173,6 +179,8 @@ __global__ void __launch_bounds__(256) k_sp_count(const SpArgs A)
 
 __global__ void __launch_bounds__(256) k_sp_apply(const SpArgs A)
 {
+    let_next_in();
+    after_previous();
     const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
     if (x >= A.w || y >= A.h) return;
     int r = A.lab[y * A.w + x];
@@ -203,21 +211,21 @@ extern "C" int pyrsgm_gb300_filter_speckles(short* d_disp, size_t pitch_bytes, i
     const int nv = (tx - 1) * height, nh = (ty - 1) * width;   // border pixels: left edges, upper edges
     cudaError_t e;
     int launches = 3;
-    pg::k_sp_tile<<<dim3(tx, ty), 256, 0, stream>>>(A);
+    pg::launch_after(pg::k_sp_tile, dim3(tx, ty), 256, 0, stream, A);
     e = pg::launched(stream, "k_sp_tile");
     if (e == cudaSuccess && nv + nh > 0) {
-        pg::k_sp_link<<<(nv + nh + 255) / 256, 256, 0, stream>>>(A, nv, nh);
+        pg::launch_after(pg::k_sp_link, (nv + nh + 255) / 256, 256, 0, stream, A, nv, nh);
         e = pg::launched(stream, "k_sp_link");
         ++launches;
         if (e == cudaSuccess) {
-            pg::k_sp_count<<<(int)((n + 255) / 256), 256, 0, stream>>>(A);
+            pg::launch_after(pg::k_sp_count, (int)((n + 255) / 256), 256, 0, stream, A);
             e = pg::launched(stream, "k_sp_count");
         }
     } else {
         --launches;   // one tile: its sizes are final
     }
     if (e == cudaSuccess) {
-        pg::k_sp_apply<<<dim3((width + 31) / 32, (height + 7) / 8), 256, 0, stream>>>(A);
+        pg::launch_after(pg::k_sp_apply, dim3((width + 31) / 32, (height + 7) / 8), 256, 0, stream, A);
         e = pg::launched(stream, "k_sp_apply");
     }
     pg::count_launches(launches);
