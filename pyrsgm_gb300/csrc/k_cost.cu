@@ -350,48 +350,63 @@ __global__ void k_p2_table(int* lut, int P2, float alpha, float beta, float lowe
 // Census cost volume.  Coarse / single-scale: kernel_CensusCost
 // (src/sgm_kernels.cu:303-327), 24 when x - d - minD is outside the image.
 // Refine: kernel_CensusCostLocal (src/sgm_kernels.cu:1112-1133), kMax for a
-// geometry-invalid label.  One thread per pixel writes its D labels, eight
-// per 16-byte store (label pairs or single labels when D is not a multiple
-// of eight).
+// geometry-invalid label.  A thread per pixel and eight labels, so that a
+// warp stores whole lines whatever D is (a thread per pixel, its labels D * 2
+// bytes from the next one's, took 42 us for 641x479 with 96 labels, 19 for
+// 1080p with 16), of kCnRows rows, whose loads overlap.  The right
+// descriptors of neighbouring threads overlap and come from L1.
 // ---------------------------------------------------------------------------
+constexpr int kCnRows = 4;
+
 template <int NJ>
 __global__ void __launch_bounds__(256) k_cost_census(const __grid_constant__ Jobs<NJ> jobs)
 {
     after_previous();
     const LevelDesc& J = jobs.d[blockIdx.z];
-    const int x = blockIdx.x * 32 + (threadIdx.x & 31);
-    const int y = blockIdx.y * 8 + (threadIdx.x >> 5);
-    if (x >= J.w || y >= J.h) return;
-    const int W = J.w, D = J.D;
-    const size_t p = (size_t)y * W + x;
-    const uint32_t cl = reinterpret_cast<const uint32_t*>(J.featL)[p];
-    const uint32_t* rrow = reinterpret_cast<const uint32_t*>(J.featR) + (size_t)y * W;
-    // label d reads right pixel x - off - d when lo <= d <= hi, else `fill`
-    int off, lo, hi, fill;
-    if (J.refine) {
-        off = J.base[p];
-        label_range(J, x, off, lo, hi);
-        fill = kMax;
-    } else {
-        off = J.minD;
-        lo = imax(0, x - off - (W - 1));
-        hi = imin(D - 1, x - off);
-        fill = 24;
-    }
-    auto cost = [&](int d) -> uint32_t {
-        return (d >= lo && d <= hi) ? (uint32_t)__popc(cl ^ __ldg(&rrow[x - off - d])) : (uint32_t)fill;
-    };
-    int16_t* out = J.C + p * D;
-    if (!PG_IN(p * D, D, (size_t)W * J.h * D, 10)) return;
-    if ((D & 7) == 0) {
-        for (int d0 = 0; d0 < D; d0 += 8) {
-            uint32_t w[4];
+    const int W = J.w, D = J.D, y0 = blockIdx.y * kCnRows;
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    const int x = D == 16 ? i >> 1 : i / (D / 8);
+    if (x >= W || y0 >= J.h) return;
+    const int d0 = (i - x * (D / 8)) * 8;
+    const int rows = imin(kCnRows, J.h - y0);
+    const size_t p0 = (size_t)y0 * W + x;
+    const uint32_t* const fl = reinterpret_cast<const uint32_t*>(J.featL);
+    const uint32_t* const fr = reinterpret_cast<const uint32_t*>(J.featR);
+    uint32_t cl[kCnRows];
+    int off[kCnRows];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) w[i] = cost(d0 + 2 * i) | (cost(d0 + 2 * i + 1) << 16);
-            reinterpret_cast<uint4*>(out + d0)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    for (int r = 0; r < kCnRows; ++r) {
+        const size_t p = p0 + (size_t)(r < rows ? r : 0) * W;
+        cl[r] = __ldg(fl + p);
+        off[r] = J.refine ? (int)__ldg(J.base + p) : J.minD;
+    }
+#pragma unroll
+    for (int r = 0; r < kCnRows; ++r) {
+        if (r >= rows) break;
+        const size_t p = p0 + (size_t)r * W;
+        // label d reads right pixel x - off - d when lo <= d <= hi, else `fill`
+        int lo, hi, fill;
+        if (J.refine) {
+            label_range(J, x, off[r], lo, hi);
+            fill = kMax;
+        } else {
+            lo = imax(0, x - off[r] - (W - 1));
+            hi = imin(D - 1, x - off[r]);
+            fill = 24;
         }
-    } else {
-        for (int d = 0; d < D; ++d) out[d] = (int16_t)cost(d);
+        uint32_t c[8];
+        const uint32_t* q = fr + (p - x) + (x - off[r] - d0);
+        if (lo <= d0 && hi >= d0 + 7) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) c[k] = (uint32_t)__popc(cl[r] ^ __ldg(q - k));
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                c[k] = d0 + k >= lo && d0 + k <= hi ? (uint32_t)__popc(cl[r] ^ __ldg(q - k)) : (uint32_t)fill;
+        }
+        if (!PG_IN(p * D + d0, 8, (size_t)W * J.h * D, 10)) continue;
+        *reinterpret_cast<uint4*>(J.C + p * D + d0) =
+            make_uint4(c[0] | (c[1] << 16), c[2] | (c[3] << 16), c[4] | (c[5] << 16), c[6] | (c[7] << 16));
     }
 }
 
@@ -1100,7 +1115,9 @@ cudaError_t launch_cost(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t
     const LevelDesc& J0 = jobs.d[0];
     prof_begin(st);
     if (J0.cost == COST_CENSUS) {
-        dim3 g((e.max_w + 31) / 32, (e.max_h + 7) / 8, jobs.n);
+        int chunks = 0;   // of eight labels, in the widest row
+        for (int i = 0; i < jobs.n; ++i) chunks = std::max(chunks, jobs.d[i].w * (jobs.d[i].D / 8));
+        dim3 g((chunks + 255) / 256, (e.max_h + kCnRows - 1) / kCnRows, jobs.n);
         launch_after(k_cost_census<NJ>, g, 256, 0, st, jobs);
     } else if (J0.refine) {
         cudaError_t err = cudaFuncSetAttribute(k_cost_bt_tiled<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
