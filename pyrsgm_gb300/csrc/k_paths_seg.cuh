@@ -671,22 +671,34 @@ __global__ void __launch_bounds__(sg::max_seg<NW>() * 32) k_seg(const __grid_con
 }
 
 // Segments for a launch of `blocks` chain groups whose longest walk has n
-// steps: as many as keep every block resident at 16 warps per SM (128
-// registers a thread).  A segment more than that makes a second wave: 429
-// groups (2879x1987) took 215 us with 5 segments and 256 with 8, 255 groups
-// (1080p) 86 us with 7 and 106 with 9.  Short segments are walked again for
-// longer than they saved: 64 steps at least (2879x1987 pyramid: 1247 us a
-// call with 64, 1262 with 40, 1270 with 130), 40 for the first four segments
-// of small levels (160x96: 42 us a call, 46 at 64).
+// steps.
+// Refinement levels: as many as fill the SMs where there are one or two
+// groups per SM (960x540 42 us with 8, 1080p 90 with 7), else five, four for
+// short walks: a block then holds a few rows over a stretch that L2 keeps
+// between its two directions, and three blocks of five warps are as many as
+// shared memory and L1 serve well.  1080p rows of 16 pairs: 1543 us with one
+// segment, 1275 with 4, 1099 with 5, 1091 with 6, 1110 with 7, 1220 with 8,
+// 1220 with 12, 1354 with 16.
+// Coarse and single-scale levels forget their start over 100 to 200 steps
+// and walk more segments again and again (mixed batch, 64 labels: 204 us with
+// 1, 134 with 2, 137 with 4, 175 with 8, 276 with 16); columns alone
+// (k_rowadd does the rows) take what keeps every group resident (641x479, 96
+// labels: 37 us with 8, 46 with 4).
+// A segment holds at least 64 steps (2879x1987 pyramid: 1247 us a call with
+// 64, 1262 with 40, 1270 with 130), 40 for the first four segments of small
+// levels (160x96: 42 us a call, 46 at 64).
 constexpr int kMinSeg = 64, kMinSegSmall = 40;
 constexpr int kMaxRefineLabels = 256;   // pyrsgm_compute_level takes no more on a refinement level
 constexpr size_t kSmemPerBlock = 227 * 1024;
 constexpr int kWarmSteps = 16;   // 0 to 32 measured within 5 % of each other, 64 10 % slower
 
-inline int segments_for(long long blocks, int n, int most)
+template <int MODE>
+int segments_for(long long blocks, int n, bool rows_too, int most)
 {
-    const long long per_sm = (blocks + sm_count() - 1) / sm_count();
-    const long long want = std::max<long long>(1, 16 / std::max<long long>(1, per_sm));
+    const long long per_sm = std::max<long long>(1, (blocks + sm_count() - 1) / sm_count());
+    long long want;
+    if (MODE == sg::kRefine) want = per_sm == 1 ? 16 : per_sm == 2 ? 7 : n >= 480 ? 5 : 4;
+    else want = std::max<long long>(2, std::min<long long>(16 / per_sm, rows_too ? 4 : 16));
     const long long fit = std::max(n / kMinSeg, std::min(4, n / kMinSegSmall));
     return (int)std::max<long long>(1, std::min<long long>(std::min<long long>(want, most), fit));
 }
@@ -706,7 +718,7 @@ cudaError_t launch_seg_mode(const Jobs<NJ>& jobs, bool rows_too, cudaStream_t st
         n = std::max(n, rows_too ? std::max(d.w, d.h) : d.h);
     }
     if (grid == 0) return cudaSuccess;
-    int segs = segments_for(blocks, n, sg::max_seg<NW>());
+    int segs = segments_for<MODE>(blocks, n, rows_too, sg::max_seg<NW>());
     while (segs > 1 && sg::seg_smem<NW, T, MODE>(segs) > kSmemPerBlock) --segs;
     const size_t smem = sg::seg_smem<NW, T, MODE>(segs);
     const cudaError_t err =

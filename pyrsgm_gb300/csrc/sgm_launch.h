@@ -85,7 +85,8 @@ int sm_count();
 
 // 0 (choose per launch), 8, or 2/4: the packed kernels' words per thread.
 int packed_words_override();
-// Warps per SM the NW = 8 shape must fill before a launch takes it.
+// Warps per SM the wide shape must fill before a launch takes it by itself
+// (INT_MAX: it is taken only when forced or measured faster).
 int packed_min_warps_per_sm();
 // 1: fused two-pass form of the 16-label pyramid levels (opt-in).
 int fused_mode();
