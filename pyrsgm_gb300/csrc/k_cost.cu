@@ -686,115 +686,145 @@ __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_const
 // when q - (base_p + d) leaves the image), clamps the sum to kMax - 1, and
 // writes kMax for a geometry-invalid label.  The sum depends on p only
 // through the window and the real disparity, so one 32x16 tile evaluates
-// each (window pixel, real disparity) pair once when the real disparities
-// its pixels need, [min base, max base + D - 1], span at most kTiRn:
-//   staging: the features of every window row of the tile (left: one per
+// each (window pixel, real disparity) pair once, 16 labels at a time and one
+// pass per cluster of bases: the pixels whose real disparities span at most
+// kTiRn.  Most tiles are one cluster.  A pass:
+//   staging: the features of the window rows of the cluster (left: one per
 //            window column, clamped; right: the ones its disparities reach)
 //            are copied once into shared memory with cp.async, a warp per
 //            row; right pixels outside the image get a feature of cost 255;
-//   phase 1: the (window row, two adjacent real disparities) units are
-//            numbered row-major and cut into groups of 32, one unit per
-//            lane, dealt to the 8 warps in turn; a lane walks the window
-//            columns left to right and keeps the running sums of the last
-//            blockSize costs of both disparities (sums along x, into shared
-//            memory), loading each left and right feature once for the two.
-//            A tile usually needs 17 real disparities, so numbering the
-//            units this way keeps nearly every lane busy;
+//   phase 1: a lane takes four adjacent real disparities of a window row and
+//            half of the tile's columns, walks the window columns left to
+//            right and keeps the running sums of the last blockSize costs
+//            (sums along x, into shared memory).  Disparity i + 1 needs at
+//            column j the right feature that i needed at column j - 1, so it
+//            loads one left and one right feature per column for four costs.
+//            A tile usually needs 17 real disparities: 200 units of 20
+//            columns for 256 lanes;
 //   phase 2: a thread per two vertical neighbours adds blockSize rows of
 //            those sums for each, two labels per 32-bit add, from their
 //            real-disparity offset.  The two have one parent and so one
 //            offset, and share all but two of their window rows.
+// Later passes of a tile hold few pixels: only the rows and the column
+// halves with pixels of the cluster are staged and summed.
 // Window sums are exact integers (at most 25 * 255 here, no intermediate
-// clamp in the reference).  Tiles whose parents disagree more widely take a
-// pass per cluster of bases; what is left after kTiClusters of them, wider
-// windows and more than kTiRn labels evaluate each window directly.
+// clamp in the reference).  What is left after kTiClusters passes and wider
+// windows evaluate each window directly.
+// Bound by instruction issue (seven instructions a cost; 52 % of the slots
+// with two disparities a lane, which kept the shared-memory pipe at 64 %).
 // ---------------------------------------------------------------------------
-constexpr int kTiX = 32, kTiY = 16, kTiRn = 32, kTiMaxHalf = 2;
+constexpr int kTiX = 32, kTiY = 16, kTiMaxHalf = 2;
+constexpr int kTiD = 16;         // labels of a pass
+constexpr int kTiRn = 28;        // real disparities of a cluster
 constexpr int kTiWarps = 8;
 constexpr int kTiClusters = 8;   // passes of a tile
 constexpr int kTiRows = kTiY + 2 * kTiMaxHalf;      // window rows at most
-constexpr int kTiRs = kTiRn + 2;   // halves per (row, column): 17 words, odd, so columns hit distinct banks
+// Sums along x of a row: 14 words a column (7 pairs of words, odd, so that
+// the columns' 8-byte reads hit distinct banks), the rows 10 words further
+// (5 pairs: the writes of the lanes of five quads and three rows do too).
+constexpr int kTiCs = kTiRn / 2, kTiRowS = kTiX * kTiCs + 10;
+constexpr int kTiSeg = kTiX / 2;                    // columns a lane walks (without the window's border)
 constexpr int kTiSL = kTiX + 2 * kTiMaxHalf;        // staged left features per window row
-constexpr int kTiSR = kTiSL + kTiRn - 1;            // staged right features per window row
-constexpr size_t kTiHs = (size_t)kTiRows * kTiX * kTiRs * 2;
+// Staged right features: pixel p of a row at (p & 3) * kTiSub + (p >> 2), so
+// that lanes of adjacent quads read adjacent ones.
+constexpr int kTiSub = 17, kTiSR = 4 * kTiSub - 1;
+constexpr size_t kTiHs = (size_t)kTiRows * kTiRowS * 4;
 constexpr size_t kTiSmem = kTiHs + (size_t)kTiRows * (kTiSL + kTiSR) * 16;
+static_assert(kTiHs % 16 == 0, "the staged features are 16-byte aligned");
+static_assert((kTiSL + kTiRn - 2) / 4 < kTiSub, "the right features of a row fit");
+static_assert(kTiD + kTiRn % 4 <= kTiRn && kTiRn % 4 == 0, "whole quads");
 
-// Sums along x, for a cluster of real disparities rmin .. rmin + rn - 1,
-// of every window row of the tile (see above).
+// The part of a tile that a cluster's pixels cover.
+struct TileArea {
+    int r0, nr;     // window rows
+    int seg0, ns;   // column halves
+};
+
+// Sums along x, for the 4 nq real disparities from rmin on, of the window
+// rows and column halves of `a` (see above).
 template <int HW>
-__device__ __forceinline__ void bt_row_sums(const LevelDesc& J, uint16_t* hs, uint4* st, int x0, int y0, int rmin,
-                                            int rn, int warp, int lane)
+__device__ __forceinline__ void bt_row_sums(const LevelDesc& J, uint32_t* hs, uint4* st, int x0, int y0, int rmin,
+                                            int nq, const TileArea& a, int warp, int lane)
 {
-    constexpr int R = kTiY + 2 * HW;     // window rows
     constexpr int SW = kTiX + 2 * HW;    // window columns
+    constexpr int NC = kTiSeg + 2 * HW;  // ... of a half
     constexpr int Q = HW > 0 ? 2 * HW : 1;
     const int W = J.w, H = J.h;
     uint4* sl = st;                      // [R][kTiSL]  left, columns x0 - HW + j (clamped)
-    uint4* sr = st + kTiRows * kTiSL;    // [R][kTiSR]  right, columns xrs + k
-    const int xrs = x0 - HW - (rmin + rn - 1);
-    const int nsr = SW + rn - 1;
-    for (int r = warp; r < R; r += kTiWarps) {
+    uint4* sr = st + kTiRows * kTiSL;    // [R][kTiSR]  right, columns xrs + p
+    const int xrs = x0 - HW - (rmin + 4 * nq - 1);
+    const int nsr = SW + 4 * nq - 1;
+    for (int r = a.r0 + warp; r < a.r0 + a.nr; r += kTiWarps) {
         const size_t grow = (size_t)iclamp(y0 - HW + r, 0, H - 1) * W;
         for (int j = lane; j < SW; j += 32)
             tile_cp16(sl + r * kTiSL + j, J.featL + grow + iclamp(x0 - HW + j, 0, W - 1));
-        for (int k = lane; k < nsr; k += 32) {
-            const int xx = xrs + k;
-            if (xx >= 0 && xx < W) tile_cp16(sr + r * kTiSR + k, J.featR + grow + xx);
-            else sr[r * kTiSR + k] = bt_outside();
+        uint4* o = sr + r * kTiSR + (lane & 3) * kTiSub + (lane >> 2);
+        for (int p = lane; p < nsr; p += 32, o += 8) {
+            const int xx = xrs + p;
+            if (xx >= 0 && xx < W) tile_cp16(o, J.featR + grow + xx);
+            else *o = bt_outside();
         }
     }
     tile_commit_wait();
     __syncthreads();
     // no window column is clamped
     const bool interior = x0 - HW >= 0 && x0 + kTiX - 1 + HW < W;
-    // Units: (window row, real-disparity pair ri, ri + 1), numbered
-    // row-major, one per lane.  Real disparity ri + 1 needs at window column
-    // j the right feature that ri needed at column j - 1, so a lane loads
-    // one left and one right feature per column for two sums and stores both
-    // as one word.  With rn odd the last pair's second half is past the
-    // cluster: computed, never read.
-    const int rp = (rn + 1) >> 1;
-    const int pairs = R * rp;
-    for (int f0 = warp * 32; f0 < pairs; f0 += kTiWarps * 32) {
-        const int f = f0 + lane;
-        const bool on = f < pairs;
-        const int fr = on ? f : pairs - 1;
-        const int row = fr / rp, ri = 2 * (fr - row * rp);
-        const uint4* lrow = sl + row * kTiSL;
+    const int units = a.nr * nq * a.ns;
+    for (int f = warp * 32 + lane; f < units; f += kTiWarps * 32) {
+        const int t = f / nq, q = f - t * nq;
+        const bool second = t >= a.nr;
+        const int row = a.r0 + (second ? t - a.nr : t), j0 = (a.seg0 + (second ? 1 : 0)) * kTiSeg;
+        const uint4* lp = sl + row * kTiSL + j0;
         const uint4* rrow = sr + row * kTiSR;
-        uint32_t* out = reinterpret_cast<uint32_t*>(hs + (size_t)row * kTiX * kTiRs + ri);
-        uint32_t h[Q], s = 0;   // the last 2 HW costs; their sum
+        uint2* out = reinterpret_cast<uint2*>(hs + row * kTiRowS + j0 * kTiCs + 2 * q);
+        uint32_t h0[Q], h1[Q], s0 = 0, s1 = 0;   // the last 2 HW costs; their sums
 #pragma unroll
-        for (int i = 0; i < Q; ++i) h[i] = 0;
-        auto column = [&](int j, int u, uint32_t e0, uint32_t e1) {
-            const uint32_t p = e0 | (e1 << 16);
-            s += p;
-            if (j >= 2 * HW && on) out[(j - 2 * HW) * (kTiRs / 2)] = s;
-            s -= HW > 0 ? h[u % Q] : p;
-            h[u % Q] = p;
+        for (int i = 0; i < Q; ++i) h0[i] = h1[i] = 0;
+        // add the four costs of window column j of the half (u: its place in the turn)
+        auto column = [&](int j, int u, const uint32_t (&e)[4]) {
+            const uint32_t p0 = e[0] | (e[1] << 16), p1 = e[2] | (e[3] << 16);
+            s0 += p0;
+            s1 += p1;
+            if (j >= 2 * HW) {
+                *out = make_uint2(s0, s1);
+                out += kTiCs / 2;
+            }
+            s0 -= HW > 0 ? h0[u % Q] : p0;
+            s1 -= HW > 0 ? h1[u % Q] : p1;
+            h0[u % Q] = p0;
+            h1[u % Q] = p1;
         };
         if (interior) {
-            // right feature of window column j for ri: srl[j]; for ri + 1: srl[j - 1]
-            const uint4* srl = rrow - ri + rn - 1;
-            uint4 rprev = ri + 1 < rn ? srl[-1] : bt_outside();
+            // disparity rmin + 4 q + i needs right pixel j0 + 4 (nq - q) - 1 + j - i at column j
+            const uint4* rp = rrow + (j0 >> 2) + nq - 1 - q;
+            uint4 win[4];   // right pixel p at p & 3
+#pragma unroll
+            for (int i = 1; i < 4; ++i) win[(3 - i) & 3] = rp[((3 - i) & 3) * kTiSub];
 #pragma unroll 1
-            for (int j0 = 0; j0 < SW; j0 += 4) {
+            for (int j = 0; j < NC; j += 4) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    if (SW % 4 != 0 && j0 + u >= SW) break;
-                    const uint4 l = lrow[j0 + u], r = srl[j0 + u];
-                    column(j0 + u, u, bt_pixel(l, r), bt_pixel(l, rprev));
-                    rprev = r;
+                    if (NC % 4 != 0 && j + u >= NC) break;
+                    const uint4 l = lp[j + u];
+                    win[(3 + u) & 3] = rp[((3 + u) & 3) * kTiSub + ((3 + u) >> 2)];
+                    uint32_t e[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) e[i] = bt_pixel(l, win[(3 + u - i) & 3]);
+                    column(j + u, u, e);
                 }
+                ++rp;
             }
         } else {
 #pragma unroll 1
-            for (int j0 = 0; j0 < SW; j0 += Q) {
+            for (int j = 0; j < NC; j += Q) {
 #pragma unroll
                 for (int u = 0; u < Q; ++u) {
-                    const int k = iclamp(x0 - HW + j0 + u, 0, W - 1) - (rmin + ri) - xrs;
-                    const uint4 l = lrow[j0 + u];
-                    column(j0 + u, u, bt_pixel(l, rrow[k]), bt_pixel(l, rrow[imax(k - 1, 0)]));
+                    const int p = iclamp(x0 - HW + j0 + j + u, 0, W - 1) - (rmin + 4 * q) - xrs;
+                    const uint4 l = lp[j + u];
+                    uint32_t e[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) e[i] = bt_pixel(l, rrow[((p - i) & 3) * kTiSub + ((p - i) >> 2)]);
+                    column(j + u, u, e);
                 }
             }
         }
@@ -809,10 +839,10 @@ __global__ void __launch_bounds__(256, 3) k_cost_bt_tiled(const __grid_constant_
     const int x0 = blockIdx.x * kTiX, y0 = blockIdx.y * kTiY;
     if (x0 >= J.w || y0 >= J.h) return;
     const int W = J.w, H = J.h, D = J.D, h = J.bs / 2;
-    extern __shared__ __align__(16) uint16_t hs[];   // [kTiRows][kTiX][kTiRs], then the staged features
+    extern __shared__ __align__(16) uint32_t hs[];   // [kTiRows] rows of sums, then the staged features
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint4* stg = reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(hs) + kTiHs);
-    __shared__ int wred[2][kTiWarps];
+    __shared__ int wred[3][kTiWarps];
     // a thread's two pixels: (x0 + lane, y0 + 2 warp) and the one below
     const int x = x0 + lane;
     int yq[2], bq[2];
@@ -824,157 +854,178 @@ __global__ void __launch_bounds__(256, 3) k_cost_bt_tiled(const __grid_constant_
         bq[i] = inq[i] ? (int)J.base[(size_t)yq[i] * W + x] : (int)kNoParent;
         hasq[i] = inq[i] && bq[i] != kNoParent;
     }
-    auto block_minmax = [&](bool in0, bool in1, int& mn, int& mx) {
+    // lowest and highest base of the pixels in0, in1, and where they lie
+    auto block_minmax = [&](bool in0, bool in1, int& mn, int& mx, TileArea& area) {
         const int a = __reduce_min_sync(0xffffffffu, imin(in0 ? bq[0] : INT_MAX, in1 ? bq[1] : INT_MAX));
         const int z = __reduce_max_sync(0xffffffffu, imax(in0 ? bq[0] : INT_MIN, in1 ? bq[1] : INT_MIN));
+        const unsigned m = __ballot_sync(0xffffffffu, in0 || in1);
         __syncthreads();   // wred reused
-        if (lane == 0) { wred[0][warp] = a; wred[1][warp] = z; }
+        if (lane == 0) { wred[0][warp] = a; wred[1][warp] = z; wred[2][warp] = (int)m; }
         __syncthreads();
         mn = INT_MAX;
         mx = INT_MIN;
+        unsigned cols = 0;
+        int first = kTiWarps, last = 0;
 #pragma unroll
-        for (int i = 0; i < kTiWarps; ++i) { mn = imin(mn, wred[0][i]); mx = imax(mx, wred[1][i]); }
+        for (int i = 0; i < kTiWarps; ++i) {
+            mn = imin(mn, wred[0][i]);
+            mx = imax(mx, wred[1][i]);
+            const unsigned c = (unsigned)wred[2][i];
+            cols |= c;
+            if (c) { first = imin(first, i); last = i; }
+        }
+        area.r0 = 2 * first;
+        area.nr = 2 * (last - first + 1) + 2 * h;
+        area.seg0 = (cols & 0xffffu) ? 0 : 1;
+        area.ns = (cols & 0xffffu) && (cols >> 16) ? 2 : 1;
     };
     const bool vec = (D & 7) == 0;
-    // Clusters of bases, lowest first: the pixels whose real disparities lie
-    // within kTiRn of the lowest one left.  11-26 % of the tiles of a 1080p
-    // scene hold a depth edge or a wild parent and need more than one; a
-    // pass costs less than the window sums of a few pixels, and two passes
-    // at most left 1-2 % of the pixels to those (a seventh of the kernel's
-    // instructions, in blocks that outlasted the others).
-    bool todo[2] = {hasq[0] && h <= kTiMaxHalf && D <= kTiRn, hasq[1] && h <= kTiMaxHalf && D <= kTiRn};
-    for (int c = 0; c < kTiClusters; ++c) {
-        int rmin, top;
-        block_minmax(todo[0], todo[1], rmin, top);
-        if (top == INT_MIN) break;
-        if (top + D - rmin > kTiRn) {
-            const int last = rmin + kTiRn - D;
-            int lowest;
-            block_minmax(todo[0] && bq[0] <= last, todo[1] && bq[1] <= last, lowest, top);
-        }
-        const int rn = top + D - rmin;
-        const bool mine[2] = {todo[0] && bq[0] <= top, todo[1] && bq[1] <= top};
-        if (h == 2) bt_row_sums<2>(J, hs, stg, x0, y0, rmin, rn, warp, lane);
-        else if (h == 1) bt_row_sums<1>(J, hs, stg, x0, y0, rmin, rn, warp, lane);
-        else bt_row_sums<0>(J, hs, stg, x0, y0, rmin, rn, warp, lane);
-        __syncthreads();
-        // packed pair sums of 2h+1 rows from offset ri0 = b - rmin (halves),
-        // 8 labels per chunk
-        auto put = [&](int i, int d0, const uint32_t (&acc)[5], uint32_t sh, int lo, int hi) {
-            int16_t* out = J.C + ((size_t)yq[i] * W + x) * D;
-            if (!PG_IN(((size_t)yq[i] * W + x) * D, D, (size_t)W * H * D, 11)) return;
-            uint32_t w[4];
+    for (int dc = 0; dc < D; dc += kTiD) {
+        const int nd = imin(kTiD, D - dc);
+        // Clusters of bases, lowest first: the pixels whose real disparities
+        // lie within kTiRn of the lowest one left.  11-26 % of the tiles of a
+        // 1080p scene hold a depth edge or a wild parent and need more than
+        // one; a pass costs less than the window sums of a few pixels, and
+        // two passes at most left 1-2 % of the pixels to those (a seventh of
+        // the kernel's instructions, in blocks that outlasted the others).
+        bool todo[2] = {hasq[0] && h <= kTiMaxHalf, hasq[1] && h <= kTiMaxHalf};
+        for (int c = 0; c < kTiClusters; ++c) {
+            int low, top;
+            TileArea area;
+            block_minmax(todo[0], todo[1], low, top, area);
+            if (top == INT_MIN) break;
+            if (top + nd - low > kTiRn) {
+                const int last = low + kTiRn - nd;
+                int lowest;
+                block_minmax(todo[0] && bq[0] <= last, todo[1] && bq[1] <= last, lowest, top, area);
+            }
+            const int rmin = low + dc, nq = (top + nd - low + 3) >> 2;
+            const bool mine[2] = {todo[0] && bq[0] <= top, todo[1] && bq[1] <= top};
+            if (h == 2) bt_row_sums<2>(J, hs, stg, x0, y0, rmin, nq, area, warp, lane);
+            else if (h == 1) bt_row_sums<1>(J, hs, stg, x0, y0, rmin, nq, area, warp, lane);
+            else bt_row_sums<0>(J, hs, stg, x0, y0, rmin, nq, area, warp, lane);
+            __syncthreads();
+            // the 16 labels of pixel i from its pair sums, which start
+            // `off` (0 to 3) halves before its first label
+            auto put = [&](int i, uint32_t (&acc)[10], int off, int lo, int hi) {
+                int16_t* out = J.C + ((size_t)yq[i] * W + x) * D + dc;
+                if (!PG_IN(((size_t)yq[i] * W + x) * D, D, (size_t)W * H * D, 11)) return;
+                const bool two = off & 2;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) w[q] = __funnelshift_r(acc[q], acc[q + 1], sh);
-            if (lo > d0 || hi < d0 + 7) {
+                for (int q = 0; q < 9; ++q) acc[q] = two ? acc[q + 1] : acc[q];
+                const uint32_t sh = (uint32_t)(off & 1) * 16;
+                uint32_t w[8];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int d = d0 + 2 * q;
-                    if (d < lo || d > hi) w[q] = (w[q] & 0xffff0000u) | (uint32_t)kMax;
-                    if (d + 1 < lo || d + 1 > hi) w[q] = (w[q] & 0xffffu) | ((uint32_t)kMax << 16);
+                for (int q = 0; q < 8; ++q) w[q] = __funnelshift_r(acc[q], acc[q + 1], sh);
+                if (lo > dc || hi < dc + nd - 1) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const int d = dc + 2 * q;
+                        if (d < lo || d > hi) w[q] = (w[q] & 0xffff0000u) | (uint32_t)kMax;
+                        if (d + 1 < lo || d + 1 > hi) w[q] = (w[q] & 0xffffu) | ((uint32_t)kMax << 16);
+                    }
                 }
-            }
-            if (vec) {
-                reinterpret_cast<uint4*>(out + d0)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-            } else {
-                for (int q = 0; q < 8 && d0 + q < D; ++q)
-                    out[d0 + q] = (int16_t)((w[q >> 1] >> ((q & 1) * 16)) & 0xffffu);
-            }
-        };
-        auto rowsum = [&](int k, int col) {   // window row k, words from half `col`
-            return reinterpret_cast<const uint32_t*>(hs + (k * kTiX + lane) * kTiRs) + (col >> 1);
-        };
-        if (mine[0] && mine[1] && bq[0] == bq[1]) {
-            int lo, hi;
-            label_range(J, x, bq[0], lo, hi);
-            const int ri0 = bq[0] - rmin;
-            const uint32_t sh = (uint32_t)(ri0 & 1) * 16;
-            for (int d0 = 0; d0 < D; d0 += 8) {
-                uint32_t top[5], bot[5];
-                const uint32_t* r0 = rowsum(2 * warp, ri0 + d0);
-                const uint32_t* r1 = rowsum(2 * warp + 2 * h + 1, ri0 + d0);
+                if (vec) {
+                    reinterpret_cast<uint4*>(out)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                    if (nd > 8) reinterpret_cast<uint4*>(out)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 16; ++q)
+                        if (q < nd) out[q] = (int16_t)((w[q >> 1] >> ((q & 1) * 16)) & 0xffffu);
+                }
+            };
+            auto rowsum = [&](int k, int o, uint32_t (&v)[10]) {   // window row k, from disparity offset o & ~3
+                const uint2* p = reinterpret_cast<const uint2*>(hs + k * kTiRowS + lane * kTiCs) + (o >> 2);
 #pragma unroll
                 for (int j = 0; j < 5; ++j) {
-                    top[j] = r0[j];
-                    bot[j] = r1[j];
+                    const uint2 a = p[j];
+                    v[2 * j] = a.x;
+                    v[2 * j + 1] = a.y;
                 }
-                for (int k = 1; k <= 2 * h; ++k) {   // the rows both windows hold
-                    const uint32_t* row = rowsum(2 * warp + k, ri0 + d0);
-#pragma unroll
-                    for (int j = 0; j < 5; ++j) {
-                        const uint32_t v = row[j];
-                        top[j] += v;
-                        bot[j] += v;
-                    }
-                }
-                put(0, d0, top, sh, lo, hi);
-                put(1, d0, bot, sh, lo, hi);
-            }
-        } else {
-#pragma unroll 1
-            for (int i = 0; i < 2; ++i) {
-                if (!(i ? mine[1] : mine[0])) continue;
-                const int bb = i ? bq[1] : bq[0];
+            };
+            if (mine[0] && mine[1] && bq[0] == bq[1]) {
                 int lo, hi;
-                label_range(J, x, bb, lo, hi);
-                const uint32_t sh = (uint32_t)((bb - rmin) & 1) * 16;
-                for (int d0 = 0; d0 < D; d0 += 8) {
-                    uint32_t acc[5] = {0u, 0u, 0u, 0u, 0u};
-                    for (int k = 0; k <= 2 * h; ++k) {
-                        const uint32_t* row = rowsum(2 * warp + i + k, bb - rmin + d0);
+                label_range(J, x, bq[0], lo, hi);
+                const int o = bq[0] - low;
+                uint32_t above[10], below[10];
+                rowsum(2 * warp, o, above);
+                rowsum(2 * warp + 2 * h + 1, o, below);
+                for (int k = 1; k <= 2 * h; ++k) {   // the rows both windows hold
+                    uint32_t v[10];
+                    rowsum(2 * warp + k, o, v);
 #pragma unroll
-                        for (int j = 0; j < 5; ++j) acc[j] += row[j];
+                    for (int j = 0; j < 10; ++j) {
+                        above[j] += v[j];
+                        below[j] += v[j];
                     }
-                    if (i) put(1, d0, acc, sh, lo, hi);
-                    else put(0, d0, acc, sh, lo, hi);
+                }
+                put(0, above, o & 3, lo, hi);
+                put(1, below, o & 3, lo, hi);
+            } else {
+#pragma unroll 1
+                for (int i = 0; i < 2; ++i) {
+                    if (!(i ? mine[1] : mine[0])) continue;
+                    const int bb = i ? bq[1] : bq[0];
+                    int lo, hi;
+                    label_range(J, x, bb, lo, hi);
+                    uint32_t acc[10];
+                    rowsum(2 * warp + i, bb - low, acc);
+                    for (int k = 1; k <= 2 * h; ++k) {
+                        uint32_t v[10];
+                        rowsum(2 * warp + i + k, bb - low, v);
+#pragma unroll
+                        for (int j = 0; j < 10; ++j) acc[j] += v[j];
+                    }
+                    if (i) put(1, acc, (bb - low) & 3, lo, hi);
+                    else put(0, acc, (bb - low) & 3, lo, hi);
                 }
             }
+            todo[0] = todo[0] && !mine[0];
+            todo[1] = todo[1] && !mine[1];
+            // (the next cluster's reductions come before its row sums overwrite hs)
         }
-        todo[0] = todo[0] && !mine[0];
-        todo[1] = todo[1] && !mine[1];
-        // (the next cluster's reductions come before its row sums overwrite hs)
-    }
-    // direct window per pixel (no parent, or in no cluster)
+        // direct window per pixel (no parent, or in no cluster)
 #pragma unroll 1
-    for (int i = 0; i < 2; ++i) {
-        const bool in = i ? inq[1] : inq[0], has = i ? hasq[1] : hasq[0], left = i ? todo[1] : todo[0];
-        const bool wide = h > kTiMaxHalf || D > kTiRn;   // no clusters at all
-        if (!in || (has && !left && !wide)) continue;
-        const int y = i ? yq[1] : yq[0], b = i ? bq[1] : bq[0];
-        int lo, hi;
-        label_range(J, x, b, lo, hi);
-        int16_t* out = J.C + ((size_t)y * W + x) * D;
-        for (int d0 = 0; d0 < D; d0 += 8) {
-            int sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            if (b != kNoParent) {
-                for (int dy = -h; dy <= h; ++dy) {
-                    const int gy = iclamp(y + dy, 0, H - 1);
-                    const uint4* lrow = J.featL + (size_t)gy * W;
-                    const uint4* rrow = J.featR + (size_t)gy * W;
-                    for (int dx = -h; dx <= h; ++dx) {
-                        const int gx = iclamp(x + dx, 0, W - 1);
-                        const uint4 lf = __ldg(&lrow[gx]);
-#pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            const int x2 = gx - (b + d0 + q);
-                            sum[q] += (x2 >= 0 && x2 < W) ? (int)bt_pixel(lf, __ldg(&rrow[x2])) : 255;
+        for (int i = 0; i < 2; ++i) {
+            const bool in = i ? inq[1] : inq[0], has = i ? hasq[1] : hasq[0], left = i ? todo[1] : todo[0];
+            const bool wide = h > kTiMaxHalf;   // no clusters at all
+            if (!in || (has && !left && !wide)) continue;
+            const int y = i ? yq[1] : yq[0], b = i ? bq[1] : bq[0];
+            int lo, hi;
+            label_range(J, x, b, lo, hi);
+            int16_t* out = J.C + ((size_t)y * W + x) * D;
+            for (int d0 = dc; d0 < dc + nd; d0 += 8) {
+                int sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                if (b != kNoParent) {
+                    for (int dy = -h; dy <= h; ++dy) {
+                        const int gy = iclamp(y + dy, 0, H - 1);
+                        const uint4* lrow = J.featL + (size_t)gy * W;
+                        const uint4* rrow = J.featR + (size_t)gy * W;
+                        for (int dx = -h; dx <= h; ++dx) {
+                            const int gx = iclamp(x + dx, 0, W - 1);
+                            const uint4 lf = __ldg(&lrow[gx]);
+    #pragma unroll
+                            for (int q = 0; q < 8; ++q) {
+                                const int x2 = gx - (b + d0 + q);
+                                sum[q] += (x2 >= 0 && x2 < W) ? (int)bt_pixel(lf, __ldg(&rrow[x2])) : 255;
+                            }
                         }
                     }
                 }
-            }
-            uint32_t w[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int d = d0 + 2 * q;
-                const uint32_t v0 = (d >= lo && d <= hi) ? (uint32_t)imin(sum[2 * q], kMax - 1) : (uint32_t)kMax;
-                const uint32_t v1 =
-                    (d + 1 >= lo && d + 1 <= hi) ? (uint32_t)imin(sum[2 * q + 1], kMax - 1) : (uint32_t)kMax;
-                w[q] = v0 | (v1 << 16);
-            }
-            if (vec) {
-                reinterpret_cast<uint4*>(out + d0)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-            } else {
-                for (int q = 0; q < 8 && d0 + q < D; ++q) out[d0 + q] = (int16_t)((w[q >> 1] >> ((q & 1) * 16)) & 0xffffu);
+                uint32_t w[4];
+    #pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int d = d0 + 2 * q;
+                    const uint32_t v0 = (d >= lo && d <= hi) ? (uint32_t)imin(sum[2 * q], kMax - 1) : (uint32_t)kMax;
+                    const uint32_t v1 =
+                        (d + 1 >= lo && d + 1 <= hi) ? (uint32_t)imin(sum[2 * q + 1], kMax - 1) : (uint32_t)kMax;
+                    w[q] = v0 | (v1 << 16);
+                }
+                if (vec) {
+                    reinterpret_cast<uint4*>(out + d0)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                } else {
+                    for (int q = 0; q < 8 && d0 + q < D; ++q) out[d0 + q] = (int16_t)((w[q >> 1] >> ((q & 1) * 16)) & 0xffffu);
+                }
             }
         }
     }
