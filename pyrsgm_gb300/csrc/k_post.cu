@@ -49,19 +49,21 @@ __device__ __forceinline__ uint32_t median9(const Col3& a, const Col3& b, const 
     return med3(__vimax3_s16x2(a.lo, b.lo, c.lo), med3(a.mid, b.mid, c.mid), __vimin3_s16x2(a.hi, b.hi, c.hi));
 }
 
-// One block: 128 x 8 pixels, a warp per row, a thread per 4 adjacent pixels.
-// The (LR-checked) disparities of the tile and a halo of one row and four
-// columns are computed once into shared memory, four pixels at a time, in
-// three rounds so that a thread's loads overlap: raw disparities, the disp2
-// keys they point at, decisions; the confidences are loaded before all of
-// them.  The median takes the in-image neighbours only (sorted, middle
-// element) at the image border.  Instruction bound before (280 a pixel, 33
-// us on a 1080p level), latency bound below.
+// One block: 128 x 8 pixels.  The (LR-checked) disparities of the tile and a
+// halo of one row and four columns are computed once into shared memory, a
+// thread per 4 adjacent pixels: 340 of the block's 352 threads (256 threads in
+// two rounds spent the second one on a third of them).  Loads come first, in
+// three rounds so that they overlap: confidences and raw disparities, the
+// disp2 keys they point at, decisions.  Then 8 warps take a row each, 4
+// pixels a thread; the median takes the in-image neighbours only (sorted,
+// middle element) at the image border.  Bound by the latency of the dependent
+// loads and by instruction issue (32 levels of 1080p: 496 -> 433 us).
 constexpr int kPoX = 128, kPoY = 8;
 constexpr int kPoG = kPoX / 4 + 2;   // groups of 4 pixels per staged row: columns x0 - 4 .. x0 + 131
+constexpr int kPoN = (kPoY + 2) * kPoG, kPoThreads = (kPoN + 31) / 32 * 32;
 
 template <int NJ>
-__global__ void __launch_bounds__(256) k_post(const __grid_constant__ Jobs<NJ> jobs)
+__global__ void __launch_bounds__(kPoThreads) k_post(const __grid_constant__ Jobs<NJ> jobs)
 {
     let_next_in();
     after_previous();
@@ -77,7 +79,7 @@ __global__ void __launch_bounds__(256) k_post(const __grid_constant__ Jobs<NJ> j
     const bool quad = (W & 3) == 0;   // rows of raw disparities and confidences start on 4-pixel boundaries
     const int tx = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int xb = x0 + 4 * tx, y = y0 + warp;
-    const int np = y < H ? imin(4, W - xb) : 0;
+    const int np = warp < kPoY && y < H ? imin(4, W - xb) : 0;
     __shared__ __align__(16) uint2 td[kPoY + 2][kPoG];   // row r, group g: pixels x0 - 4 + 4 g .. of row y0 - 1 + r
     float cin[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (np > 0) {
@@ -91,82 +93,82 @@ __global__ void __launch_bounds__(256) k_post(const __grid_constant__ Jobs<NJ> j
                 if (j < np) cin[j] = __ldg(c + j);
         }
     }
-    {
-        constexpr int kN = (kPoY + 2) * kPoG, kPer = (kN + 255) / 256;
-        int dv[kPer][4], xg[kPer], rowp[kPer];   // (a level has far fewer than 2^31 pixels)
+    if (threadIdx.x < kPoN) {
+        const int r = threadIdx.x / kPoG, g = threadIdx.x - r * kPoG;
+        const int yy = y0 - 1 + r, xg = x0 - 4 + 4 * g;
+        const bool in = yy >= 0 && yy < H && xg >= 0 && xg < W;
+        const uint32_t inv2 = (uint32_t)(uint16_t)inv * 0x10001u;
+        uint2 a = make_uint2(inv2, inv2);   // the four disparities
+        if (in) {
+            const int16_t* p = J.disp_raw + (size_t)yy * W + xg;
+            if (quad) {
+                a = __ldg(reinterpret_cast<const uint2*>(p));
+            } else {
+                uint32_t v[4];
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const int i = threadIdx.x + 256 * k;
-            const int r = i / kPoG, g = i - r * kPoG;
-            const int yy = y0 - 1 + r;
-            xg[k] = x0 - 4 + 4 * g;
-            const bool in = i < kN && yy >= 0 && yy < H && xg[k] >= 0 && xg[k] < W;
-            rowp[k] = in ? yy * W : -1;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) dv[k][j] = inv;
-            if (in) {
-                const int16_t* p = J.disp_raw + (size_t)rowp[k] + xg[k];
-                if (quad) {
-                    const uint2 a = __ldg(reinterpret_cast<const uint2*>(p));
-                    dv[k][0] = (int)(int16_t)(a.x & 0xffffu);
-                    dv[k][1] = (int)(int16_t)(a.x >> 16);
-                    dv[k][2] = (int)(int16_t)(a.y & 0xffffu);
-                    dv[k][3] = (int)(int16_t)(a.y >> 16);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (xg[k] + j < W) dv[k][j] = (int)__ldg(p + j);
-                }
+                for (int j = 0; j < 4; ++j) v[j] = xg + j < W ? (uint32_t)(uint16_t)__ldg(p + j) : (uint32_t)(uint16_t)inv;
+                a = make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
             }
         }
-        if (check) {
-            // The key of right pixel rx holds 0xffff - x' of its winner x'
-            // (all ones: none); the winner's disparity there is x' - rx, and
+        if (check && in) {
+            // The key of right pixel rx holds the cost and 0xffff - x' of its
+            // winner x' (all ones: none); the winner's disparity there is x' - rx, and
             // rx + d0 = x, so that disp2 - d0 = x' - x.  A right pixel
             // without a winner has disparity `inv` in the reference, which
             // counts where it is not below minD (minD > 1).
-            unsigned k0[kPer][4], k1[kPer][4];
-#pragma unroll
-            for (int k = 0; k < kPer; ++k)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    k0[k][j] = k1[k][j] = 0xffffffffu;
-                    if (rowp[k] >= 0 && dv[k][j] != inv) {
-                        const int x = xg[k] + j, r0 = x - (dv[k][j] >> 4), r1 = x - ((dv[k][j] + 15) >> 4);
-                        const unsigned* row = J.keys + (size_t)rowp[k];
-                        if ((unsigned)r0 < (unsigned)W) k0[k][j] = __ldg(row + r0);
-                        if ((unsigned)r1 < (unsigned)W) k1[k][j] = __ldg(row + r1);
-                    }
-                }
-            const bool pyr = J.pyr != 0, none_counts = inv >= J.minD;
+            const unsigned* row = J.keys + (size_t)yy * W;
             const int maxdiff = J.maxdiff;
+            unsigned k0[4], k1[4];
 #pragma unroll
-            for (int k = 0; k < kPer; ++k)
+            for (int j = 0; j < 4; ++j) {
+                const int d = (int)(int16_t)(j < 2 ? a.x >> (16 * j) : a.y >> (16 * (j - 2)));
+                const int r0 = xg + j - (d >> 4), r1 = xg + j - ((d + 15) >> 4);
+                k0[j] = k1[j] = 0xffffffffu;
+                if ((unsigned)r0 < (unsigned)W) k0[j] = __ldg(row + r0);
+                if ((unsigned)r1 < (unsigned)W) k1[j] = __ldg(row + r1);
+            }
+            bool bad[4];
+            if (inv < J.minD && maxdiff >= 0 && maxdiff <= 65536) {
+                // |x' - x| <= maxdiff as one unsigned comparison; the top bit
+                // (a cost never has it) keeps no winner far from any x
+                const unsigned span = 2u * (unsigned)maxdiff;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const int x = xg[k] + j;
-                    bool on0 = k0[k][j] != 0xffffffffu, on1 = k1[k][j] != 0xffffffffu;
-                    int e0 = abs((int)(~k0[k][j] & 0xffffu) - x), e1 = abs((int)(~k1[k][j] & 0xffffu) - x);
+                    const unsigned c = (unsigned)(0xffff + maxdiff - xg - j);
+                    const bool far0 = c - (k0[j] & 0x8000ffffu) > span, far1 = c - (k1[j] & 0x8000ffffu) > span;
+                    bad[j] = far0 && far1 && (J.pyr || (k0[j] != 0xffffffffu && k1[j] != 0xffffffffu));
+                }
+            } else {
+                const bool none_counts = inv >= J.minD;
+#pragma unroll 1
+                for (int j = 0; j < 4; ++j) {
+                    const int d = (int)(int16_t)(j < 2 ? a.x >> (16 * j) : a.y >> (16 * (j - 2)));
+                    const int x = xg + j, d0 = d >> 4, d1 = (d + 15) >> 4;
+                    const unsigned q0 = k0[0], q1 = k1[0];
+                    bool on0 = q0 != 0xffffffffu, on1 = q1 != 0xffffffffu;
+                    int e0 = abs((int)(~q0 & 0xffffu) - x), e1 = abs((int)(~q1 & 0xffffu) - x);
                     if (none_counts) {
-                        const int d0 = dv[k][j] >> 4, d1 = (dv[k][j] + 15) >> 4;
                         if (!on0) e0 = abs(inv - d0);
                         if (!on1) e1 = abs(inv - d1);
                         on0 = (unsigned)(x - d0) < (unsigned)W;
                         on1 = (unsigned)(x - d1) < (unsigned)W;
                     }
-                    const bool bad = pyr ? !((on0 && e0 <= maxdiff) || (on1 && e1 <= maxdiff))
+                    const bool b = J.pyr ? !((on0 && e0 <= maxdiff) || (on1 && e1 <= maxdiff))
                                          : (on0 && e0 > maxdiff) && (on1 && e1 > maxdiff);
-                    if (bad) dv[k][j] = inv;
-                }
-        }
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const int i = threadIdx.x + 256 * k;
-            if (i < kN)
-                (&td[0][0])[i] = make_uint2(__byte_perm(dv[k][0], dv[k][1], 0x5410), __byte_perm(dv[k][2], dv[k][3], 0x5410));
+                    for (int i = 0; i < 3; ++i) { k0[i] = k0[i + 1]; k1[i] = k1[i + 1]; bad[i] = bad[i + 1]; }
+                    bad[3] = b;
+                }
+            }
+            // (an invalid disparity stays what it is)
+            if (bad[0]) a.x = __byte_perm(a.x, inv2, 0x3254);
+            if (bad[1]) a.x = __byte_perm(a.x, inv2, 0x5410);
+            if (bad[2]) a.y = __byte_perm(a.y, inv2, 0x3254);
+            if (bad[3]) a.y = __byte_perm(a.y, inv2, 0x5410);
         }
-        __syncthreads();
+        (&td[0][0])[threadIdx.x] = a;
     }
+    __syncthreads();
     if (np <= 0) return;
     uint2 d = td[warp + 1][tx + 1], m = d;   // checked disparities, median
     if (med) {
@@ -254,7 +256,7 @@ cudaError_t launch_post(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t
 {
     dim3 g((e.max_w + kPoX - 1) / kPoX, (e.max_h + kPoY - 1) / kPoY, jobs.n);
     prof_begin(st);
-    launch_after(k_post<NJ>, g, 256, 0, st, jobs);
+    launch_after(k_post<NJ>, g, kPoThreads, 0, st, jobs);
     count_launch();
     if (prof_enabled()) {
         double by = 0;
