@@ -21,12 +21,36 @@ __device__ __forceinline__ int reflect101(int i, int n)
     return i < 0 ? 0 : i;
 }
 
-// One block: 128 x 16 output pixels, a thread per 4 adjacent outputs of a
-// row.  The source tile (rows 2*y0 - 2 .. 2*y0 + 32, columns 2*x0 - 4 ..
-// 2*x0 + 259, word aligned) is staged as words when it lies inside the
-// image and the rows are word aligned, else byte by byte with reflected
-// indices.  Each thread sums the five taps of its 11 source columns
-// vertically, then the five horizontal taps of each output.
+// Bytes c .. c + 3 of an image row as a word: one load where the row is word
+// aligned there, two otherwise, single bytes at the indices that `map` gives
+// where the four leave [0, w) or the words the image [first, end).
+template <typename Map>
+__device__ __forceinline__ uint32_t load4(const uint8_t* row, int c, int w, const uint8_t* first, const uint8_t* end,
+                                          Map map)
+{
+    if (c >= 0 && c + 4 <= w) {
+        const unsigned s = (unsigned)(reinterpret_cast<uintptr_t>(row + c) & 3u);
+        const uint8_t* a = row + c - s;
+        if (s == 0) return __ldg(reinterpret_cast<const uint32_t*>(a));
+        if (a >= first && a + 8 <= end) {
+            const uint32_t* q = reinterpret_cast<const uint32_t*>(a);
+            return __funnelshift_r(__ldg(q), __ldg(q + 1), 8 * s);
+        }
+    }
+    uint32_t v = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v |= (uint32_t)__ldg(row + map(c + j)) << (8 * j);
+    return v;
+}
+
+// One block: 128 x 16 output pixels, a thread per 4 adjacent outputs of two
+// rows.  The source tile (rows 2*y0 - 2 .. 2*y0 + 32, columns 2*x0 - 4 ..
+// 2*x0 + 259) is staged as words, also at the border (80 of the 272 tiles of
+// 960x540 outputs lie there; staged byte by byte they took twice as long as
+// the others) and where rows are not word aligned.  Vertical sums are at
+// most 16 * 255 and the sums of both directions 256 * 255 + 128, so two
+// columns share a register throughout: even and odd source columns apart,
+// the taps of two outputs come out as one product each.
 constexpr int kPdX = 128, kPdY = 16;
 constexpr int kPdSWB = 2 * kPdX + 8;    // staged source bytes per row
 constexpr int kPdSWW = kPdSWB / 4;
@@ -40,52 +64,88 @@ __global__ void __launch_bounds__(256) k_pyrdown(const __grid_constant__ PyrDown
     const PyrDownDesc& P = b.d[blockIdx.z];
     const int x0 = blockIdx.x * kPdX, y0 = blockIdx.y * kPdY;
     if (x0 >= P.dw || y0 >= P.dh) return;
-    __shared__ uint32_t tw[kPdSH][kPdSWW];   // byte c of row r: source (reflect(2*y0 - 2 + r), reflect(2*x0 - 4 + c))
-    const int sx0 = 2 * x0 - 4, sy0 = 2 * y0 - 2;
-    const bool aligned = ((reinterpret_cast<uintptr_t>(P.src) | (uintptr_t)P.sstep) & 3u) == 0;
-    if (aligned && sx0 >= 0 && sx0 + kPdSWB <= P.sw && sy0 >= 0 && sy0 + kPdSH <= P.sh) {
-        for (int i = threadIdx.x; i < kPdSH * kPdSWW; i += 256) {
-            const int r = i / kPdSWW, k = i - r * kPdSWW;
-            tw[r][k] = __ldg(reinterpret_cast<const uint32_t*>(P.src + (size_t)(sy0 + r) * P.sstep + sx0) + k);
+    __shared__ __align__(8) uint32_t tw[kPdSH][kPdSWW];   // byte c of row r: source (reflect(2*y0 - 2 + r), reflect(2*x0 - 4 + c))
+    const int sx0 = 2 * x0 - 4, sy0 = 2 * y0 - 2, sw = P.sw, sh = P.sh;
+    const uint8_t* const first = P.src;
+    const uint8_t* const end = first + (size_t)(sh - 1) * P.sstep + sw;
+    const int tx = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // a warp per row
+    if (((reinterpret_cast<uintptr_t>(first) | (uintptr_t)P.sstep) & 3u) == 0) {
+        const bool in0 = sx0 + 4 * tx >= 0 && sx0 + 4 * tx + 4 <= sw, in1 = sx0 + 4 * tx + 132 <= sw,
+                   in2 = tx < kPdSWW - 64 && sx0 + 4 * tx + 260 <= sw;
+#pragma unroll
+        for (int r = warp; r < kPdSH; r += 8) {
+            const uint32_t* q =
+                reinterpret_cast<const uint32_t*>(first + (size_t)reflect101(sy0 + r, sh) * P.sstep + sx0) + tx;
+            if (in0) tw[r][tx] = __ldg(q);
+            if (in1) tw[r][tx + 32] = __ldg(q + 32);
+            if (in2) tw[r][tx + 64] = __ldg(q + 64);
+        }
+        // the words with columns outside that an output needs: the first one, and from `from` on
+        const int left = sx0 < 0 ? 1 : 0, from = imax((sw - sx0) >> 2, left);
+        const int last = (2 * imin(x0 + kPdX - 1, P.dw - 1) + 2 - sx0) >> 2;
+        const int edge = left + imax(0, imin(last + 1, kPdSWW) - from);
+        for (int i = threadIdx.x; i < kPdSH * edge; i += 256) {
+            const int r = i / edge, m = i - r * edge, k = m < left ? 0 : from + m - left;
+            const uint8_t* row = first + (size_t)reflect101(sy0 + r, sh) * P.sstep;
+            uint32_t v = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v |= (uint32_t)__ldg(row + reflect101(sx0 + 4 * k + j, sw)) << (8 * j);
+            tw[r][k] = v;
         }
     } else {
-        uint8_t* tb = reinterpret_cast<uint8_t*>(&tw[0][0]);
-        for (int i = threadIdx.x; i < kPdSH * kPdSWB; i += 256) {
-            const int r = i / kPdSWB, c = i - r * kPdSWB;
-            tb[i] = __ldg(P.src + (size_t)reflect101(sy0 + r, P.sh) * P.sstep + reflect101(sx0 + c, P.sw));
+        for (int r = warp; r < kPdSH; r += 8) {
+            const uint8_t* row = first + (size_t)reflect101(sy0 + r, sh) * P.sstep;
+#pragma unroll
+            for (int k = tx; k < kPdSWW; k += 32)
+                tw[r][k] = load4(row, sx0 + 4 * k, sw, first, end, [&](int c) { return reflect101(c, sw); });
         }
     }
     __syncthreads();
-    const int tx = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int xb = x0 + 4 * tx;
-    if (xb >= P.dw) return;
+    const int xb = x0 + 4 * tx, yb = y0 + 2 * warp;
+    if (xb >= P.dw || yb >= P.dh) return;
     const int np = imin(4, P.dw - xb);
-#pragma unroll 1
-    for (int ty = warp; ty < kPdY; ty += 8) {
-        const int y = y0 + ty;
-        if (y >= P.dh) break;
-        // vertical taps of source columns 2*xb - 2 .. 2*xb + 8 (tile bytes 8*tx + 2 .. 8*tx + 12)
-        int v[11];
+    // tile bytes 8 * tx + 2 .. 8 * tx + 12 are the source columns of the four
+    // outputs: even ones 0 | 2, 4 | 6, 8 | 10, 12 | 14, odd ones 1 | 3, ...
+    uint32_t ev[2][4], od[2][3];
 #pragma unroll
-        for (int k = 0; k < 11; ++k) v[k] = 0;
-        const int w5[5] = {1, 4, 6, 4, 1};
+    for (int o = 0; o < 2; ++o) {
 #pragma unroll
-        for (int ky = 0; ky < 5; ++ky) {
-            const uint32_t* row = tw[2 * ty + ky] + 2 * tx;
-            const uint32_t q0 = row[0], q1 = row[1], q2 = row[2], q3 = row[3];
+        for (int k = 0; k < 4; ++k) ev[o][k] = 0;
 #pragma unroll
-            for (int k = 0; k < 11; ++k) {
-                const int bi = k + 2;
-                const uint32_t q = bi < 4 ? q0 : bi < 8 ? q1 : bi < 12 ? q2 : q3;
-                v[k] += w5[ky] * (int)((q >> (8 * (bi & 3))) & 0xffu);
+        for (int k = 0; k < 3; ++k) od[o][k] = 0;
+    }
+#pragma unroll
+    for (int r = 0; r < 7; ++r) {
+        const uint2* row = reinterpret_cast<const uint2*>(tw[4 * warp + r]) + tx;
+        const uint2 a = row[0], z = row[1];
+        const uint32_t q[4] = {a.x, a.y, z.x, z.y};
+        constexpr uint32_t w5[5] = {1, 4, 6, 4, 1};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t e = __byte_perm(q[k], 0, 0x4240), u = __byte_perm(q[k], 0, 0x4341);
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                const int ky = r - 2 * o;
+                if (ky < 0 || ky > 4) continue;
+                ev[o][k] += w5[ky] * e;
+                if (k < 3) od[o][k] += w5[ky] * u;
             }
         }
-        uint32_t out = 0;
+    }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int sum = v[2 * j] + 4 * v[2 * j + 1] + 6 * v[2 * j + 2] + 4 * v[2 * j + 3] + v[2 * j + 4];
-            out |= (uint32_t)((sum + 128) >> 8) << (8 * j);
-        }
+    for (int o = 0; o < 2; ++o) {
+        const int y = yb + o;
+        if (y >= P.dh) break;
+        const uint32_t(&e)[4] = ev[o];
+        const uint32_t(&u)[3] = od[o];
+        // outputs 0 | 1 (centres 4 | 6) and 2 | 3 (centres 8 | 10)
+        const uint32_t e01 = __funnelshift_r(e[0], e[1], 16), e12 = __funnelshift_r(e[1], e[2], 16),
+                       e23 = __funnelshift_r(e[2], e[3], 16);
+        const uint32_t u01 = __funnelshift_r(u[0], u[1], 16), u12 = __funnelshift_r(u[1], u[2], 16);
+        const uint32_t s0 = e01 + e12 + 6 * e[1] + 4 * (u01 + u[1]) + 0x00800080u;
+        const uint32_t s1 = e12 + e23 + 6 * e[2] + 4 * (u12 + u[2]) + 0x00800080u;
+        const uint32_t out = __byte_perm(s0, s1, 0x7531);
         uint8_t* dst = P.dst + (size_t)y * P.dstep + xb;
         if (np == 4 && (reinterpret_cast<uintptr_t>(dst) & 3u) == 0) {
             *reinterpret_cast<uint32_t*>(dst) = out;
@@ -116,8 +176,7 @@ __global__ void __launch_bounds__(256) k_pyrdown(const __grid_constant__ PyrDown
 //
 // One block: 128 x 8 pixels of one view, a warp per row.  The image tile
 // with its 2-pixel border (4 columns on each side, so rows stay word
-// aligned) is staged as words when it lies inside the image and the rows are
-// word aligned, else byte by byte with replicated borders.  Census: a thread
+// aligned) is staged as words, bytes only where columns are replicated.  Census: a thread
 // per 4 adjacent pixels, 16-byte stores.  BT: gradients of 4 adjacent pixels
 // per thread on 16-bit pairs, laid down with the intensities as one word per
 // pixel; then a thread per pixel, 32 apart, makes the intervals of both
@@ -185,18 +244,12 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
             pcf[2 * j] = pcf[2 * j + 1] = __ldg(crow + px);
         }
     }
-    const bool aligned = ((reinterpret_cast<uintptr_t>(img) | (uintptr_t)step) & 3u) == 0;
-    if (aligned && x0 >= 4 && x0 + kFtX + 4 <= W && y0 >= 2 && y0 + kFtY + 2 <= H) {
-        for (int i = threadIdx.x; i < kFtSH * kFtSWW; i += 256) {
-            const int r = i / kFtSWW, k = i - r * kFtSWW;
-            tw[r][k] = __ldg(reinterpret_cast<const uint32_t*>(img + (size_t)(y0 - 2 + r) * step + x0 - 4) + k);
-        }
-    } else {
-        uint8_t* tb = reinterpret_cast<uint8_t*>(&tw[0][0]);
-        for (int i = threadIdx.x; i < kFtSH * kFtSWB; i += 256) {
-            const int r = i / kFtSWB, c = i - r * kFtSWB;
-            tb[i] = __ldg(img + (size_t)iclamp(y0 - 2 + r, 0, H - 1) * step + iclamp(x0 - 4 + c, 0, W - 1));
-        }
+    const uint8_t* const end = img + (size_t)(H - 1) * step + W;
+#pragma unroll
+    for (int i = threadIdx.x; i < kFtSH * kFtSWW; i += 256) {
+        const int r = i / kFtSWW, k = i - r * kFtSWW;
+        tw[r][k] = load4(img + (size_t)iclamp(y0 - 2 + r, 0, H - 1) * step, x0 - 4 + 4 * k, W, img, end,
+                         [&](int c) { return iclamp(c, 0, W - 1); });
     }
     __syncthreads();
     if (y >= H) return;
