@@ -834,15 +834,21 @@ __device__ __forceinline__ void bt_row_sums(const LevelDesc& J, uint32_t* hs, ui
     uint4* sr = st + kTiRows * kTiSL;    // [R][kTiSR]  right, columns xrs + p
     const int xrs = x0 - HW - (rmin + 4 * nq - 1);
     const int nsr = SW + 4 * nq - 1;
+    // a warp per row; the columns (and which are outside) are those of every row
+    const int gl0 = iclamp(x0 - HW + lane, 0, W - 1), gl1 = imin(x0 - HW + 32 + lane, W - 1);
+    const int xr0 = xrs + lane, xr1 = xr0 + 32;
+    const bool in0 = xr0 >= 0 && xr0 < W, in1 = xr1 >= 0 && xr1 < W, more = lane + 32 < nsr;
     for (int r = a.r0 + warp; r < a.r0 + a.nr; r += kTiWarps) {
         const size_t grow = (size_t)iclamp(y0 - HW + r, 0, H - 1) * W;
-        for (int j = lane; j < SW; j += 32)
-            tile_cp16(sl + r * kTiSL + j, J.featL + grow + iclamp(x0 - HW + j, 0, W - 1));
+        const uint4 *fl = J.featL + grow, *fr = J.featR + grow;
         uint4* o = sr + r * kTiSR + (lane & 3) * kTiSub + (lane >> 2);
-        for (int p = lane; p < nsr; p += 32, o += 8) {
-            const int xx = xrs + p;
-            if (xx >= 0 && xx < W) tile_cp16(o, J.featR + grow + xx);
-            else *o = bt_outside();
+        tile_cp16(sl + r * kTiSL + lane, fl + gl0);
+        if (lane < SW - 32) tile_cp16(sl + r * kTiSL + 32 + lane, fl + gl1);
+        if (in0) tile_cp16(o, fr + xr0);
+        else *o = bt_outside();
+        if (more) {
+            if (in1) tile_cp16(o + 8, fr + xr1);
+            else o[8] = bt_outside();
         }
     }
     tile_commit_wait();
@@ -942,18 +948,12 @@ __global__ void __launch_bounds__(256, 3) k_cost_bt_tiled(const __grid_constant_
         __syncthreads();   // wred reused
         if (lane == 0) { wred[0][warp] = a; wred[1][warp] = z; wred[2][warp] = (int)m; }
         __syncthreads();
-        mn = INT_MAX;
-        mx = INT_MIN;
-        unsigned cols = 0;
-        int first = kTiWarps, last = 0;
-#pragma unroll
-        for (int i = 0; i < kTiWarps; ++i) {
-            mn = imin(mn, wred[0][i]);
-            mx = imax(mx, wred[1][i]);
-            const unsigned c = (unsigned)wred[2][i];
-            cols |= c;
-            if (c) { first = imin(first, i); last = i; }
-        }
+        const int l8 = lane & (kTiWarps - 1);
+        mn = __reduce_min_sync(0xffffffffu, wred[0][l8]);
+        mx = __reduce_max_sync(0xffffffffu, wred[1][l8]);
+        const unsigned c = (unsigned)wred[2][l8], cols = __reduce_or_sync(0xffffffffu, c);
+        const unsigned rows = __ballot_sync(0xffffffffu, c != 0) & ((1u << kTiWarps) - 1);
+        const int first = __ffs((int)rows) - 1, last = 31 - __clz((int)rows);
         area.r0 = 2 * first;
         area.nr = 2 * (last - first + 1) + 2 * h;
         area.seg0 = (cols & 0xffffu) ? 0 : 1;
@@ -1028,16 +1028,21 @@ __global__ void __launch_bounds__(256, 3) k_cost_bt_tiled(const __grid_constant_
                 label_range(J, x, bq[0], lo, hi);
                 const int o = bq[0] - low;
                 uint32_t above[10], below[10];
-                rowsum(2 * warp, o, above);
-                rowsum(2 * warp + 2 * h + 1, o, below);
+#pragma unroll
+                for (int j = 0; j < 10; ++j) below[j] = 0;
                 for (int k = 1; k <= 2 * h; ++k) {   // the rows both windows hold
                     uint32_t v[10];
                     rowsum(2 * warp + k, o, v);
 #pragma unroll
-                    for (int j = 0; j < 10; ++j) {
-                        above[j] += v[j];
-                        below[j] += v[j];
-                    }
+                    for (int j = 0; j < 10; ++j) below[j] += v[j];
+                }
+                uint32_t v[10];
+                rowsum(2 * warp, o, above);
+                rowsum(2 * warp + 2 * h + 1, o, v);
+#pragma unroll
+                for (int j = 0; j < 10; ++j) {
+                    above[j] += below[j];
+                    below[j] += v[j];
                 }
                 put(0, above, o & 3, lo, hi);
                 put(1, below, o & 3, lo, hi);
