@@ -83,23 +83,32 @@ __global__ void __launch_bounds__(256) k_wta_sum(const __grid_constant__ Jobs<NJ
             t[8 * r] = a.x; t[8 * r + 1] = a.y; t[8 * r + 2] = a.z; t[8 * r + 3] = a.w;
             t[8 * r + 4] = b.x; t[8 * r + 5] = b.y; t[8 * r + 6] = b.z; t[8 * r + 7] = b.w;
         }
+        // cost in the high half, label in the low one (the shift as a product: the other pipe)
         unsigned best = 0xffffffffu;
 #pragma unroll
         for (int j = 0; j < 8 * R; ++j) {
             const unsigned d = 16u * (gl + G * (j / 8)) + 2 * (j % 8);
-            best = __vimin3_u32(best, (t[j] << 16) | d, (t[j] & 0xffff0000u) | (d + 1));
+            best = __vimin3_u32(best, t[j] * 65536u + d, (t[j] & 0xffff0000u) | (d + 1));
         }
 #pragma unroll
         for (int o = 1; o < G; o <<= 1) best = umin(best, __shfl_xor_sync(0xffffffffu, best, o));
         const int bd = (int)(best & 0xffffu);
-        unsigned far = kMax;
+        // minimum over the labels further than one from the best, two at a
+        // time: d - bd + 1 is 0, 1 or 2 at the others, which become SHRT_MAX
+        // (from 3 on the addition sets the sign)
+        uint32_t far2 = pk::kMax2;
 #pragma unroll
-        for (int j = 0; j < 8 * R; ++j) {
-            const int d = 16 * (gl + G * (j / 8)) + 2 * (j % 8);
-            const unsigned u0 = (unsigned)(d - bd + 1) <= 2u ? (unsigned)kMax : (t[j] & 0xffffu);
-            const unsigned u1 = (unsigned)(d - bd + 2) <= 2u ? (unsigned)kMax : (t[j] >> 16);
-            far = __vimin3_u32(far, u0, u1);
+        for (int r = 0; r < R; ++r) {
+            const uint32_t first = pk::dup(16 * (gl + G * r) + 1 - bd) + 0x00010000u;   // of labels 0 and 1
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t far3 = __viaddmin_u16x2(first, 0x00020002u * j, 0x00030003u) + 0x7ffd7ffdu;
+                t[8 * r + j] |= ~pk::sign_mask2(far3) & pk::kMax2;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) far2 = __vimin3_u16x2(far2, t[8 * r + j], t[8 * r + j + 1]);
         }
+        unsigned far = umin(far2 & 0xffffu, far2 >> 16);
 #pragma unroll
         for (int o = 1; o < G; o <<= 1) far = umin(far, __shfl_xor_sync(0xffffffffu, far, o));
         if (gl == i) {
