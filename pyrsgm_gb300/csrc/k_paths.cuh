@@ -27,17 +27,20 @@
 #include "sgm_launch.h"
 #include "k_paths_packed.cuh"
 #include "k_paths_seg.cuh"
+#include "k_wta_group.cuh"
 #include "k_fused.cuh"
 
 namespace pg {
 
-// Winner-take-all of the packed levels.
+// Winner-take-all of the packed levels: a thread per pixel with 16 and 32
+// labels, four lanes with 64.
 template <int D, bool PYR, int NJ>
 cudaError_t launch_wta(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
 {
     dim3 gw((e.max_w + 31) / 32, (e.max_h + 7) / 8, jobs.n);
     prof_begin(st);
-    launch_after(k_wta<D, PYR, NJ>, gw, 256, 0, st, jobs);
+    if constexpr (D <= 32) launch_after(k_wta<D, PYR, NJ>, gw, 256, 0, st, jobs);
+    else launch_after(k_wta_group<D / 16, 1, 3, PYR, NJ>, gw, 256, 0, st, jobs);
     count_launch();
     prof_end(PK_WTA, jobs_vox(jobs) * 2 * (jobs.d[0].paths >= 3 ? 3 : jobs.d[0].paths) + jobs_px(jobs) * (2 + 6 + 4), st);
     return launched(st, "k_wta");

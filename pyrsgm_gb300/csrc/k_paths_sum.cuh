@@ -6,6 +6,7 @@
 #pragma once
 
 #include "k_paths_seg.cuh"
+#include "k_wta_group.cuh"
 
 namespace pg {
 
@@ -45,90 +46,6 @@ __global__ void __launch_bounds__(32) k_rowadd(const __grid_constant__ Jobs<NJ> 
     for (int i = 0; i < NW; ++i) s.L[i] = spec[i] = kMax2;
     s.mp2 = kMax2;
     seg_walk<NW, T, MODE, kAdd>(X, s, 0, 0, n > 0 ? n : -(1 << 30), nch, 1, 0, 0, true, spec);
-}
-
-// Winner-take-all over the sums in V.  G lanes read a pixel's labels, 16 R
-// each, and reduce; after G pixels every lane has one winner of its own, and
-// the rules and outputs run on full warps.
-template <int G, int R, bool PYR, int NJ>
-__global__ void __launch_bounds__(256) k_wta_sum(const __grid_constant__ Jobs<NJ> jobs)
-{
-    if (NJ == 1) let_next_in();   // (in a batch the next label count's chains may follow)
-    after_previous();
-    const LevelDesc& J = jobs.d[blockIdx.z];
-    const int W = J.w, D = J.D, lane = threadIdx.x & 31, gl = lane % G;
-    const int y = blockIdx.y * 8 + (threadIdx.x >> 5), x0 = blockIdx.x * 32;
-    if (x0 >= W || y >= J.h) return;
-    int xlo = 0, xhi = W;
-    if (!PYR) {
-        xlo = imax(J.minD + D, 0);
-        xhi = imin(W + imin(J.minD, 0), W - 1);   // the last column has no winner
-    }
-    const int16_t* row = J.V + (size_t)y * W * D;
-    unsigned myBest = 0;
-    int myAlt = 0;
-#pragma unroll 2
-    for (int i = 0; i < G; ++i) {
-        const int x = imin(x0 + lane - gl + i, W - 1);
-        uint32_t t[8 * R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int d0 = 16 * (gl + G * r);
-            uint4 a = make_uint4(pk::kMax2, pk::kMax2, pk::kMax2, pk::kMax2), b = a;
-            if (d0 < D) {
-                const uint4* p = reinterpret_cast<const uint4*>(row + (size_t)x * D + d0);
-                a = __ldg(p);
-                b = __ldg(p + 1);
-            }
-            t[8 * r] = a.x; t[8 * r + 1] = a.y; t[8 * r + 2] = a.z; t[8 * r + 3] = a.w;
-            t[8 * r + 4] = b.x; t[8 * r + 5] = b.y; t[8 * r + 6] = b.z; t[8 * r + 7] = b.w;
-        }
-        // cost in the high half, label in the low one (the shift as a product: the other pipe)
-        unsigned best = 0xffffffffu;
-#pragma unroll
-        for (int j = 0; j < 8 * R; ++j) {
-            const unsigned d = 16u * (gl + G * (j / 8)) + 2 * (j % 8);
-            best = __vimin3_u32(best, t[j] * 65536u + d, (t[j] & 0xffff0000u) | (d + 1));
-        }
-#pragma unroll
-        for (int o = 1; o < G; o <<= 1) best = umin(best, __shfl_xor_sync(0xffffffffu, best, o));
-        const int bd = (int)(best & 0xffffu);
-        // minimum over the labels further than one from the best, two at a
-        // time: d - bd + 1 is 0, 1 or 2 at the others, which become SHRT_MAX
-        // (from 3 on the addition sets the sign)
-        uint32_t far2 = pk::kMax2;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const uint32_t first = pk::dup(16 * (gl + G * r) + 1 - bd) + 0x00010000u;   // of labels 0 and 1
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t far3 = __viaddmin_u16x2(first, 0x00020002u * j, 0x00030003u) + 0x7ffd7ffdu;
-                t[8 * r + j] |= ~pk::sign_mask2(far3) & pk::kMax2;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; j += 2) far2 = __vimin3_u16x2(far2, t[8 * r + j], t[8 * r + j + 1]);
-        }
-        unsigned far = umin(far2 & 0xffffu, far2 >> 16);
-#pragma unroll
-        for (int o = 1; o < G; o <<= 1) far = umin(far, __shfl_xor_sync(0xffffffffu, far, o));
-        if (gl == i) {
-            myBest = best;
-            myAlt = (int)far;
-        }
-    }
-    const int x = x0 + lane;
-    if (x >= W) return;
-    const size_t p = (size_t)y * W + x;
-    if (x < xlo || x >= xhi) {
-        J.disp_raw[p] = (int16_t)((J.minD - 1) * 16);
-        J.conf_raw[p] = 0.0f;
-        return;
-    }
-    const int minCost = (int)(myBest >> 16), bd = (int)(myBest & 0xffffu);
-    const int c0 = bd > 0 ? (int)__ldg(row + (size_t)x * D + bd - 1) : 0;
-    const int c2 = bd + 1 < D ? (int)__ldg(row + (size_t)x * D + bd + 1) : 0;
-    const int base = (PYR && J.refine) ? (int)J.base[p] : J.minD;
-    pk::wta_out<PYR>(J, D, y, x, base, minCost, bd, myAlt, c0, minCost, c2);
 }
 
 template <int NW, int T, int MODE, int NJ>
@@ -183,10 +100,10 @@ cudaError_t launch_sum(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t 
     if (err != cudaSuccess) return err;
     dim3 gw((e.max_w + 31) / 32, (e.max_h + 7) / 8, jobs.n);
     prof_begin(st);
-    launch_after(k_wta_sum<G, R, PYR, NJ>, gw, 256, 0, st, jobs);
+    launch_after(k_wta_group<G, R, 1, PYR, NJ>, gw, 256, 0, st, jobs);
     count_launch();
     prof_end(PK_WTA, jobs_vox(jobs) * 2 + jobs_px(jobs) * (2 + 6 + 4), st);
-    return launched(st, "k_wta_sum");
+    return launched(st, "k_wta_group");
 }
 
 template <bool PYR, int NJ>
