@@ -204,7 +204,7 @@ struct State {
     uint32_t mp2;   // minimum over the chain's labels, in both halves
 };
 
-template <int NW, int T>
+template <int NW, int T, bool LONE = false>
 __device__ __forceinline__ uint32_t chain_min_dup(const uint32_t (&L)[NW])
 {
     uint32_t m = L[0];
@@ -216,6 +216,21 @@ __device__ __forceinline__ uint32_t chain_min_dup(const uint32_t (&L)[NW])
         m = __vminu2(m, L[NW - 1]);
     }
     m = __vminu2(m, __funnelshift_l(m, m, 16));
+    // Across lanes: a shuffle a level of the tree or a warp reduction a chain.
+    // Two reductions are shorter than four dependent shuffles (641x479 with 96
+    // labels 209 us a call, 182); four against three only where a lone warp
+    // waits for each step (LONE; 720p with 48 labels 311, 285; the segments
+    // of 64 labels 217, 222).
+    if constexpr (T == 16 || (LONE && T == 8)) {
+        const unsigned g = (threadIdx.x & 31) / T;
+        uint32_t r = m;
+#pragma unroll
+        for (unsigned i = 0; i < 32 / T; ++i) {
+            const uint32_t a = __reduce_min_sync(0xffffffffu, g == i ? m : 0xffffffffu);
+            if (g == i) r = a;
+        }
+        return r;
+    }
 #pragma unroll
     for (int o = 1; o < T; o <<= 1) m = __vminu2(m, __shfl_xor_sync(0xffffffffu, m, o));
     return m;
@@ -239,7 +254,7 @@ __device__ __forceinline__ uint32_t window_at(int delta)
 //   min(c + best - minPrev, min(c + P2, MAX)),
 // so that only the neighbours' minimum and minPrev are on it.  `guard`: an
 // active chain's best may reach SHRT_MAX (see k_seg), which then stays.
-template <int NW, int T, int MODE>
+template <int NW, int T, int MODE, bool LONE>
 __device__ __forceinline__ void seg_step(State<NW, T>& s, const uint32_t (&c)[NW], uint32_t at, uint32_t p22,
                                          uint32_t p12, uint32_t* win, int k, bool guard)
 {
@@ -284,7 +299,7 @@ __device__ __forceinline__ void seg_step(State<NW, T>& s, const uint32_t (&c)[NW
 #pragma unroll
         for (int m = 0; m < NW; ++m) s.L[m] |= pk::sign_mask2(__vminu2(best[m], lj2) + kOne2) & kMax2;
     }
-    s.mp2 = chain_min_dup<NW, T>(s.L);
+    s.mp2 = chain_min_dup<NW, T, LONE>(s.L);
 }
 
 // The block's adaptive-P2 table; returns whether an active chain's best may
@@ -520,7 +535,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
 #pragma unroll
                 for (int i = 0; i < NW; ++i) cc[i] |= mask[i];
             }
-            seg_step<NW, T, MODE>(s, cc, at, p22, X.p12, X.win + (q & 1) * G::BUFW, k, X.guard);
+            seg_step<NW, T, MODE, ADD>(s, cc, at, p22, X.p12, X.win + (q & 1) * G::BUFW, k, X.guard);
             bool put = (unsigned)(t + q - ts) < span;
             if constexpr (FIX) put = put && act;
             uint32_t res[NW];
