@@ -520,10 +520,26 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
         }
         const uint32_t* cin = X.ring + slot * G::SLOTW + X.c * G::CSTR + k * NW;
         slot = slot + 1 == kSC ? 0 : slot + 1;
+        // ADD: a lone warp waits for every load, so a chunk's costs and sums
+        // are read ahead of its steps (641x479 with 96 labels 182 us a call, 179)
+        constexpr bool kEarly = ADD && NW <= 8;
+        uint32_t ce[kEarly ? kCH : 1][NW], ve[kEarly ? kCH : 1][NW];
+        if constexpr (kEarly) {
+#pragma unroll
+            for (int q = 0; q < kCH; ++q) {
+                pk::ldw<NW>(cin + q * (D / 2), ce[q]);
+                pk::ldw<NW>(cin + kSC * G::SLOTW + q * (D / 2), ve[q]);
+            }
+        }
 #pragma unroll
         for (int q = 0; q < kCH; ++q) {
             uint32_t cc[NW];
-            pk::ldw<NW>(cin + q * (D / 2), cc);
+            if constexpr (kEarly) {
+#pragma unroll
+                for (int i = 0; i < NW; ++i) cc[i] = ce[q][i];
+            } else {
+                pk::ldw<NW>(cin + q * (D / 2), cc);
+            }
             uint32_t at = 0, p22 = p2const;
             if (need) {
                 at = T == 1 ? info[q < G::QL ? q : 0]
@@ -545,7 +561,12 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
                 const int both = rl_n - 1 - 2 * (t + q);   // steps until the other direction gets here
                 uint32_t v[NW];
                 bool sum = paths >= 3 || (paths == 2 && both < 0);
-                pk::ldw<NW>(cin + kSC * G::SLOTW + q * (D / 2), v);
+                if constexpr (kEarly) {
+#pragma unroll
+                    for (int i = 0; i < NW; ++i) v[i] = ve[q][i];
+                } else {
+                    pk::ldw<NW>(cin + kSC * G::SLOTW + q * (D / 2), v);
+                }
                 if (paths >= 2 && both <= 0 && both > -2 * kCH * kSC) {
                     if (both == 0) {   // the same pixel: L->R first
                         if (put && !(X.c & 1)) {
