@@ -55,13 +55,14 @@ def params_for(cost: int) -> dict:
 
 
 # Measured DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per
-# byte the aggregation kernels move by their own design, from the full
-# captures of the 1080p-level launches of eight pairs
-# (profiles/stage_kernels_1080p_8pairs.md): k_gtb 1066.8, k_grow 2147.6,
-# k_wta 1834.9 and k_gtbw 1854.7 MB against 1111.5, 2222.9, 1791.6 and
-# 1808.2 MB of their own bytes.  Every kernel streams its volumes once per
-# launch, so the ratio carries over to a step by each kind's own bytes.
-AGG_TRAFFIC_PER_OWN_BYTE = {"path_tb": 1066.8 / 1111.5, "path_row": 2147.6 / 2222.9, "wta": 1834.9 / 1791.6,
+# byte the aggregation kernels move by their own design, from captures of
+# the 1080p-level launches of eight pairs: k_seg 2993.0 and k_wta 1828.7 MB
+# against 3334.3 and 1791.6 MB of their own bytes
+# (profiles/segmented_chains_1080p_8pairs.md), and of the wide shape k_gtb
+# 1066.8 and k_gtbw 1854.7 against 1111.5 and 1808.2
+# (profiles/stage_kernels_1080p_8pairs.md).  The ratio carries over to a
+# step by each kind's own bytes.
+AGG_TRAFFIC_PER_OWN_BYTE = {"path_tb": 1066.8 / 1111.5, "path_row": 2993.0 / 3334.3, "wta": 1828.7 / 1791.6,
                             "tbw": 1854.7 / 1808.2}
 
 
@@ -668,7 +669,7 @@ def job_rate(world: int, units_per_rank: float, max_ms: float) -> float:
 
 # profiled stages of the aggregation and the kernels behind them
 AGG_STAGES = ("path_tb", "path_row", "wta", "tblr", "rlw", "tbw")
-AGG_KERNELS = {"path_tb": "k_gtb/k_path_tb", "path_row": "k_grow/k_path_row", "wta": "k_wta",
+AGG_KERNELS = {"path_tb": "k_gtb", "path_row": "k_seg/k_rowadd/k_grow", "wta": "k_wta/k_wta_group",
                "tblr": "k_tblr", "rlw": "k_rlw", "tbw": "k_gtbw"}
 PROF_NAMES = ["pyrdown", "features", "labels", "cost", "path_tb", "path_row", "post", "p2table", "wta", "tblr",
               "rlw", "tbw"]

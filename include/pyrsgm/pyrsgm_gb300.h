@@ -236,9 +236,9 @@ int pyrsgm_gb300_filter_speckles(short* d_disp, size_t pitch_bytes, int width, i
                                  int max_speckle_size, int max_diff, cudaStream_t stream);
 
 /* Shape of the 16/32/64-label aggregation kernels: 0 chooses per launch
- * (one thread per 16 labels when the launch has rows enough to fill the
- * GPU, else a chain spread over more threads), 8 forces the former, 2 or 4
- * the latter.  Results are identical either way.  Returns the previous
+ * (chains cut into segments that run at the same time), 8 forces the wide
+ * shape (one thread per 16 labels, whole chains), 2 or 4 the segmented one.
+ * Results are identical either way.  Returns the previous
  * setting, or -1 for another value.  The environment variable
  * PYRSGM_GB300_PACKED_NW gives the initial setting. */
 int pyrsgm_gb300_set_packed_words(int words);

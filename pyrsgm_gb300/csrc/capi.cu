@@ -3,9 +3,9 @@
 //
 // Argument checks, parameter sanitising, clamps and error convention follow
 // the reference host code (src/sgm_kernels.cu:1607-2076, src/pyrdown.cu:56-74).
-// The kernel sequence differs: features -> (refine labels) -> cost ->
-// (T->B) -> row pass (L->R + R->L + WTA + disp2 + LR check) -> median and
-// outputs, 4-6 launches per level instead of ~17.
+// The kernel sequence differs: features and refine labels -> cost -> the
+// chains of all paths -> (row sums) -> winner and disp2 -> LR check, median
+// and outputs, 5 or 6 launches per level instead of ~17.
 #include <algorithm>
 #include <atomic>
 #include <climits>

@@ -1,9 +1,11 @@
-// k_paths_packed.cuh -- path aggregation for D = 16, 32 and 64 labels: the
-// labels of one path chain are packed two per 32-bit word and held by T
-// threads, eight words (16 labels) each.  This is the shape for launches
-// with many rows: it spends the fewest instructions per pixel and fills the
-// GPU with whole chains.  Launches with few rows cut their chains into
-// segments (k_paths_seg.cuh).
+// k_paths_packed.cuh -- path aggregation for D = 16, 32 and 64 labels in the
+// wide shape: the labels of one path chain are packed two per 32-bit word and
+// held by T threads, eight words (16 labels) each, a chain is walked whole.
+// It spends the fewest instructions per pixel, but even 32 pairs of 1080p
+// leave the SMs with few warps, so the segmented shape (k_paths_seg.cuh) is
+// the default at every size (packed_nw); this one runs when a caller or the
+// autotuner asks for it.  The packed arithmetic, the winner rules and k_wta
+// serve both.
 //
 // The recurrence of a step (reference: src/sgm_kernels.cu:560-565
 // single-scale, 1230-1252 pyramid) runs on 16-bit pairs with the DPX

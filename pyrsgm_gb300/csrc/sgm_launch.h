@@ -112,7 +112,7 @@ struct TuneKey {
 struct TuneEntry {
     int nw;              // chosen words per thread
     float ms_wide;       // NW = 8 shape, best of two
-    float ms_spread;     // spread shape (NW = 2, or 4 for 64 labels), best of two
+    float ms_spread;     // segmented shape, best of two
 };
 bool autotune_enabled();
 bool tuning_thread();
