@@ -790,8 +790,12 @@ __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_const
 // Window sums are exact integers (at most 25 * 255 here, no intermediate
 // clamp in the reference).  What is left after kTiClusters passes and wider
 // windows evaluate each window directly.
-// Bound by instruction issue (seven instructions a cost; 52 % of the slots
-// with two disparities a lane, which kept the shared-memory pipe at 64 %).
+// Bound by the integer pipe (seven instructions a cost; 62 %) and the
+// barriers between the phases, three blocks per SM.  The base level of a
+// 1080p pair: 158 us with direct sums for wide tiles, 98 with clusters, 94
+// with four disparities a lane instead of two (which kept the shared-memory
+// pipe at 64 %), 87 with the reductions, the staging and the shared rows as
+// they are now.
 // ---------------------------------------------------------------------------
 constexpr int kTiX = 32, kTiY = 16, kTiMaxHalf = 2;
 constexpr int kTiD = 16;         // labels of a pass
