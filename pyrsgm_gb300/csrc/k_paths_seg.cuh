@@ -230,10 +230,11 @@ __device__ __forceinline__ uint32_t chain_min_dup(const uint32_t (&L)[NW])
             if (g == i) r = a;
         }
         return r;
-    }
+    } else {
 #pragma unroll
-    for (int o = 1; o < T; o <<= 1) m = __vminu2(m, __shfl_xor_sync(0xffffffffu, m, o));
-    return m;
+        for (int o = 1; o < T; o <<= 1) m = __vminu2(m, __shfl_xor_sync(0xffffffffu, m, o));
+        return m;
+    }
 }
 
 // Window position of a label shift: byte offset of the word holding label

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(256) k_sp_tile(const SpArgs A)
         if (y >= A.h) break;
         const int p = y * A.w + x, r = root[k];
         A.size[p] = r == i ? cnt[i] : 0;
-        A.lab[p] = r < 0 ? -1 : (blockIdx.y * kSpTile + r / kSpTile) * A.w + blockIdx.x * kSpTile + r % kSpTile;
+        A.lab[p] = r < 0 ? -1 : ((int)blockIdx.y * kSpTile + r / kSpTile) * A.w + (int)blockIdx.x * kSpTile + r % kSpTile;
     }
 }
 
