@@ -48,8 +48,7 @@ using pk::kOne2;
 // Level semantics of a walk.
 enum { kSingle = 0, kCoarse = 1, kRefine = 2 };
 // What a walk does with the path costs: store them; store them until they
-// equal the stored ones; add them to the sum in V (rows of both directions
-// in step).
+// equal the stored ones; add them to the sum in V.
 enum { kStore = 0, kAgain = 1, kAdd = 2 };
 
 constexpr int kCH = 4;       // steps per chunk
@@ -92,7 +91,7 @@ __host__ __device__ constexpr int warp_words(int rings = 1)
 template <int NW, int T, int MODE>
 constexpr size_t add_smem()
 {
-    return 4 * (256 + (size_t)warp_words<NW, T, MODE>(2));
+    return 4 * (256 + 2 * (size_t)warp_words<NW, T, MODE>(2));   // a warp a direction
 }
 template <int NW, int T, int MODE>
 constexpr size_t seg_smem(int segs)
@@ -130,7 +129,7 @@ template <int NW>
 __device__ __forceinline__ void store_words(int16_t* p, int d0, int Dr, const uint32_t (&v)[NW])
 {
     if constexpr (NW == 2) {
-        *reinterpret_cast<uint2*>(p) = make_uint2(v[0], v[1]);
+        if (d0 < Dr) *reinterpret_cast<uint2*>(p) = make_uint2(v[0], v[1]);
     } else {
 #pragma unroll
         for (int i = 0; i < NW / 4; ++i) {
@@ -218,10 +217,10 @@ __device__ __forceinline__ uint32_t chain_min_dup(const uint32_t (&L)[NW])
     m = __vminu2(m, __funnelshift_l(m, m, 16));
     // Across lanes: a shuffle a level of the tree or a warp reduction a chain.
     // Two reductions are shorter than four dependent shuffles (641x479 with 96
-    // labels 209 us a call, 182); four against three only where a lone warp
-    // waits for each step (LONE; 720p with 48 labels 311, 285; the segments
-    // of 64 labels 217, 222).
-    if constexpr (T == 16 || (LONE && T == 8)) {
+    // labels 209 us a call, 182), as is one than five; four against three only
+    // where a lone warp waits for each step (LONE; 720p with 48 labels 311,
+    // 285; the segments of 64 labels 217, 222).
+    if constexpr (T >= 16 || (LONE && T == 8)) {
         const unsigned g = (threadIdx.x & 31) / T;
         uint32_t r = m;
 #pragma unroll
@@ -345,6 +344,8 @@ struct Ctx {
     Walk w;              // this lane's chain
     int16_t* out;        // its path-cost volume
     uint32_t p12;
+    int stop = 0;        // kAdd: the walk's end
+    bool sums = false;   // kAdd: V holds other paths' costs, which are added to
 };
 
 // Walk the steps [t0, t0 + 4 * nch) of the warp's chains that lie below each
@@ -352,7 +353,9 @@ struct Ctx {
 // chains a lane copies for).  Steps before ts are not stored.  FIX: only the
 // chains with `act` set are walked, the state of step t0 - 1 is in `s`, a
 // chain stops at the first step whose costs equal the stored ones; returns
-// whether it reached te without one.
+// whether it reached te without one.  ADD: chains of one direction (every
+// second one from g0 on); t0 may be up to three steps before the chain's
+// start, where the ring's SHRT_MAX keeps the state empty.
 template <int NW, int T, int MODE, int KIND>
 __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>& s, int t0, int ts, int te, int nch,
                                          int segs, int b, int wch, bool act, uint32_t (&spec)[NW])
@@ -364,7 +367,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
     const int lane = X.lane, k = X.k;
     const int Dr = labels_of<D>(J);
     // the descriptor's fields that the loop reads, in registers
-    const int minD = J.minD, maxD = J.maxD, wLast = J.w - 1, paths = J.paths, rl_n = X.e.rl_n, P2 = J.P2;
+    const int minD = J.minD, maxD = J.maxD, wLast = J.w - 1, P2 = J.P2;
     const int16_t* const Bg = J.base;
     const uint8_t* const Lg = J.left;
     int16_t* const Vg = J.V;
@@ -374,6 +377,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
     // number apart (of the same direction); from 64 on the chain of copy j
     // is a constant and its pieces lie a fixed number of pixels apart.
     constexpr bool kApart = G::PPC < 32;
+    static_assert(!ADD || !kApart, "the chains of a warp are two apart");
     constexpr int kChains = kApart ? 1 : G::CPW;            // start pointers a lane keeps
     constexpr int kStep = kApart ? 32 / G::PPC : 1;         // chains between two copies
     constexpr int kPer = kApart ? 1 : G::PPC / 32;          // copies per chain
@@ -386,10 +390,10 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
 #pragma unroll
     for (int i = 0; i < kChains; ++i) {
         const int cc = kApart ? lane / G::PPC : i;
-        const Walk w = walk_of<MODE>(J, X.e, X.rows, X.g0 + cc);
+        const Walk w = walk_of<MODE>(J, X.e, X.rows, X.g0 + cc * (ADD ? 2 : 1));
         const int len = ((w.n + segs - 1) / segs + kCH - 1) / kCH * kCH;
-        const int first = b * len, tb = first - wch * kCH;
-        lim[i] = w.n > 0 && off0 < Dr ? imin(w.n, first + len) - tb - q0 : -(1 << 30);
+        const int first = b * len, tb = ADD ? t0 : first - wch * kCH;
+        lim[i] = w.n > 0 && off0 < Dr ? (ADD ? X.stop : imin(w.n, first + len)) - tb - q0 : -(1 << 30);
         advD[i] = w.dp * Dr;
         src[i] = J.C + (w.p0 + (long long)w.dp * (tb + q0)) * Dr + off0;
         if (kApart) {
@@ -400,6 +404,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
     }
     const uint32_t dst0 =
         pk::smem_addr(X.ring + (kApart ? (lane / G::PPC) * G::CSTR : 0) + q0 * (D / 2) + off0 / 2);
+    const int early = -t0 - q0;   // ADD: pixels of the first chunk before the chain's start
     int ci_issue = 0;
     auto issue = [&](int slot) {
 #pragma unroll
@@ -408,7 +413,8 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
             const int i = kApart ? 0 : j / kPer, jj = kApart ? 0 : j % kPer;
             const int dq = kApart ? 0 : G::PPX <= 32 ? jj * kQ : jj / (G::PPX > 32 ? G::PPX / 32 : 1);
             const int doff = G::PPX <= 32 ? 0 : 256 * (jj % (G::PPX > 32 ? G::PPX / 32 : 1));
-            const bool in = kCH * ci_issue + dq < lim[i] && (kApart ? j < jmax : off0 + doff < Dr);
+            const bool in = kCH * ci_issue + dq < lim[i] && (!ADD || ci_issue > 0 || dq >= early) &&
+                            (kApart ? j < jmax : off0 + doff < Dr);
             const int16_t* p = src[i] + (kApart ? j * apart : (long long)dq * advD[i] + doff);
             const uint32_t dst =
                 dst0 + 4 * (slot * G::SLOTW + (kApart ? j * kStep : i) * G::CSTR + dq * (D / 2) + doff / 2);
@@ -441,7 +447,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
         for (int i = 0; i < G::QL; ++i) {
             const int tq = t + k + T * i;
             v[i] = {0u, 0u};
-            if (need && k < kCH && tq < te) load_pixel(tq, v[i]);
+            if (need && k < kCH && tq < te && (!ADD || tq >= 0)) load_pixel(tq, v[i]);
         }
     };
     Pixel pix[kAhead + 1][G::QL], first{0u, 0u};
@@ -559,30 +565,14 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
 #pragma unroll
             for (int i = 0; i < NW; ++i) res[i] = s.L[i];
             if constexpr (ADD) {
-                const int both = rl_n - 1 - 2 * (t + q);   // steps until the other direction gets here
-                uint32_t v[NW];
-                bool sum = paths >= 3 || (paths == 2 && both < 0);
-                if constexpr (kEarly) {
+                if (X.sums) {
+                    uint32_t v[NW];
+                    if constexpr (kEarly) {
 #pragma unroll
-                    for (int i = 0; i < NW; ++i) v[i] = ve[q][i];
-                } else {
-                    pk::ldw<NW>(cin + kSC * G::SLOTW + q * (D / 2), v);
-                }
-                if (paths >= 2 && both <= 0 && both > -2 * kCH * kSC) {
-                    if (both == 0) {   // the same pixel: L->R first
-                        if (put && !(X.c & 1)) {
-#pragma unroll
-                            for (int i = 0; i < NW; ++i)
-                                if (sum) res[i] = pk::gcombine<MODE != kSingle>(v[i], res[i]);
-                            store_words<NW>(op, 2 * NW * k, Dr, res);
-                        }
-                        put = put && (X.c & 1);
-                        sum = true;
+                        for (int i = 0; i < NW; ++i) v[i] = ve[q][i];
+                    } else {
+                        pk::ldw<NW>(cin + kSC * G::SLOTW + q * (D / 2), v);
                     }
-                    __syncwarp();
-                    if (put) load_words<NW>(op, 2 * NW * k, Dr, v);
-                }
-                if (sum) {
 #pragma unroll
                     for (int i = 0; i < NW; ++i) res[i] = pk::gcombine<MODE != kSingle>(v[i], res[i]);
                 }

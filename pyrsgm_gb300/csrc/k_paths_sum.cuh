@@ -12,43 +12,58 @@
 namespace pg {
 
 // Rows of both directions added to V, for the label counts that keep one
-// path volume (every one but 16, 32 and 64): a warp walks both directions of
-// 16 / T rows in step.  12 bytes per label move (the costs, V in and out, for
-// each direction).  Bound by the latency of a step (641x479 with 96 labels:
-// 89 us, 138 ns a step; 1316 us on scalar chains with the winner inside) and,
-// from 128 labels on, by memory (720p: 193 us, 215 before the reductions of
-// chain_min_dup; 2965 on scalar chains).
+// path volume (every one but 16, 32 and 64): a warp a direction, a block the
+// two of 32 / T rows.  Each direction comes first to half of the columns;
+// after a barrier it adds to what the other one left in the rest.  12 bytes
+// per label move (the costs, V in and out, for each direction).  Bound by
+// the latency of a step (641x479 with 96 labels: 81 us, 148 ns a step; 89
+// with both directions in one warp, 16 lanes each, which met in the middle
+// and read V again there; 1316 on scalar chains with the winner inside) and,
+// from 128 labels on, by memory (720p: 184 us, 193 and 2965).
 template <int NW, int T, int MODE, int NJ>
-__global__ void __launch_bounds__(32) k_rowadd(const __grid_constant__ Jobs<NJ> jobs)
+__global__ void __launch_bounds__(64) k_rowadd(const __grid_constant__ Jobs<NJ> jobs)
 {
     using namespace sg;
     using G = Geo<NW, T>;
     const LevelDesc& J = jobs.d[blockIdx.y];
     extern __shared__ __align__(16) uint32_t smem[];
-    const int lane = threadIdx.x, g0 = blockIdx.x * G::CPW;
-    if (g0 >= 2 * J.h) {
+    const int lane = threadIdx.x & 31, dir = threadIdx.x >> 5, row0 = blockIdx.x * G::CPW;
+    if (row0 >= J.h) {
         after_previous();
         return;
     }
     const Extent<MODE> e(J);
     int* lut = reinterpret_cast<int*>(smem);
-    uint32_t* mine = smem + 256;
+    uint32_t* mine = smem + 256 + dir * warp_words<NW, T, MODE>(2);
     for (int i = lane; i < warp_words<NW, T, MODE>(2); i += 32) mine[i] = kMax2;
     let_next_in();
     after_previous();
-    const bool guard = __any_sync(0xffffffffu, load_penalties(J, lut));
-    __syncwarp();
+    const bool guard = __syncthreads_or(load_penalties(J, lut));
     const int k = lane % T;
     Ctx<NW, T, MODE> X{J, lut, mine, mine + 2 * kSC * G::SLOTW + lane / T + NW * k * G::WST, nullptr, lane, lane / T, k,
-                       e, true, J.adaptive != 0, guard, g0, {}, J.V, pk::dup(imin(J.P1, 0x8000))};
-    X.w = walk_of<MODE>(J, e, true, g0 + X.c);
-    const int n = X.w.n, nch = (imax(e.lr_n, e.rl_n) + kCH - 1) / kCH;
+                       e, true, J.adaptive != 0, guard, 2 * row0 + dir, {}, J.V, pk::dup(imin(J.P1, 0x8000))};
+    X.w = walk_of<MODE>(J, e, true, 2 * (row0 + X.c) + dir);
+    // L->R comes first to the first `half` columns of its walk, R->L to the
+    // others.  Both first parts end on whole chunks: R->L starts `pad` steps
+    // early.
+    const int half = imin(e.lr_n, e.rl_n / 2) / kCH * kCH;
+    const int pad = dir ? (kCH - e.rl_n % kCH) % kCH : 0;
+    const int n = dir ? e.rl_n : e.lr_n, mid = dir ? e.rl_n - half : half;
+    const bool on = X.w.n > 0;
     State<NW, T> s;
     uint32_t spec[NW];
 #pragma unroll
     for (int i = 0; i < NW; ++i) s.L[i] = spec[i] = kMax2;
     s.mp2 = kMax2;
-    seg_walk<NW, T, MODE, kAdd>(X, s, 0, 0, n > 0 ? n : -(1 << 30), nch, 1, 0, 0, true, spec);
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {
+        const int t0 = part ? mid : -pad;
+        X.stop = part ? n : mid;
+        X.sums = J.paths >= 3 || part;
+        const int nch = (X.stop - t0 + kCH - 1) / kCH;
+        seg_walk<NW, T, MODE, kAdd>(X, s, t0, imax(t0, 0), on ? X.stop : -(1 << 30), nch, 1, 0, 0, true, spec);
+        __syncthreads();   // what the other direction has left
+    }
 }
 
 template <int NW, int T, int MODE, int NJ>
@@ -60,7 +75,7 @@ cudaError_t launch_rowadd_mode(const Jobs<NJ>& jobs, const LevelExtent& e, cudaS
         cudaFuncSetAttribute(k_rowadd<NW, T, MODE, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     prof_begin(st);
-    launch_after(k_rowadd<NW, T, MODE, NJ>, dim3((2 * e.max_h + G::CPW - 1) / G::CPW, jobs.n), 32, smem, st, jobs);
+    launch_after(k_rowadd<NW, T, MODE, NJ>, dim3((e.max_h + G::CPW - 1) / G::CPW, jobs.n), 64, smem, st, jobs);
     count_launch();
     if (prof_enabled()) {
         // each direction reads the cost volume; V is read (T->B or the first
@@ -77,14 +92,18 @@ cudaError_t launch_rowadd_mode(const Jobs<NJ>& jobs, const LevelExtent& e, cudaS
     return launched(st, "k_rowadd");
 }
 
-// Columns into V, rows added to it, the winner from it.
-template <int NW, int T, int G, int R, bool PYR, int NJ>
+// Columns into V, rows added to it, the winner from it.  On rows of fixed
+// labels a chain takes twice the threads, of half the words, up to a whole
+// warp (RNW, RT): their warps are few and wait for each step (720p, 96
+// labels or so at 4 x 16 against 2 x 32: 80 labels 397 and 324 us a call, 128
+// 452 and 411).
+template <int NW, int T, int G, int R, bool PYR, int NJ, int RNW = NW, int RT = T>
 cudaError_t launch_sum(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
 {
     cudaError_t err = launch_seg<NW, T, PYR, NJ>(jobs, false, st);
     if (err != cudaSuccess) return err;
     if constexpr (!PYR) {
-        err = launch_rowadd_mode<NW, T, sg::kSingle, NJ>(jobs, e, st);
+        err = launch_rowadd_mode<RNW, RT, sg::kSingle, NJ>(jobs, e, st);
     } else {
         Jobs<NJ> part;
         for (int ref = 0; ref < 2 && err == cudaSuccess; ++ref) {
@@ -94,9 +113,9 @@ cudaError_t launch_sum(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t 
             if (part.n == 0) continue;
             if constexpr (2 * NW * T <= kMaxRefineLabels) {
                 err = ref ? launch_rowadd_mode<NW, T, sg::kRefine, NJ>(part, e, st)
-                          : launch_rowadd_mode<NW, T, sg::kCoarse, NJ>(part, e, st);
+                          : launch_rowadd_mode<RNW, RT, sg::kCoarse, NJ>(part, e, st);
             } else {
-                err = ref ? cudaErrorInvalidValue : launch_rowadd_mode<NW, T, sg::kCoarse, NJ>(part, e, st);
+                err = ref ? cudaErrorInvalidValue : launch_rowadd_mode<RNW, RT, sg::kCoarse, NJ>(part, e, st);
             }
         }
     }
@@ -113,9 +132,9 @@ template <bool PYR, int NJ>
 cudaError_t launch_paths_sum(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
 {
     switch (path_variant(jobs.d[0].D)) {
-    case 64: return launch_sum<4, 8, 4, 1, PYR, NJ>(jobs, e, st);
-    case 128: return launch_sum<4, 16, 8, 1, PYR, NJ>(jobs, e, st);
-    case 256: return launch_sum<8, 16, 16, 1, PYR, NJ>(jobs, e, st);
+    case 64: return launch_sum<4, 8, 4, 1, PYR, NJ, 2, 16>(jobs, e, st);
+    case 128: return launch_sum<4, 16, 8, 1, PYR, NJ, 2, 32>(jobs, e, st);
+    case 256: return launch_sum<8, 16, 16, 1, PYR, NJ, 4, 32>(jobs, e, st);
     case 512: return launch_sum<16, 16, 32, 1, PYR, NJ>(jobs, e, st);
     case 1024: return launch_sum<32, 16, 32, 2, PYR, NJ>(jobs, e, st);
     default: return cudaErrorInvalidValue;

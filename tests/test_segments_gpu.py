@@ -99,3 +99,18 @@ def test_one_volume_large_label_counts_match_the_oracle(w, h, D):
 def test_one_volume_pyramid_levels_match_the_oracle(refine, paths, w, h, D):
     _check(cases._lvl("sum", w, h, D, cases.BT if D == 48 else cases.CENSUS, refine, paths=paths, adaptive=paths != 2,
                       maxD=min(w - 1, 2 * D), seed=w))
+
+
+# ... and walks of a few steps, whose parts are less than a chunk.
+@pytest.mark.parametrize("extra", [1, 2, 3, 4, 5, 7, 9, 14])
+@pytest.mark.parametrize("D", [48, 80, 128, 144])
+@pytest.mark.parametrize("paths,minD", [(1, 0), (2, 0), (3, 0), (3, -3), (2, 4)])
+def test_one_volume_short_rows_match_the_oracle(extra, D, paths, minD):
+    _check(cases._ss("sum", D + max(minD, 0) + extra, 19, D, cases.CENSUS, paths=paths, minD=minD, adaptive=extra % 2 == 1))
+
+
+@pytest.mark.parametrize("w", [49, 50, 51, 52, 55])
+@pytest.mark.parametrize("refine", [False, True])
+@pytest.mark.parametrize("paths", [1, 2, 3])
+def test_one_volume_narrow_levels_match_the_oracle(w, refine, paths):
+    _check(cases._lvl("sum", w, 23, 48, cases.BT, refine, paths=paths, adaptive=paths != 2, seed=w))
