@@ -125,11 +125,11 @@ __device__ __forceinline__ void load_words(const int16_t* p, int d0, int Dr, uin
     }
 }
 
-template <int NW>
+template <int NW, bool FULL>   // FULL: the level has every label of the chain
 __device__ __forceinline__ void store_words(int16_t* p, int d0, int Dr, const uint32_t (&v)[NW])
 {
     if constexpr (NW == 2) {
-        if (d0 < Dr) *reinterpret_cast<uint2*>(p) = make_uint2(v[0], v[1]);
+        if (FULL || d0 < Dr) *reinterpret_cast<uint2*>(p) = make_uint2(v[0], v[1]);
     } else {
 #pragma unroll
         for (int i = 0; i < NW / 4; ++i) {
@@ -578,7 +578,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
                 }
             }
             if (put && PG_IN(op - X.out, imin(2 * NW, Dr - 2 * NW * k), (size_t)J.w * J.h * Dr, 6))
-                store_words<NW>(op, 2 * NW * k, Dr, res);
+                store_words<NW, D <= 32>(op, 2 * NW * k, Dr, res);
             op += ostep;
         }
         if constexpr (FIX) {

@@ -94,9 +94,9 @@ cudaError_t launch_rowadd_mode(const Jobs<NJ>& jobs, const LevelExtent& e, cudaS
 
 // Columns into V, rows added to it, the winner from it.  On rows of fixed
 // labels a chain takes twice the threads, of half the words, up to a whole
-// warp (RNW, RT): their warps are few and wait for each step (720p, 96
-// labels or so at 4 x 16 against 2 x 32: 80 labels 397 and 324 us a call, 128
-// 452 and 411).
+// warp (RNW, RT): their warps are few and wait for each step (720p Census,
+// 4 words on 16 lanes against 2 on 32: 80 labels 397 and 324 us a call, 128
+// labels 452 and 411).
 template <int NW, int T, int G, int R, bool PYR, int NJ, int RNW = NW, int RT = T>
 cudaError_t launch_sum(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st)
 {
