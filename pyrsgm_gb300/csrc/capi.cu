@@ -201,7 +201,15 @@ int run_level_single(const LevelDesc& d, cudaStream_t st, float alpha, float bet
     if (d.adaptive) err = launch_p2_table(const_cast<int*>(d.p2lut), d.P2, alpha, beta, lower, upper, st);
     if (err == cudaSuccess) err = launch_prepare(j, e, st);
     if (err == cudaSuccess) err = launch_cost(j, e, st);
-    if (err == cudaSuccess) err = launch_paths(j, e, st);
+    if (err == cudaSuccess) {
+        // the packed chains hold path costs as unsigned halves: no penalty below zero
+        if (d.P1 < 0 || d.P2 < 0) {
+            err = launch_paths_signed(d, st);
+            j.d[0].post &= ~POST_LRCHECK;   // done
+        } else {
+            err = launch_paths(j, e, st);
+        }
+    }
     if (err == cudaSuccess) err = launch_post(j, e, st);
     if (err != cudaSuccess) {
         std::fprintf(stderr, "pyrsgm-gb300 %s: %s\n", what, cudaGetErrorString(err));

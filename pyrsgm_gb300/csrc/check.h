@@ -14,7 +14,8 @@
 // Sites: 1, 2 k_gtb cost loads and path-cost stores; 3, 4 k_grow cost runs
 // in and path-cost runs out; 5, 6 k_seg loads and stores; 7 k_gtbw
 // loads; 8 k_post disparity output; 9 k_features feature row; 10
-// k_cost_census cost row; 11 k_cost_bt_tiled cost row.
+// k_cost_census cost row; 11 k_cost_bt_tiled cost row; 12 k_path_signed
+// sums.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -170,6 +170,9 @@ cudaError_t launch_cost(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t
 // All jobs in one call share pyr (mode) and the path shape of their D.
 template <int NJ>
 cudaError_t launch_paths(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st);
+// Paths, winner and LR check of one level with a penalty below zero
+// (k_paths_signed.cu); the post pass is left without the check.
+cudaError_t launch_paths_signed(const LevelDesc& d, cudaStream_t st);
 template <int NJ>
 cudaError_t launch_post(const Jobs<NJ>& jobs, const LevelExtent& e, cudaStream_t st);
 
