@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(256) k_pyrdown(const __grid_constant__ PyrDown
 // ---------------------------------------------------------------------------
 // Features.  Census: 5x5, replicate borders, MSB first, dy-major, bit =
 // neighbour < centre (src/sgm_kernels.cu:251-298).  BT: the Sobel-like
-// x-gradient clipped to +-ftzero and offset by ftzero
+// x-gradient clipped to +-ftzero and offset by ftzero, as a byte
 // (src/sgm_kernels.cu:94-118), plus for both the gradient and intensity
 // channels the half-sample interval [lo, hi] of dev_bt_channel_cost
 // (src/sgm_kernels.cu:1002-1028) with clamped neighbours.  Census pixels
@@ -280,7 +280,9 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
     }
     __syncthreads();
     if (y >= H) return;
-    const int ftzero = imax(J.pfc, 15) | 1;
+    // The gradient (at most 1020) is a byte in the reference: with a cap from
+    // 128 on, gradient + cap wraps.
+    const int ftzero = imax(J.pfc, 15) | 1, clip = imin(ftzero, 1020), offset = ftzero & 255;
     {
         const size_t p = (size_t)y * W + xb;
         if (!PG_IN((size_t)y * W + x0, imin(kFtX, W - x0), (size_t)W * H, 9)) return;
@@ -323,7 +325,7 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
         } else {
             // columns xb - 1 .. xb + 4 of the three rows as 16-bit pairs
             // (xb - 1, xb), (xb + 1, xb + 2), (xb + 3, xb + 4)
-            const uint32_t lim = (uint32_t)ftzero * 0x10001u;
+            const uint32_t lim = (uint32_t)clip * 0x10001u, off2 = (uint32_t)offset * 0x10001u;
             uint32_t v[3] = {0u, 0u, 0u}, mid[3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
@@ -340,7 +342,7 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
             uint32_t g[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i)
-                g[i] = __vadd2(__vmaxs2(__vmins2(__vsub2(v[i + 1], v[i]), lim), __vsub2(0u, lim)), lim);
+                g[i] = __vadd2(__vmaxs2(__vmins2(__vsub2(v[i + 1], v[i]), lim), __vsub2(0u, lim)), off2) & 0x00ff00ffu;
             // intensities (xb, xb + 1), (xb + 2, xb + 3)
             const uint32_t in0 = __byte_perm(mid[0], mid[1], 0x5432), in1 = __byte_perm(mid[1], mid[2], 0x5432);
             *reinterpret_cast<uint4*>(&gi[rr][4 + 4 * tx]) =
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
                     const uint8_t* r = tb + (rr + 1 + k) * kFtSWB + c;
                     d += (k == 1 ? 2 : 1) * ((int)r[1] - (int)r[-1]);
                 }
-                gi[rr][c] = (uint32_t)(iclamp(d, -ftzero, ftzero) + ftzero) | (uint32_t)tb[(rr + 2) * kFtSWB + c] << 16;
+                gi[rr][c] = (uint32_t)((iclamp(d, -clip, clip) + offset) & 255) | (uint32_t)tb[(rr + 2) * kFtSWB + c] << 16;
             }
             __syncwarp();
             uint4* out = feat + (size_t)y * W;
