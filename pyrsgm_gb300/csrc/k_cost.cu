@@ -1201,8 +1201,7 @@ cudaError_t launch_bt_strip(const Jobs<NJ>& jobs, cudaStream_t st)
             best = turns;
         }
     }
-    const cudaError_t err =
-        cudaFuncSetAttribute(k_cost_bt_strip<HW, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t err = allow_smem(k_cost_bt_strip<HW, NJ>);
     if (err != cudaSuccess) return err;
     launch_after(k_cost_bt_strip<HW, NJ>, dim3(gx, (max_h + strip - 1) / strip, jobs.n), kBsThreads, smem, st, jobs, strip);
     return cudaGetLastError();
@@ -1237,8 +1236,7 @@ cudaError_t launch_bt_fixed(const Jobs<NJ>& jobs, cudaStream_t st)
         else {
             const int SW = kBxX + 2 * maxHalf, SH = kBxY + 2 * maxHalf;
             const size_t smem = ((SH * SW * kBxD + 15) & ~15) + (size_t)SH * kBxX * kBxD * 2;
-            if (smem > 48 * 1024)
-                err = cudaFuncSetAttribute(k_cost_bt_box<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (smem > 48 * 1024) err = allow_smem(k_cost_bt_box<NJ>);
             if (err != cudaSuccess) return err;
             const int nxt = (max_w + kBxX - 1) / kBxX;
             dim3 g(nxt * ((max_D + kBxD - 1) / kBxD), (max_h + kBxY - 1) / kBxY, part.n);

@@ -716,7 +716,6 @@ __global__ void __launch_bounds__(sg::max_seg<NW>() * 32) k_seg(const __grid_con
 // levels (160x96: 42 us a call, 46 at 64).
 constexpr int kMinSeg = 64, kMinSegSmall = 40;
 constexpr int kMaxRefineLabels = 256;   // pyrsgm_compute_level takes no more on a refinement level
-constexpr size_t kSmemPerBlock = 227 * 1024;
 constexpr int kWarmSteps = 16;   // 0 to 32 measured within 5 % of each other, 64 10 % slower
 
 template <int MODE>
@@ -748,8 +747,7 @@ cudaError_t launch_seg_mode(const Jobs<NJ>& jobs, bool rows_too, cudaStream_t st
     int segs = segments_for<MODE>(blocks, n, rows_too, sg::max_seg<NW>());
     while (segs > 1 && sg::seg_smem<NW, T, MODE>(segs) > kSmemPerBlock) --segs;
     const size_t smem = sg::seg_smem<NW, T, MODE>(segs);
-    const cudaError_t err =
-        cudaFuncSetAttribute(k_seg<NW, T, MODE, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t err = allow_smem(k_seg<NW, T, MODE, NJ>);
     if (err != cudaSuccess) return err;
     prof_begin(st);
     launch_after(k_seg<NW, T, MODE, NJ>, dim3(grid, jobs.n), segs * 32, smem, st, jobs, rows_too ? 1 : 0, kWarmSteps);

@@ -153,6 +153,20 @@ void launch_after(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaS
     cudaLaunchKernelExC(&c, reinterpret_cast<const void*>(kernel), p);
 }
 
+// Dynamic shared memory of kernels whose launches need different amounts.
+// The limit set here belongs to the kernel on the device, not to the thread
+// or the launch: set to what each launch needs, a second thread could lower
+// it between the set and the launch of the first.  So every launch sets the
+// same, the most a block can have (such a kernel has no static shared
+// memory); what a launch takes is its own argument still.
+constexpr int kSmemPerBlock = 227 * 1024;
+template <class... P>
+cudaError_t allow_smem(void (*kernel)(P...))
+{
+    return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kSmemPerBlock);
+}
+
 // Count of kernel launches issued by this library (process-wide); a CUDA
 // graph replay counts the kernels it contains.
 void count_launch();
