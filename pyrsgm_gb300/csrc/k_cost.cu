@@ -31,15 +31,15 @@ __device__ __forceinline__ uint32_t load4(const uint8_t* row, int c, int w, cons
     if (c >= 0 && c + 4 <= w) {
         const unsigned s = (unsigned)(reinterpret_cast<uintptr_t>(row + c) & 3u);
         const uint8_t* a = row + c - s;
-        if (s == 0) return __ldg(reinterpret_cast<const uint32_t*>(a));
+        if (s == 0) return *reinterpret_cast<const uint32_t*>(a);
         if (a >= first && a + 8 <= end) {
             const uint32_t* q = reinterpret_cast<const uint32_t*>(a);
-            return __funnelshift_r(__ldg(q), __ldg(q + 1), 8 * s);
+            return __funnelshift_r(*q, q[1], 8 * s);
         }
     }
     uint32_t v = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v |= (uint32_t)__ldg(row + map(c + j)) << (8 * j);
+    for (int j = 0; j < 4; ++j) v |= (uint32_t)row[map(c + j)] << (8 * j);
     return v;
 }
 
@@ -79,9 +79,9 @@ __global__ void __launch_bounds__(256) k_pyrdown(const __grid_constant__ PyrDown
         for (int r = warp; r < kPdSH; r += 8) {
             const uint32_t* q =
                 reinterpret_cast<const uint32_t*>(first + (size_t)reflect101(sy0 + r, sh) * P.sstep + sx0) + tx;
-            if (in0) tw[r][tx] = __ldg(q);
-            if (in1) tw[r][tx + 32] = __ldg(q + 32);
-            if (in2) tw[r][tx + 64] = __ldg(q + 64);
+            if (in0) tw[r][tx] = *q;
+            if (in1) tw[r][tx + 32] = q[32];
+            if (in2) tw[r][tx + 64] = q[64];
         }
         // the words with columns outside that an output needs: the first one, and from `from` on
         const int left = sx0 < 0 ? 1 : 0, from = imax((sw - sx0) >> 2, left);
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256) k_pyrdown(const __grid_constant__ PyrDown
             const uint8_t* row = first + (size_t)reflect101(sy0 + r, sh) * P.sstep;
             uint32_t v = 0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v |= (uint32_t)__ldg(row + reflect101(sx0 + 4 * k + j, sw)) << (8 * j);
+            for (int j = 0; j < 4; ++j) v |= (uint32_t)row[reflect101(sx0 + 4 * k + j, sw)] << (8 * j);
             tw[r][k] = v;
         }
     } else {
@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
 #pragma unroll
         for (int j = 0; j < 2; ++j) {   // xb is even: pixels 2 j and 2 j + 1 have one parent
             const int px = imin((xb >> 1) + j, J.pw - 1);
-            praw[2 * j] = praw[2 * j + 1] = __ldg(prow + px);
-            pcf[2 * j] = pcf[2 * j + 1] = __ldg(crow + px);
+            praw[2 * j] = praw[2 * j + 1] = prow[px];
+            pcf[2 * j] = pcf[2 * j + 1] = crow[px];
         }
     }
     if (((reinterpret_cast<uintptr_t>(img) | (uintptr_t)step) & 3u) == 0) {
@@ -254,8 +254,8 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
         for (int r = rr; r < kFtSH; r += 8) {
             const uint32_t* q =
                 reinterpret_cast<const uint32_t*>(img + (size_t)iclamp(y0 - 2 + r, 0, H - 1) * step + x0 - 4) + tx;
-            if (in0) tw[r][tx] = __ldg(q);
-            if (in1) tw[r][tx + 32] = __ldg(q + 32);
+            if (in0) tw[r][tx] = *q;
+            if (in1) tw[r][tx + 32] = q[32];
         }
         // the words with columns outside that a pixel needs: the first one, and from `from` on
         const int left = x0 == 0 ? 1 : 0, from = imax((W - x0 + 4) >> 2, left);
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
             const uint8_t* row = img + (size_t)iclamp(y0 - 2 + r, 0, H - 1) * step;
             uint32_t v = 0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v |= (uint32_t)__ldg(row + iclamp(x0 - 4 + 4 * k + j, 0, W - 1)) << (8 * j);
+            for (int j = 0; j < 4; ++j) v |= (uint32_t)row[iclamp(x0 - 4 + 4 * k + j, 0, W - 1)] << (8 * j);
             tw[r][k] = v;
         }
     } else {
@@ -459,8 +459,8 @@ __global__ void __launch_bounds__(256) k_cost_census(const __grid_constant__ Job
 #pragma unroll
     for (int r = 0; r < kCnRows; ++r) {
         const size_t p = p0 + (size_t)(r < rows ? r : 0) * W;
-        cl[r] = __ldg(fl + p);
-        off[r] = J.refine ? (int)__ldg(J.base + p) : J.minD;
+        cl[r] = fl[p];
+        off[r] = J.refine ? (int)J.base[p] : J.minD;
     }
 #pragma unroll
     for (int r = 0; r < kCnRows; ++r) {
@@ -480,11 +480,11 @@ __global__ void __launch_bounds__(256) k_cost_census(const __grid_constant__ Job
         const uint32_t* q = fr + (p - x) + (x - off[r] - d0);
         if (lo <= d0 && hi >= d0 + 7) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) c[k] = (uint32_t)__popc(cl[r] ^ __ldg(q - k));
+            for (int k = 0; k < 8; ++k) c[k] = (uint32_t)__popc(cl[r] ^ q[-k]);
         } else {
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-                c[k] = d0 + k >= lo && d0 + k <= hi ? (uint32_t)__popc(cl[r] ^ __ldg(q - k)) : (uint32_t)fill;
+                c[k] = d0 + k >= lo && d0 + k <= hi ? (uint32_t)__popc(cl[r] ^ q[-k]) : (uint32_t)fill;
         }
         if (!PG_IN(p * D + d0, 8, (size_t)W * J.h * D, 10)) continue;
         *reinterpret_cast<uint4*>(J.C + p * D + d0) =
@@ -1094,11 +1094,11 @@ __global__ void __launch_bounds__(256, 3) k_cost_bt_tiled(const __grid_constant_
                         const uint4* rrow = J.featR + (size_t)gy * W;
                         for (int dx = -h; dx <= h; ++dx) {
                             const int gx = iclamp(x + dx, 0, W - 1);
-                            const uint4 lf = __ldg(&lrow[gx]);
+                            const uint4 lf = lrow[gx];
     #pragma unroll
                             for (int q = 0; q < 8; ++q) {
                                 const int x2 = gx - (b + d0 + q);
-                                sum[q] += (x2 >= 0 && x2 < W) ? (int)bt_pixel(lf, __ldg(&rrow[x2])) : 255;
+                                sum[q] += (x2 >= 0 && x2 < W) ? (int)bt_pixel(lf, rrow[x2]) : 255;
                             }
                         }
                     }

@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(256) k_wta(const __grid_constant__ Jobs<NJ> jo
     auto load = [&](const int16_t* v, uint32_t (&o)[DW]) {
 #pragma unroll
         for (int i = 0; i < DW / 4; ++i) {
-            const uint4 q = __ldg(reinterpret_cast<const uint4*>(v + p * D) + i);
+            const uint4 q = reinterpret_cast<const uint4*>(v + p * D)[i];
             o[4 * i] = q.x; o[4 * i + 1] = q.y; o[4 * i + 2] = q.z; o[4 * i + 3] = q.w;
         }
     };

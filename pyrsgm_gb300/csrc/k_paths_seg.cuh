@@ -439,8 +439,8 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
         uint32_t base, img;
     };
     auto load_pixel = [&](int t, Pixel& v) {
-        if (MODE == kRefine) v.base = (uint32_t)(uint16_t)__ldg(Bg + X.w.p0 + (long long)X.w.dp * t);
-        if (X.adaptive) v.img = __ldg(Lg + X.w.l0 + (long long)X.w.dl * t);
+        if (MODE == kRefine) v.base = (uint32_t)(uint16_t)Bg[X.w.p0 + (long long)X.w.dp * t];
+        if (X.adaptive) v.img = Lg[X.w.l0 + (long long)X.w.dl * t];
     };
     auto load_chunk = [&](int t, Pixel (&v)[G::QL]) {
 #pragma unroll

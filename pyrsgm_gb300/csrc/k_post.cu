@@ -85,12 +85,12 @@ __global__ void __launch_bounds__(kPoThreads) k_post(const __grid_constant__ Job
     if (np > 0) {
         const float* c = J.conf_raw + (size_t)y * W + xb;
         if (quad) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(c));
+            const float4 v = *reinterpret_cast<const float4*>(c);
             cin[0] = v.x; cin[1] = v.y; cin[2] = v.z; cin[3] = v.w;
         } else {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (j < np) cin[j] = __ldg(c + j);
+                if (j < np) cin[j] = c[j];
         }
     }
     if (threadIdx.x < kPoN) {
@@ -102,11 +102,11 @@ __global__ void __launch_bounds__(kPoThreads) k_post(const __grid_constant__ Job
         if (in) {
             const int16_t* p = J.disp_raw + (size_t)yy * W + xg;
             if (quad) {
-                a = __ldg(reinterpret_cast<const uint2*>(p));
+                a = *reinterpret_cast<const uint2*>(p);
             } else {
                 uint32_t v[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) v[j] = xg + j < W ? (uint32_t)(uint16_t)__ldg(p + j) : (uint32_t)(uint16_t)inv;
+                for (int j = 0; j < 4; ++j) v[j] = xg + j < W ? (uint32_t)(uint16_t)p[j] : (uint32_t)(uint16_t)inv;
                 a = make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
             }
         }
@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(kPoThreads) k_post(const __grid_constant__ Job
                 const int d = (int)(int16_t)(j < 2 ? a.x >> (16 * j) : a.y >> (16 * (j - 2)));
                 const int r0 = xg + j - (d >> 4), r1 = xg + j - ((d + 15) >> 4);
                 k0[j] = k1[j] = 0xffffffffu;
-                if ((unsigned)r0 < (unsigned)W) k0[j] = __ldg(row + r0);
-                if ((unsigned)r1 < (unsigned)W) k1[j] = __ldg(row + r1);
+                if ((unsigned)r0 < (unsigned)W) k0[j] = row[r0];
+                if ((unsigned)r1 < (unsigned)W) k1[j] = row[r1];
             }
             bool bad[4];
             if (inv < J.minD && maxdiff >= 0 && maxdiff <= 65536) {

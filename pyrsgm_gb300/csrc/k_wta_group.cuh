@@ -24,7 +24,7 @@ namespace pg {
 
 __device__ __forceinline__ void load16(const int16_t* p, uint32_t (&v)[8])
 {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+    const uint4 *q = reinterpret_cast<const uint4*>(p), a = q[0], b = q[1];
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
     v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
@@ -134,8 +134,8 @@ __global__ void __launch_bounds__(256) k_wta_group(const __grid_constant__ Jobs<
     }
     const int minCost = (int)(myBest >> 16), bd = (int)(myBest & 0xffffu);
     if constexpr (VOLS == 1) {
-        c0 = bd > 0 ? (int)__ldg(row + (size_t)x * D + bd - 1) : 0;
-        c2 = bd + 1 < D ? (int)__ldg(row + (size_t)x * D + bd + 1) : 0;
+        c0 = bd > 0 ? (int)row[(size_t)x * D + bd - 1] : 0;
+        c2 = bd + 1 < D ? (int)row[(size_t)x * D + bd + 1] : 0;
     }
     const int base = (PYR && J.refine) ? (int)J.base[p] : J.minD;
     pk::wta_out<PYR>(J, D, y, x, base, minCost, bd, myAlt, c0, minCost, c2);

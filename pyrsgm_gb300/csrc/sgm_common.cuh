@@ -89,6 +89,10 @@ __host__ __device__ __forceinline__ bool uses_packed(int D) { return D == 16 || 
 // the SMs that finish first (with it in every kernel the rows of a 720p level
 // with 128 labels took half as long again, and 32 pairs 9.8 instead of 9.0
 // ms).
+// What a kernel of the stream has written is read with plain loads (or
+// __ldcg), never with __ldg: that one is for memory no kernel writes while
+// the reading one is resident, and this one may be resident while the one
+// before still writes; nothing would have to keep it behind the wait.
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
