@@ -974,7 +974,8 @@ __global__ void __launch_bounds__(256, 3) k_cost_bt_tiled(const __grid_constant_
         // one; a pass costs less than the window sums of a few pixels, and
         // two passes at most left 1-2 % of the pixels to those (a seventh of
         // the kernel's instructions, in blocks that outlasted the others).
-        bool todo[2] = {hasq[0] && h <= kTiMaxHalf, hasq[1] && h <= kTiMaxHalf};
+        const bool tiled = h >= 0 && h <= kTiMaxHalf;   // (a negative block size: an empty window)
+        bool todo[2] = {hasq[0] && tiled, hasq[1] && tiled};
         for (int c = 0; c < kTiClusters; ++c) {
             int low, top;
             TileArea area;
@@ -1079,8 +1080,7 @@ __global__ void __launch_bounds__(256, 3) k_cost_bt_tiled(const __grid_constant_
 #pragma unroll 1
         for (int i = 0; i < 2; ++i) {
             const bool in = i ? inq[1] : inq[0], has = i ? hasq[1] : hasq[0], left = i ? todo[1] : todo[0];
-            const bool wide = h > kTiMaxHalf;   // no clusters at all
-            if (!in || (has && !left && !wide)) continue;
+            if (!in || (has && !left && tiled)) continue;
             const int y = i ? yq[1] : yq[0], b = i ? bq[1] : bq[0];
             int lo, hi;
             label_range(J, x, b, lo, hi);
@@ -1208,7 +1208,8 @@ cudaError_t launch_bt_strip(const Jobs<NJ>& jobs, cudaStream_t st)
 }
 
 // BT cost of fixed disparities: by window size, 3 to 7 pixels in strips, any
-// other through k_cost_bt_box.
+// other through k_cost_bt_box.  The C entry points take any block size: a
+// negative one has empty windows, whose sums are 0.
 template <int NJ>
 cudaError_t launch_bt_fixed(const Jobs<NJ>& jobs, cudaStream_t st)
 {
@@ -1221,6 +1222,11 @@ cudaError_t launch_bt_fixed(const Jobs<NJ>& jobs, cudaStream_t st)
             const LevelDesc& d = jobs.d[i];
             const int h = d.bs / 2;
             if ((h >= 1 && h <= 3 ? h : 0) != half) continue;
+            if (h < 0) {
+                const cudaError_t err = cudaMemsetAsync(d.C, 0, (size_t)d.w * d.h * d.D * sizeof(int16_t), st);
+                if (err != cudaSuccess) return err;
+                continue;
+            }
             part.d[part.n++] = d;
             maxHalf = std::max(maxHalf, h);
             max_w = std::max(max_w, d.w);
@@ -1234,8 +1240,9 @@ cudaError_t launch_bt_fixed(const Jobs<NJ>& jobs, cudaStream_t st)
         else if (half == 2) err = launch_bt_strip<2, NJ>(part, st);
         else if (half == 3) err = launch_bt_strip<3, NJ>(part, st);
         else {
-            const int SW = kBxX + 2 * maxHalf, SH = kBxY + 2 * maxHalf;
-            const size_t smem = ((SH * SW * kBxD + 15) & ~15) + (size_t)SH * kBxX * kBxD * 2;
+            const size_t SW = kBxX + 2 * (size_t)maxHalf, SH = kBxY + 2 * (size_t)maxHalf;
+            const size_t smem = SH * SW * kBxD + SH * kBxX * kBxD * 2;
+            if (smem > kSmemPerBlock) return cudaErrorInvalidValue;
             if (smem > 48 * 1024) err = allow_smem(k_cost_bt_box<NJ>);
             if (err != cudaSuccess) return err;
             const int nxt = (max_w + kBxX - 1) / kBxX;
