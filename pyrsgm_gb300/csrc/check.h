@@ -12,10 +12,12 @@
 // for pyrsgm_gb300_check_report.
 //
 // Sites: 1, 2 k_gtb cost loads and path-cost stores; 3, 4 k_grow cost runs
-// in and path-cost runs out; 5, 6 k_seg loads and stores; 7 k_gtbw
-// loads; 8 k_post disparity output; 9 k_features feature row; 10
-// k_cost_census cost row; 11 k_cost_bt_tiled cost row; 12 k_path_signed
-// sums.
+// in and path-cost runs out; 5, 6 k_seg and k_rowadd loads (of the costs; the
+// sums k_rowadd adds to lie at the same index of a volume of the same size)
+// and stores; 7 k_gtbw loads; 8 k_post disparity output; 9 k_features feature
+// row; 10 k_cost_census cost row; 11 k_cost_bt_tiled cost row; 12
+// k_path_signed sums; 13 k_cost_bt_strip cost stores; 14 k_wta_group volume
+// loads.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -747,7 +747,7 @@ __global__ void __launch_bounds__(kBsThreads) k_cost_bt_strip(const __grid_const
                     const uint2 a = *reinterpret_cast<const uint2*>(add + (r * TX + step * i) * db);
                     run[i].x += a.x;
                     run[i].y += a.y;
-                    if (put && x0 + xq + step * i < W)
+                    if (put && x0 + xq + step * i < W && PG_IN(orow - J.C + (long long)step * i * D, 4, (size_t)W * H * D, 13))
                         *reinterpret_cast<uint2*>(orow + (size_t)(step * i) * D) = run[i];
                     run[i].x -= before[i][0].x;
                     run[i].y -= before[i][0].y;

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(256) k_wta_group(const __grid_constant__ Jobs<
             uint32_t v[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) v[j] = pk::kMax2;
-            if (d0 < D) {
+            if (d0 < D && PG_IN(row0 + (size_t)x * D + d0, 16, (size_t)W * J.h * D, 14)) {
                 const size_t at = (size_t)x * D + d0;
                 load16((VOLS == 1 ? row : J.Vr + row0) + at, v);
                 if constexpr (VOLS == 3) {

@@ -1,6 +1,6 @@
-"""Rules of the CUDA sources that hold for kernels which may be resident while
-the kernel before them still writes (sgm_launch.h: launch_after), checked on
-the text."""
+"""Rules of the CUDA sources, checked on their text: those for kernels which
+may be resident while the kernel before them still writes (sgm_launch.h:
+launch_after), and the list of the checked build's sites."""
 import glob
 import os
 import re
@@ -50,3 +50,18 @@ def test_kernels_let_in_early_wait_for_the_one_before():
         assert wait, k
         # (an early return waits in its own block)
         assert "return" not in before and not re.search(r"J\.\w+\s*\[|cp16|tile_cp16|atomic", before), k
+
+
+def test_check_sites_are_the_listed_ones():
+    """The sites that check.h lists are those of the kernels, each its number,
+    and every kernel that writes or reads a volume has one."""
+    with open(os.path.join(CSRC, "check.h")) as h:
+        text = re.sub(r"\n//", " ", h.read())
+    listed = text[text.index("Sites: "):text.index("#pragma once")]
+    listed = re.sub(r"\([^)]*\)", "", listed)
+    numbers = {int(n) for n in re.findall(r"(?<![\w-])(\d+)(?=[ ,])", listed)}
+    used = {int(n) for f, t in _code().items() for n in re.findall(r"PG_IN\((?:[^;{]*?), (\d+)\)", t)}
+    assert used == numbers == set(range(1, max(numbers) + 1))
+    for k in ("k_seg", "k_rowadd", "k_grow", "k_gtb", "k_gtbw", "k_post", "k_features", "k_cost_census",
+              "k_cost_bt_tiled", "k_cost_bt_strip", "k_path_signed", "k_wta_group"):
+        assert re.search(r"\b" + k + r"\b", listed), k
