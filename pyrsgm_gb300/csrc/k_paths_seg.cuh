@@ -61,6 +61,7 @@ __host__ __device__ constexpr int max_seg() { return NW >= 32 ? 4 : NW >= 16 ? 8
 
 template <int NW, int T>
 struct Geo {
+    static_assert(T >= 2, "a chain is held by several lanes");
     static constexpr int D = 2 * NW * T;     // labels a chain can hold
     static constexpr int CPW = 32 / T;       // chains per warp
     static constexpr int PPX = D / 8;        // 16-byte pieces per pixel
@@ -74,9 +75,7 @@ struct Geo {
     static constexpr int LENW = PADW + D + 2;
     // Word w of chain c lies at w * WST + c: the stride makes the windows of
     // a chain's lanes (NW words apart) fall into distinct banks.
-    static constexpr int WST = NW == 8   ? (T == 2 ? 18 : T == 4 ? 9 : T == 8 ? 5 : CPW)
-                               : NW == 2 ? 20
-                                         : (T == 2 ? 20 : T == 4 ? 10 : T == 8 ? 9 : CPW);
+    static constexpr int WST = T >= 16 ? CPW : NW == 2 || T == 2 ? 20 : T == 4 ? 10 : 9;
     static constexpr int BUFW = (LENW * WST + 3) / 4 * 4;   // (the rings between the windows stay 16-byte aligned)
     static constexpr int QL = kCH > T ? kCH / T : 1;   // pixels of a chunk a lane prepares
 };
@@ -263,7 +262,7 @@ __device__ __forceinline__ void seg_step(State<NW, T>& s, const uint32_t (&c)[NW
     if constexpr (MODE == kRefine) {
 #pragma unroll
         for (int i = 0; i < NW; ++i) win[(G::PADW + i) * G::WST] = s.L[i];
-        if (T > 1) __syncwarp();
+        __syncwarp();
         const uint32_t* wp = reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(win) + (at & 0xfffcu));
         const uint32_t sh = at << 4;   // the funnel takes it modulo 32
         uint32_t w0[NW + 2];
@@ -274,13 +273,10 @@ __device__ __forceinline__ void seg_step(State<NW, T>& s, const uint32_t (&c)[NW
 #pragma unroll
         for (int m = 0; m < NW; ++m) n0[m] = __funnelshift_r(w[m], w[m + 1], 16);
     } else {
-        uint32_t wl = kMax2, wr = kMax2;
-        if constexpr (T > 1) {
-            wl = __shfl_up_sync(0xffffffffu, s.L[NW - 1], 1, T);
-            wr = __shfl_down_sync(0xffffffffu, s.L[0], 1, T);
-            if (k == 0) wl = kMax2;
-            if (k == T - 1) wr = kMax2;
-        }
+        uint32_t wl = __shfl_up_sync(0xffffffffu, s.L[NW - 1], 1, T);
+        uint32_t wr = __shfl_down_sync(0xffffffffu, s.L[0], 1, T);
+        if (k == 0) wl = kMax2;
+        if (k == T - 1) wr = kMax2;
         w[0] = __funnelshift_r(wl, s.L[0], 16);
 #pragma unroll
         for (int m = 1; m < NW; ++m) w[m] = __funnelshift_r(s.L[m - 1], s.L[m], 16);
@@ -486,12 +482,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
         uint32_t info[G::QL];
         if (need) {
             uint32_t prev[G::QL];
-            if constexpr (T == 1) {
-                prev[0] = last;
-#pragma unroll
-                for (int i = 1; i < G::QL; ++i) prev[i] = cur[i - 1];
-                last = cur[G::QL - 1];
-            } else if constexpr (T == 2) {
+            if constexpr (T == 2) {
                 const uint32_t a = __shfl_xor_sync(0xffffffffu, cur[0], 1), z = __shfl_xor_sync(0xffffffffu, cur[1], 1);
                 prev[0] = k ? a : last;
                 prev[1] = k ? z : a;
@@ -549,8 +540,7 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
             }
             uint32_t at = 0, p22 = p2const;
             if (need) {
-                at = T == 1 ? info[q < G::QL ? q : 0]
-                            : __shfl_sync(0xffffffffu, info[T < kCH ? q / T : 0], T < kCH ? q % T : q, T);
+                at = __shfl_sync(0xffffffffu, info[T < kCH ? q / T : 0], T < kCH ? q % T : q, T);
                 p22 = __byte_perm(at, 0, 0x3232);
             }
             if (MODE == kCoarse && border) {
