@@ -60,8 +60,13 @@ def params_for(cost: int) -> dict:
 # against 3334.3 and 1791.6 MB of their own bytes
 # (profiles/segmented_chains_1080p_8pairs.md), and of the wide shape k_gtb
 # 1066.8 and k_gtbw 1854.7 against 1111.5 and 1808.2
-# (profiles/stage_kernels_1080p_8pairs.md).  The ratio carries over to a
-# step by each kind's own bytes.
+# (profiles/stage_kernels_1080p_8pairs.md).  A step's traffic is extrapolated
+# from these.  path_row stands for k_seg, captured in one shape (16-label
+# refinement, five segments): what L2 keeps of the costs between its two
+# directions and its columns changes with the level, and segments walked
+# again are not counted.  Where the autotuner takes the wide shape, k_grow
+# (2147.6 against 2222.9) is booked with k_seg's ratio; k_rowadd was not
+# captured and has no part in a step.
 AGG_TRAFFIC_PER_OWN_BYTE = {"path_tb": 1066.8 / 1111.5, "path_row": 2993.0 / 3334.3, "wta": 1828.7 / 1791.6,
                             "tbw": 1854.7 / 1808.2}
 
@@ -744,8 +749,8 @@ def result_line(args, world: int, headline: dict, plain: dict, pk: dict, npairs:
             "implementation_bytes_per_step": round(own / 1e9, 4),
             "traffic": round(sum(AGG_TRAFFIC_PER_OWN_BYTE[k] * prof[k]["bytes"] for k in agg_keys) / ps / 1e9, 4)
             if all(k in AGG_TRAFFIC_PER_OWN_BYTE for k in agg_keys) else None,
-            "traffic_unit": "GB per step (per kernel kind: ncu DRAM bytes per implementation byte x its "
-                            "implementation bytes)",
+            "traffic_unit": "GB per step, extrapolated (per kernel kind: ncu DRAM bytes per implementation byte of "
+                            "one captured launch x its implementation bytes)",
             "ms_per_step": round(agg_ms, 4), "launches_per_step": agg_launches,
             "avg_launch_ms": round(agg_ms / agg_launches, 5) if agg_launches else None}
         step_ms = headline["total_ms"] / args.steps

@@ -88,7 +88,12 @@ __host__ __device__ __forceinline__ bool uses_packed(int D) { return D == 16 || 
 // k_gtbw, k_cost_bt_strip) do not call it: blocks let in early pile up on
 // the SMs that finish first (with it in every kernel the rows of a 720p level
 // with 128 labels took half as long again, and 32 pairs 9.8 instead of 9.0
-// ms).
+// ms).  Batches that mix kinds of levels are the exceptions: where coarse and
+// refinement levels share a label count, the k_seg (and k_rowadd) of the
+// first kind lets that of the second in, and k_features goes by its first
+// job, whose cost may not be that of the cost kernel launched next.  The
+// order of the stream holds there as everywhere; those launches may take
+// longer.
 // What a kernel of the stream has written is read with plain loads (or
 // __ldcg), never with __ldg: that one is for memory no kernel writes while
 // the reading one is resident, and this one may be resident while the one
