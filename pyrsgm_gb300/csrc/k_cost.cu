@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(256) k_features(const __grid_constant__ Jobs<N
 
     __shared__ uint32_t tw[kFtSH][kFtSWW];   // byte c of row r: image pixel (y0 - 2 + r, x0 - 4 + c), clamped
     __shared__ __align__(16) uint32_t gi[kFtY][kFtGW];   // BT: gradient | intensity << 16 of column x0 - 4 + c
+    if (NJ > 1 && blockIdx.x + blockIdx.y + view + threadIdx.x == 0 && J.rewalked) *J.rewalked = 0;
     const int tx = threadIdx.x & 31, rr = threadIdx.x >> 5;
     const int xb = x0 + 4 * tx, y = y0 + rr;
     const int np = y < H ? imin(4, W - xb) : 0;     // pixels of this thread inside the image

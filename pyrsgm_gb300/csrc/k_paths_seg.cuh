@@ -19,8 +19,14 @@
 //   3. until no segment is marked.
 // Each round makes at least the first marked segment of a chain final, so
 // there are at most as many rounds as segments, and the result is that of
-// the serial walk whatever the costs are; scenes without texture only take
-// longer, at worst the serial walk after the parallel one.
+// the serial walk whatever the costs are.  Scenes without texture take longer:
+// at worst every segment is walked once in each round up to its own, in the
+// time of the serial walk after the parallel one on an idle GPU, in up to
+// three times the work (five segments) on a full one (see k_seg for what
+// batches do about it).  Waiting instead until the segment before is final
+// was slower on those very scenes (32 pairs of a gradient 10350 us, 10607;
+// blurred noise 10133, 10183 to 11953 with the first round cut short): a walk
+// from an end that is not final mostly meets the final one soon.
 //
 // The rows of both directions and the columns share one launch.  Costs come
 // through a ring of 4-step chunks per warp: the warp copies the 16-byte
@@ -54,6 +60,7 @@ enum { kStore = 0, kAgain = 1, kAdd = 2 };
 constexpr int kCH = 4;       // steps per chunk
 constexpr int kSC = 3;       // chunk slots per warp
 constexpr int kAhead = 3;    // chunks of look-ahead of the per-pixel inputs
+constexpr int kForgetful = 4;   // chains for each segment walked again to its end (k_seg)
 constexpr int kMaxSeg = 16;  // segments (warps) per block at most
 // ... for NW words a thread: shared memory for the rings, and registers.
 template <int NW>
@@ -602,35 +609,63 @@ __device__ __forceinline__ bool seg_walk(const Ctx<NW, T, MODE>& X, State<NW, T>
 
 }  // namespace sg
 
-// The chains of a level: blocks [0, row groups) hold rows (both directions),
-// the following ones columns; `rows_too` 0 launches the columns alone (their
-// path costs are all that is written, into V).
+// The chains of a level: groups [0, row groups) hold rows (both directions),
+// the following ones columns, a block a group; `rows_too` 0 launches the
+// columns alone (their path costs are all that is written, into V).
+//
+// Batches: images without texture (gradients, wide flat parts, sparse
+// detail) have chains that do not forget, whose segments are walked again
+// and again, up to three times the work.  A refinement level counts the
+// segments that it walks again to their ends (in launches as large as its
+// child's has to be for the rule below), and where its parent counted
+// more than one for every `kForgetful` chains, a block's warps take whole
+// chains instead, a group each: one walk, at the occupancy of the segments'.
+// Textured pairs count 0.05 a chain at most, the others 0.25 to 9.  32 pairs
+// of 1080p (us; segments, whole chains there, and before there were
+// segments): gradient 10337, 8763, 9789; diagonal one 11829, 8707, 9581;
+// sparse dots 11104, 8720, 9658; flat but for a sixteenth of the width 10777,
+// 8175, 8895; texture 7928, 7911, 9983.  A whole chain takes its n steps
+// however few there are beside it, segments a time that grows with their
+// number: whole chains pay from n / kWholePace groups per SM on (`may_whole`;
+// 12 pairs of 1080p: at 20 a level of 1920 steps 4666 and 3708, 8 pairs, at
+// 13, 2722 and 2955).
 template <int NW, int T, int MODE, int NJ>
-__global__ void __launch_bounds__(sg::max_seg<NW>() * 32) k_seg(const __grid_constant__ Jobs<NJ> jobs, int rows_too, int warm)
+__global__ void __launch_bounds__(sg::max_seg<NW>() * 32) k_seg(const __grid_constant__ Jobs<NJ> jobs, int rows_too, int warm,
+                                                                       int may_whole)
 {
     using namespace sg;
     using G = Geo<NW, T>;
     const LevelDesc& J = jobs.d[blockIdx.y];
     extern __shared__ __align__(16) uint32_t smem[];
-    const int segs = blockDim.x >> 5, b = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const Extent<MODE> e(J);
     const int Dr = labels_of<G::D>(J);
     const int rgroups = rows_too ? (2 * J.h + G::CPW - 1) / G::CPW : 0;
-    const bool rows = (int)blockIdx.x < rgroups;
-    const int g0 = (rows ? (int)blockIdx.x : (int)blockIdx.x - rgroups) * G::CPW;
-    if (!rows && g0 >= e.ncol) {   // the whole block is past the level
+    if ((int)blockIdx.x >= rgroups && ((int)blockIdx.x - rgroups) * G::CPW >= e.ncol) {   // the block is past the level
         after_previous();
         return;
     }
     int* lut = reinterpret_cast<int*>(smem);
     int* marked = reinterpret_cast<int*>(smem + 256);   // [segment][chain]: walk it (again)
-    uint32_t* mine = smem + 256 + (kMaxSeg + 1) * 32 + b * warp_words<NW, T, MODE>();
-    uint32_t* edge = smem + 256 + (kMaxSeg + 1) * 32 + segs * warp_words<NW, T, MODE>();
+    uint32_t* mine = smem + 256 + (kMaxSeg + 1) * 32 + warp * warp_words<NW, T, MODE>();
+    uint32_t* edge = smem + 256 + (kMaxSeg + 1) * 32 + warps * warp_words<NW, T, MODE>();
     for (int i = lane; i < warp_words<NW, T, MODE>(); i += 32) mine[i] = kMax2;
     if (rows_too) let_next_in();   // (columns alone: k_rowadd is next)
     after_previous();
+    // whole chains, a group a warp, or segments of one group's?
+    bool whole = false;
+    if constexpr (NJ > 1 && MODE == kRefine)
+        whole = may_whole && J.parent_rewalked && *J.parent_rewalked > (2 * J.ph + J.pw) / kForgetful;
+    const int segs = whole ? 1 : warps, b = whole ? 0 : warp;
+    const int group = whole ? (int)blockIdx.x * warps + warp : (int)blockIdx.x;
+    const bool rows = group < rgroups;
+    const int g0 = (rows ? group : group - rgroups) * G::CPW;
     const bool high = load_penalties(J, lut);
     const bool guard = __syncthreads_or(high);
+    if (whole) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *J.rewalked = INT_MAX;   // the child's chains too
+        if (!rows && g0 >= e.ncol) return;
+    }
 
     const int k = lane % T;
     Ctx<NW, T, MODE> X{J, lut, mine, mine + kSC * G::SLOTW + lane / T + NW * k * G::WST, edge, lane, lane / T, k, e,
@@ -671,6 +706,7 @@ __global__ void __launch_bounds__(sg::max_seg<NW>() * 32) k_seg(const __grid_con
         const unsigned m = T == 32 ? ne : (ne >> (X.c * T)) & ((1u << (T & 31)) - 1u);
         go = has && m != 0;
     }
+    [[maybe_unused]] int again = 0;   // segments walked again to their ends
     for (int round = 0; round < segs; ++round) {
         // a warp reads and clears its own row of marks; the warp before it
         // sets them between this barrier and the next
@@ -680,11 +716,13 @@ __global__ void __launch_bounds__(sg::max_seg<NW>() * 32) k_seg(const __grid_con
         if (__any_sync(0xffffffffu, go)) {
             const bool past = seg_walk<NW, T, MODE, kAgain>(X, s, ts, ts, te, nch, segs, b, 0, go, spec);
             if (past && X.k == 0) marked[(b + 1) * 32 + X.c] = 1;
+            if (NJ > 1 && MODE == kRefine && may_whole) again += __popc(__ballot_sync(0xffffffffu, past && X.k == 0));
         }
         __syncthreads();
         go = has && marked[b * 32 + X.c] != 0;
         start_state();
     }
+    if (NJ > 1 && MODE == kRefine && lane == 0 && again > 0 && J.rewalked) atomicAdd(J.rewalked, again);
 }
 
 // Segments for a launch of `blocks` chain groups whose longest walk has n
@@ -706,6 +744,7 @@ __global__ void __launch_bounds__(sg::max_seg<NW>() * 32) k_seg(const __grid_con
 // levels (160x96: 42 us a call, 46 at 64).
 constexpr int kMinSeg = 64, kMinSegSmall = 40;
 constexpr int kMaxRefineLabels = 256;   // pyrsgm_compute_level takes no more on a refinement level
+constexpr int kWholePace = 100;  // steps of a whole chain for each group per SM (k_seg)
 constexpr int kWarmSteps = 16;   // 0 to 32 measured within 5 % of each other, 64 10 % slower
 
 template <int MODE>
@@ -740,7 +779,8 @@ cudaError_t launch_seg_mode(const Jobs<NJ>& jobs, bool rows_too, cudaStream_t st
     const cudaError_t err = allow_smem(k_seg<NW, T, MODE, NJ>);
     if (err != cudaSuccess) return err;
     prof_begin(st);
-    launch_after(k_seg<NW, T, MODE, NJ>, dim3(grid, jobs.n), segs * 32, smem, st, jobs, rows_too ? 1 : 0, kWarmSteps);
+    launch_after(k_seg<NW, T, MODE, NJ>, dim3(grid, jobs.n), segs * 32, smem, st, jobs, rows_too ? 1 : 0, kWarmSteps,
+                 blocks * kWholePace >= (long long)n * sm_count() ? 1 : 0);
     count_launch();
     if (prof_enabled()) {
         // each path reads the cost volume and writes its costs once

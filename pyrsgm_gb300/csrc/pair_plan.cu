@@ -147,6 +147,9 @@ LevelDesc PairPlan::levelDesc(int level) const
     }
     fill_workspace_ptrs(d, ws[level]);
     d.p2lut = lut;
+    // (the levels share one P2 table: a workspace's own is free)
+    d.rewalked = ws[level].lut;
+    if (li.refine) d.parent_rewalked = ws[level + 1].lut;
     if (level > 0) {
         d.left = pyrL[level];
         d.right = pyrR[level];

@@ -49,6 +49,10 @@ struct LevelDesc {
     float* conf_raw;
     unsigned* keys;   // disp2 candidates: (cost << 16 | 0xFFFF - x) per right-image pixel
     const int* p2lut;
+    // batches: segments of this level walked again to their ends (k_seg), and
+    // the same of the parent level
+    int* rewalked;
+    const int* parent_rewalked;
     // outputs (device, optional)
     int16_t* out16;
     float* out32;
