@@ -160,11 +160,14 @@ cudaError_t launch_paths_seg16(const Jobs<NJ>& jobs, const LevelExtent& e, cudaS
 // Shape of the packed kernels for a launch: 2 (4 for 64 labels), the
 // segmented shape, or 8, the wide one (one thread per 16 labels, whole
 // chains).  With five segments a chain the segmented shape is the faster for
-// every batch measured (us, wide against segmented, 1080p: 2 pairs 2310 and
-// 771, 8 3298 and 2324, 32 9127 and 8345, 64 17177 and 16401; 64 VGA pairs of
-// 64 labels 4042 and 3335), so the wide one is taken only where
-// packed_words_override() (set through pyrsgm_gb300_set_packed_words), the
-// autotuner or PYRSGM_GB300_PACKED_WPS asks for it.
+// every batch of textured pairs measured (us, wide against segmented, 1080p:
+// 2 pairs 2310 and 771, 8 3298 and 2324, 32 9127 and 8345, 64 17177 and 16401;
+// 64 VGA pairs of 64 labels 4042 and 3335), and without texture, where its
+// batches walk whole chains too (k_seg), within 4 % of the wide one (32
+// pairs: gradients 8690 and 8761, 8605 and 8716, one grey value 7164 and
+// 7430).  So the wide one is taken only where packed_words_override() (set
+// through pyrsgm_gb300_set_packed_words), the autotuner or
+// PYRSGM_GB300_PACKED_WPS asks for it.
 inline int packed_nw(int D, long long rows)
 {
     const int force = packed_words_override();

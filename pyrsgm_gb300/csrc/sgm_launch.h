@@ -129,7 +129,7 @@ void tune_store(const TuneKey& k, const TuneEntry& e);
 // blocks may become resident while the previous kernel of the stream
 // finishes.  Every kernel waits for the whole one before it, so the order of
 // the stream is kept.  Hides the launch and the start of the blocks, 1 to 2
-// us a kernel (160x96 level, five kernels: 34 -> 27 us a call).  The launch
+// us a kernel (160x96 level, five kernels: 34 -> 28 us a call).  The launch
 // error is left for cudaGetLastError().
 template <class T>
 struct LaunchArg {

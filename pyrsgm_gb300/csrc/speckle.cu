@@ -15,7 +15,7 @@
 // pixels), the sizes of the tile roots added to their global roots, and one
 // pass that clears small regions.  The partition into regions is unique, so
 // the output is exactly that of a sequential flood fill.
-// Bound by the dependent walks of the four launches, not by the 30 bytes a
+// Bound by the dependent walks of the four launches, not by the 20 bytes a
 // pixel they move (a 1080p map: 146 us a call with a label a pixel in 32x8
 // tiles and every pixel in the border pass, 64 now).
 #include <cuda_runtime.h>
